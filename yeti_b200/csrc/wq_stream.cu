@@ -63,7 +63,6 @@ constexpr int kNE = kTQ / 2;     // max elements of a regular tile along u
 constexpr int kNEV = kTV / 2;    // ... along v
 constexpr int kThreads = kTQ * kTV;   // one thread per point of a plane tile
 constexpr int kWarps = kThreads / 32;
-constexpr int kCtasPerSm = 512 / kThreads;   // 2 (16 x 16 tiles) or 4 (16 x 8)
 constexpr int kHS = 2 * kTQ + 1; // channel stride of a warp's h block
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
@@ -158,6 +157,37 @@ __device__ __forceinline__ void load_pair(const double *p, double &a, double &b)
     b = v.y;
 }
 
+// acc += w x for two accumulators sharing the weight (one packed FMA in
+// FP32, the same bits as two scalar ones)
+__device__ __forceinline__ void fma2(float w, float x0, float x1, float2 &acc) {
+    acc = __ffma2_rn(make_float2(w, w), make_float2(x0, x1), acc);
+}
+__device__ __forceinline__ void fma2(double w, double x0, double x1, double2 &acc) {
+    acc.x += w * x0;
+    acc.y += w * x1;
+}
+// acc += w0 x0 + w1 x1.  FP32 adds the two products first: one by one onto
+// the accumulator costs an instruction less (2 % of the 64^3 p=3 apply) but
+// raises the apply's error from 9.3e-8 to 1.1e-7.  FP64, whose FMA pipe
+// is half as wide, chains two FMAs.
+__device__ __forceinline__ void mac2(float &acc, float w0, float x0, float w1, float x1) {
+    acc += w0 * x0 + w1 * x1;
+}
+__device__ __forceinline__ void mac2(double &acc, double w0, double x0, double w1, double x1) {
+    acc += w1 * x1;
+    acc += w0 * x0;
+}
+// the same for two accumulators sharing the weights: acc.x gets the products
+// with x0, x1 and acc.y those with y0, y1
+__device__ __forceinline__ void mac2(float2 &acc, float w0, float x0, float y0, float w1, float x1,
+                                     float y1) {
+    const float2 t = __fmul2_rn(make_float2(w1, w1), make_float2(x1, y1));
+    acc = __fadd2_rn(acc, __ffma2_rn(make_float2(w0, w0), make_float2(x0, y0), t));
+}
+template <class T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
+
 // ------------------------------------------------ bulk copies (TMA engine)
 constexpr int kWaitTries = 1 << 16;   // bound of every mbarrier wait
 
@@ -219,11 +249,12 @@ __host__ __device__ constexpr int pat_q0(int P, int pat, int e) {
 // Backward u of one channel of a warp's two rows: g[f] = sum_q W_kind(q,
 // f - rel(q)) h[q], walked element by element with the accumulators of the
 // element's p+1 functions named at compile time; one band row serves both
-// rows.  h: row 0 at h[q], row 1 at h[kTQ + q]; g: function f of row r at
+// rows (one packed FMA in FP32).  h: row 0 at h[q], row 1 at h[kTQ + q]; g: function f of row r at
 // g[r * RS + 27 f] (the G block's channel stride is 1).
 template <class T, int P, int PAT, bool PER>
 __device__ __forceinline__ void walk_u(const T *h, T *g, const T *tab, int kind, int ne_rt) {
     using D = Dims<P>;
+    using T2 = typename Pair<T>::type;
     constexpr int TS = D::TS, PBP = D::PBP, RS = D::RS;
     constexpr int NEM = pat_nemax(P, PAT), NF = NEM + P;
     const int ne = PAT == 1 ? NEM : ne_rt;
@@ -234,9 +265,9 @@ __device__ __forceinline__ void walk_u(const T *h, T *g, const T *tab, int kind,
         load_band<P>(tab + kind * PBP, wr[0]);
         load_band<P>(tab + TS + kind * PBP, wr[1]);
     }
-    T a0[NF], a1[NF];
+    T2 acc[NF];
 #pragma unroll
-    for (int f = 0; f < NF; f++) a0[f] = a1[f] = T(0);
+    for (int f = 0; f < NF; f++) acc[f].x = acc[f].y = T(0);
 #pragma unroll
     for (int e = 0; e < NEM; e++) {
         if (e < ne) {
@@ -255,21 +286,18 @@ __device__ __forceinline__ void walk_u(const T *h, T *g, const T *tab, int kind,
                     }
                     const T x0 = h[q], x1 = h[kTQ + q];
 #pragma unroll
-                    for (int m = 0; m <= P; m++) {
-                        a0[e + m] += w[m] * x0;
-                        a1[e + m] += w[m] * x1;
-                    }
+                    for (int m = 0; m <= P; m++) fma2(w[m], x0, x1, acc[e + m]);
                 }
             }
-            g[27 * e] = a0[e];
-            g[RS + 27 * e] = a1[e];
+            g[27 * e] = acc[e].x;
+            g[RS + 27 * e] = acc[e].y;
         }
     }
 #pragma unroll
     for (int f = 1; f < NF; f++)
         if (f >= ne && f < ne + P) {
-            g[27 * f] = a0[f];
-            g[RS + 27 * f] = a1[f];
+            g[27 * f] = acc[f].x;
+            g[RS + 27 * f] = acc[f].y;
         }
 }
 
@@ -323,6 +351,7 @@ template <class T, int P, int PAT, int NC, bool PER>
 __device__ __forceinline__ void walk_v(const T *gb, T *kp, int dfu, bool two, const T *tab, int ka,
                                        int ne_rt) {
     using D = Dims<P>;
+    using T2 = typename Pair<T>::type;
     constexpr int PBP = D::PBP, TS = D::TS, NEM = pat_nemax(P, PAT, kTV), NF = NEM + P;
     constexpr int KS = D::NFM * 18, RS = D::RS, GP = D::GP;
     const int ne = PAT == 1 ? NEM : ne_rt;
@@ -336,9 +365,9 @@ __device__ __forceinline__ void walk_v(const T *gb, T *kp, int dfu, bool two, co
     }
     const int dg = 27 * dfu;
     T *const kp1 = kp + 18 * dfu;
-    T A0[NF], A1[NF], B0[NF], B1[NF];
+    T2 K0[NF], K1[NF];   // .x: column fu, .y: column fu + dfu
 #pragma unroll
-    for (int f = 0; f < NF; f++) A0[f] = A1[f] = B0[f] = B1[f] = T(0);
+    for (int f = 0; f < NF; f++) K0[f].x = K0[f].y = K1[f].x = K1[f].y = T(0);
 #pragma unroll
     for (int e = 0; e < NEM; e++) {
         if (e < ne) {
@@ -361,30 +390,43 @@ __device__ __forceinline__ void walk_v(const T *gb, T *kp, int dfu, bool two, co
                     }
                     const T *g = gb + (q >> 1) * GP + (q & 1) * RS;
                     const T x0 = g[0], x1 = g[1], x2 = g[2];
-#pragma unroll
-                    for (int m = 0; m <= P; m++) {
-                        A0[e + m] += wa[m] * x0 + wb[m] * x1;
-                        A1[e + m] += wa[m] * x2;
-                    }
-                    if constexpr (NC == 2) {
+                    if constexpr (NC == 2 && P >= 4) {
+                        // both columns in packed FMAs: fewer instructions,
+                        // but the doubled weights take registers.  128x128x32
+                        // p=4 347 -> 327 us, 40^3 p=5 97 -> 89 us; 64^3 p=3
+                        // 144.3 -> 145.0 and p=2 131.5 -> 136 us (spills)
                         const T y0 = g[dg], y1 = g[dg + 1], y2 = g[dg + 2];
 #pragma unroll
                         for (int m = 0; m <= P; m++) {
-                            B0[e + m] += wa[m] * y0 + wb[m] * y1;
-                            B1[e + m] += wa[m] * y2;
+                            mac2(K0[e + m], wa[m], x0, y0, wb[m], x1, y1);
+                            fma2(wa[m], x2, y2, K1[e + m]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int m = 0; m <= P; m++) {
+                            mac2(K0[e + m].x, wa[m], x0, wb[m], x1);
+                            K1[e + m].x += wa[m] * x2;
+                        }
+                        if constexpr (NC == 2) {
+                            const T y0 = g[dg], y1 = g[dg + 1], y2 = g[dg + 2];
+#pragma unroll
+                            for (int m = 0; m <= P; m++) {
+                                mac2(K0[e + m].y, wa[m], y0, wb[m], y1);
+                                K1[e + m].y += wa[m] * y2;
+                            }
                         }
                     }
                 }
             }
-            store_pair(kp + e * KS, A0[e], A1[e]);
-            if (NC == 2 && two) store_pair(kp1 + e * KS, B0[e], B1[e]);
+            store_pair(kp + e * KS, K0[e].x, K1[e].x);
+            if (NC == 2 && two) store_pair(kp1 + e * KS, K0[e].y, K1[e].y);
         }
     }
 #pragma unroll
     for (int f = 1; f < NF; f++)
         if (f >= ne && f < ne + P) {
-            store_pair(kp + f * KS, A0[f], A1[f]);
-            if (NC == 2 && two) store_pair(kp1 + f * KS, B0[f], B1[f]);
+            store_pair(kp + f * KS, K0[f].x, K1[f].x);
+            if (NC == 2 && two) store_pair(kp1 + f * KS, K0[f].y, K1[f].y);
         }
 }
 
@@ -421,14 +463,14 @@ __device__ __forceinline__ void walk_v_generic(const T *gb, T *kp, int dfu, bool
         const T x0 = g[0], x1 = g[1], x2 = g[2];
 #pragma unroll
         for (int m = 0; m <= P; m++) {
-            A0[m] += wa[m] * x0 + wb[m] * x1;
+            mac2(A0[m], wa[m], x0, wb[m], x1);
             A1[m] += wa[m] * x2;
         }
         if constexpr (NC == 2) {
             const T y0 = g[dg], y1 = g[dg + 1], y2 = g[dg + 2];
 #pragma unroll
             for (int m = 0; m <= P; m++) {
-                B0[m] += wa[m] * y0 + wb[m] * y1;
+                mac2(B0[m], wa[m], y0, wb[m], y1);
                 B1[m] += wa[m] * y2;
             }
         }
@@ -471,8 +513,17 @@ struct StreamArgs {
     int wait_tries;            // polls of a wait for a coefficient copy
 };
 
+// CTAs per SM the registers are cut for.  FP32: 128 registers hold a thread's
+// work, and 51.5 KB of shared memory admit four.  FP64: the walks'
+// accumulators, the register rings and the 27 channels of a point, two
+// registers each, outgrow 128 from degree 3 on; fewer CTAs without spills are
+// faster.  Measured (us) with 4 / 3 / 2 CTAs: 64^3 p=2 249 / 247 / 294, p=3
+// 315 / 278 / 320, 128x128x32 p=4 1099 / 919 / 772, 40^3 p=5 250 / 220 / 185.
 template <class T, int P>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) k_wq_apply_stream(StreamArgs<T> a) {
+constexpr int kMinCtas = sizeof(T) == 4 || P == 2 ? 4 : P == 3 ? 3 : 2;
+
+template <class T, int P>
+__global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(StreamArgs<T> a) {
     using D = Dims<P>;
     constexpr int PB = D::PB, PBP = D::PBP, NFM = D::NFM, CPT = D::CPT;
     constexpr int TS = D::TS, GP = D::GP, ZHP = D::ZHP;
@@ -689,48 +740,26 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_wq_apply_stream(Stream
                         __syncwarp();   // the warp's Z is read; h takes its place
                         if (act) {
                             const int pt = (2 * warp + row) * nqu + qu;
-                            if constexpr (kStaged) {
-                                // point-major block in shared memory: 45 values per point
-                                const T *cp = cbuf + pt * kWQCoef;
-                                T h[27];
+                            // FP32: point-major block in shared memory, 45 values
+                            // per point; FP64: entry-major block in HBM.  Every
+                            // coefficient is read once
+                            const T *cp = kStaged ? cbuf + pt * kWQCoef
+                                                  : coef_t + (int64_t)qw * pstride + pt;
+                            T h[27];
 #pragma unroll
-                                for (int ch = 0; ch < 27; ch++) h[ch] = T(0);
+                            for (int ch = 0; ch < 27; ch++) h[ch] = T(0);
 #pragma unroll
-                                for (int I = 0; I < 9; I++) {
+                            for (int I = 0; I < 9; I++) {
 #pragma unroll
-                                    for (int J = I; J < 9; J++) {
-                                        const T sv = cp[sym9(I, J)];
-                                        const int i = I / 3, k = I % 3, j = J / 3, l = J % 3;
-                                        h[(i * 3 + k) * 3 + l] += sv * f[l][j];
-                                        if (I != J) h[(j * 3 + l) * 3 + k] += sv * f[k][i];
-                                    }
-                                }
-#pragma unroll
-                                for (int ch = 0; ch < 27; ch++) zh[ch * kHS + row * kTQ + qu] = h[ch];
-                            } else {
-                                // entry-major block in HBM, one output component at a
-                                // time (the symmetric partner entries hit L1)
-                                const T *cp = coef_t + (int64_t)qw * pstride + pt;
-#pragma unroll
-                                for (int i = 0; i < 3; i++) {
-#pragma unroll
-                                    for (int k = 0; k < 3; k++) {
-                                        T h0 = 0, h1 = 0, h2 = 0;
-#pragma unroll
-                                        for (int J = 0; J < 9; J++) {
-                                            const T sv = __ldg(cp + sym9(3 * i + k, J) * npts);
-                                            const int j = J / 3, l = J % 3;
-                                            if (l == 0) h0 += sv * f[0][j];
-                                            else if (l == 1) h1 += sv * f[1][j];
-                                            else h2 += sv * f[2][j];
-                                        }
-                                        const int ch = (i * 3 + k) * 3;
-                                        zh[(ch + 0) * kHS + row * kTQ + qu] = h0;
-                                        zh[(ch + 1) * kHS + row * kTQ + qu] = h1;
-                                        zh[(ch + 2) * kHS + row * kTQ + qu] = h2;
-                                    }
+                                for (int J = I; J < 9; J++) {
+                                    const T sv = kStaged ? cp[sym9(I, J)] : __ldg(cp + sym9(I, J) * npts);
+                                    const int i = I / 3, k = I % 3, j = J / 3, l = J % 3;
+                                    h[(i * 3 + k) * 3 + l] += sv * f[l][j];
+                                    if (I != J) h[(j * 3 + l) * 3 + k] += sv * f[k][i];
                                 }
                             }
+#pragma unroll
+                            for (int ch = 0; ch < 27; ch++) zh[ch * kHS + row * kTQ + qu] = h[ch];
                         }
                     }
                     __syncwarp();
@@ -815,8 +844,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_wq_apply_stream(Stream
                         load_pair(kb + 4, k20, k21);
                         const T s00 = k00 + k10, s01 = k01 + k11;
 #pragma unroll
-                        for (int m = 0; m < PB; m++)
-                            acc[cc][m] += w00[m] * s00 + w01[m] * s01 + w10[m] * k20 + w11[m] * k21;
+                        for (int m = 0; m < PB; m++) {
+                            if constexpr (kStaged) {
+                                acc[cc][m] += w00[m] * s00 + w01[m] * s01 + w10[m] * k20 + w11[m] * k21;
+                            } else {
+                                mac2(acc[cc][m], w00[m], s00, w01[m], s01);
+                                mac2(acc[cc][m], w10[m], k20, w11[m], k21);
+                            }
+                        }
                     }
                 }
                 // no barrier: the next B writes the Z/h parts after the
