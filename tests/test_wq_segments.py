@@ -1,0 +1,35 @@
+"""The streaming apply's plane ranges: CTAs whose ranges begin and end inside an
+element, cross from one tile into the next, or hold more than 16 planes (whose
+lengths then fall from one round of the SMs to the next).
+
+Bars as in test_wq.py: FP64 within 1e-12 relative (2-norm) of the FP64 oracle,
+FP32 within 2e-6.
+"""
+import numpy as np
+import pytest
+
+from oracle.wq_ops import WQOracle
+from yeti_b200.patches import cube_patch
+
+# (nel, p): tile planes per CTA (FP64 / FP32 on 148 SMs)
+CASES = [
+    ((9, 7, 11), 5),      # one plane each: every range is a part of an element
+    ((31, 19, 23), 4),    # about 3 and 1.5: ranges of unequal length
+    ((33, 35, 31), 2),    # about 4 and 4: ranges that cross tiles
+    ((49, 37, 45), 5),    # about 17 and 9: FP64 ranges that shorten by rounds
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nel,p", CASES)
+def test_gpu_apply_over_cut_plane_ranges(cuda_ok, nel, p):
+    from yeti_b200.wq import WQElasticity
+    P = cube_patch(nel, p, perturb=0.1, wrange=(0.8, 1.2), seed=3)
+    clamp = {"w0": (0, 1, 2), "v1": (1,)}
+    op, ref = WQElasticity(P, 1.0, 0.3, clamp), WQOracle(P, 1.0, 0.3, clamp)
+    u = np.random.default_rng(5).standard_normal(op.ndof)
+    k0 = ref.apply(u)
+    k1 = op.eval_Ku(u)
+    assert np.linalg.norm(k1 - k0) < 1e-12 * np.linalg.norm(k0)
+    k2 = op.eval_Ku(u.astype(np.float32), precision="f32").astype(np.float64)
+    assert np.linalg.norm(k2 - k0) < 2e-6 * np.linalg.norm(k0)

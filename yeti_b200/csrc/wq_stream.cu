@@ -5,8 +5,8 @@
 // Work decomposition
 // ------------------
 // The (u, v) point grid is cut into tiles of at most 16 x YETI_WQ_TV (8)
-// points made of whole elements; a CTA takes a tile and a range of elements
-// along w and marches through the w point planes of that range.  Every WQ point belongs
+// points made of whole elements; a CTA takes a tile and a range of w point
+// planes and marches through them.  Every WQ point belongs
 // to one element and, in each direction, its B0/B1/W** rows are non-zero for
 // the p+1 functions elem(q)..elem(q)+p only (checked on the host), so every
 // 1-D contraction is a band of width p+1.  Per plane:
@@ -33,7 +33,7 @@
 //   E  backward w: accumulation into a register ring of output planes
 //                  e..e+p; plane e is complete after element e and is added
 //                  to Ku (atomics: tiles overlap on the p halo functions,
-//                  element ranges overlap on p planes)
+//                  plane ranges overlap on p planes)
 //
 // The walks keep the p+1 functions of the current element in registers.  In
 // a regular tile (every element owns two points: all but the first and last
@@ -42,6 +42,7 @@
 // While a plane is processed, the next plane's coefficient block
 // (contiguous, 256-byte aligned) is prefetched into L2.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 
@@ -482,11 +483,23 @@ __device__ __forceinline__ void walk_v_generic(const T *gb, T *kp, int dfu, bool
     }
 }
 
-__device__ __forceinline__ int relu_last_plus1(const int *elem, int q0, int nq, int f0) {
-    return elem[q0 + nq - 1] - f0 + 1;
-}
-
 }  // namespace
+
+// A CTA's work item: w planes [qb, qe) of one tile, with everything the CTA
+// needs to know about the tile (read by one load instead of a chain of table
+// lookups).
+struct __align__(16) WQSeg {
+    int64_t coef;              // first coefficient of the tile's plane 0
+    int pstride;               // coefficients per w plane of the tile (padded)
+    int qb, qe, eb;            // planes, element of plane qb
+    int qu0, qv0;              // first point of the tile
+    unsigned char nqu, nqv;    // its points
+    unsigned char regu, regv;  // tile patterns (walk_u): 1 regular full, 4 regular, 2 first, 3 last,
+                               // 0 other; bit 3: periodic band rows (pattern 1 or 4)
+    unsigned char nfu, nfv, neu, nev;   // its functions and elements
+    int fu0, fv0;              // first functions
+};
+static_assert(sizeof(WQSeg) == 48, "three 16-byte loads");
 
 template <class T>
 struct StreamArgs {
@@ -494,17 +507,10 @@ struct StreamArgs {
     T *Ku;
     const int *done;
     const T *coef;
-    const int64_t *tile_off;   // first coefficient of a tile
-    const int *tile_pstride;   // coefficients per w plane of a tile (padded)
-    const int *tq0[2];         // first point of a u / v tile
-    const int *tnq[2];         // points of a u / v tile
-    const int *treg[2];        // tile pattern (walk_u): 1 regular full, 4 regular, 2 first, 3 last, 0 other
-    int ntile[2];
-    const int *elem[3];        // element owning each point
+    const int *elem[2];        // element owning each point along u, v
     const T *band[3];          // [nqp][6][round4(p+1)]: B0 B1 W00 W01 W10 W11
     const int *wq0;            // first w point of each element (nel_w + 1)
-    int nqw;                   // w points
-    const int4 *seg;           // (tile, e_begin, e_end, -)
+    const WQSeg *seg;
     const int *cta_seg;        // segments of a CTA
     int nfun[3];
     int64_t ncp;
@@ -551,22 +557,17 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     const int64_t plane = (int64_t)a.nfun[0] * a.nfun[1];
 
     for (int si = a.cta_seg[blockIdx.x]; si < a.cta_seg[blockIdx.x + 1]; si++) {
-        const int4 sg = a.seg[si];
-        const int tu = sg.x % a.ntile[0], tv = sg.x / a.ntile[0];
-        const int qu0 = a.tq0[0][tu], nqu = a.tnq[0][tu];
-        const int qv0 = a.tq0[1][tv], nqv = a.tnq[1][tv];
-        // pattern in bits 0..2, bit 3: periodic band rows (pattern 1 or 4)
-        const int patu = a.treg[0][tu] & 7, patv = a.treg[1][tv] & 7;
-        const bool peru = (a.treg[0][tu] & 8) != 0, perv = (a.treg[1][tv] & 8) != 0;
+        const WQSeg sg = a.seg[si];
+        const int qu0 = sg.qu0, nqu = sg.nqu, qv0 = sg.qv0, nqv = sg.nqv;
+        const int patu = sg.regu & 7, patv = sg.regv & 7;
+        const bool peru = (sg.regu & 8) != 0, perv = (sg.regv & 8) != 0;
         const bool regu = patu == 1 || patu == 4, regv = patv == 1 || patv == 4;
-        const int fu0 = a.elem[0][qu0], fv0 = a.elem[1][qv0];
-        const int nfu = a.elem[0][qu0 + nqu - 1] + PB - fu0;
-        const int nfv = a.elem[1][qv0 + nqv - 1] + PB - fv0;
-        const int neu = relu_last_plus1(a.elem[0], qu0, nqu, fu0);   // elements of the tile
-        const int nev = relu_last_plus1(a.elem[1], qv0, nqv, fv0);
+        const int fu0 = sg.fu0, fv0 = sg.fv0;
+        const int nfu = sg.nfu, nfv = sg.nfv;
+        const int neu = sg.neu, nev = sg.nev;
         const int npts = nqu * nqv;
-        const T *coef_t = a.coef + a.tile_off[sg.x];
-        const int pstride = a.tile_pstride[sg.x];
+        const T *coef_t = a.coef + sg.coef;
+        const int pstride = sg.pstride;
         const int pbytes = npts * kWQCoef * (int)sizeof(T);
         const int nrow = min(2, nqv - 2 * warp);   // rows of this warp (may be <= 0)
 
@@ -580,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
         if (tid < kTV) relv[tid] = tid < nqv ? a.elem[1][qv0 + tid] - fv0 : 0;
         const uint32_t cbytes = (uint32_t)((npts * kWQCoef * (int)sizeof(T) + 15) & ~15);
         if constexpr (kStaged) {
-            if (tid == 0) bulk_load(cbuf, coef_t + (int64_t)a.wq0[sg.y] * pstride, cbytes, bar);
+            if (tid == 0) bulk_load(cbuf, coef_t + (int64_t)sg.qb * pstride, cbytes, bar);
         }
         // stage D thread: (ik, fu) and (ik, fu + nfp), the nine ik fastest
         // (FP64: one fu, nfp = nfu)
@@ -653,20 +654,21 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
 #pragma unroll
         for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
-            for (int m = 0; m <= P; m++) x[cc][m] = load_x(cc, sg.y + m);
-        stage_a(a.wq0[sg.y]);
+            for (int m = 0; m <= P; m++) x[cc][m] = load_x(cc, sg.eb + m);
+        stage_a(sg.qb);
         if (!kStaged) {
-            const char *p0 = reinterpret_cast<const char *>(coef_t + (int64_t)a.wq0[sg.y] * pstride);
+            const char *p0 = reinterpret_cast<const char *>(coef_t + (int64_t)sg.qb * pstride);
             for (int off = tid * 128; off < pbytes; off += kThreads * 128) prefetch_l2(p0 + off);
         }
 
-        for (int e = sg.y; e < sg.z; e++) {
+        int e = sg.eb;
+        for (int qw = sg.qb; qw < sg.qe; e++) {
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) acc[cc][P] = T(0);
-            const int qw_end = a.wq0[e + 1];
-            for (int qw = a.wq0[e]; qw < qw_end; qw++) {
+            const int qw_end = min(a.wq0[e + 1], sg.qe);
+            for (; qw < qw_end; qw++) {
                 const T *bw = a.band[2] + (size_t)qw * 6 * PBP;
-                if (!kStaged && qw + 1 < a.nqw) {
+                if (!kStaged && qw + 1 < sg.qe) {
                     // FP64 reads the coefficients straight from HBM: prefetch
                     // the next plane into L2 (FP32 stages it with a bulk copy)
                     const char *pn = reinterpret_cast<const char *>(coef_t + (int64_t)(qw + 1) * pstride);
@@ -789,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                 __syncthreads();
                 if constexpr (kStaged) {
                     // every warp is done with the block: bring in the next plane's
-                    if (tid == 0 && qw + 1 < a.wq0[sg.z])
+                    if (tid == 0 && qw + 1 < sg.qe)
                         bulk_load(cbuf, coef_t + (int64_t)(qw + 1) * pstride, cbytes, bar);
                 }
                 // ---- D: backward v, thread (i, k) x two fu; K aliases the Z/h parts
@@ -814,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                 }
                 // ---- A of the next plane, beside D (RY is free once B is done);
                 // at an element's last plane the u ring advances first
-                if (qw + 1 < a.wq0[sg.z]) {
+                if (qw + 1 < sg.qe) {
                     if (qw + 1 == qw_end) {
 #pragma unroll
                         for (int cc = 0; cc < CPT; cc++) {
@@ -857,7 +859,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                 // no barrier: the next B writes the Z/h parts after the
                 // barrier that opens the next plane
             }
-            // output plane e is complete for this element range
+            // output plane e is complete for this plane range
 #pragma unroll
             for (int cc = 0; cc < CPT; cc++) {
                 retire(cc, e, acc[cc][0]);
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
 #pragma unroll
         for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
-            for (int m = 0; m < P; m++) retire(cc, sg.z + m, acc[cc][m]);
+            for (int m = 0; m < P; m++) retire(cc, e + m, acc[cc][m]);
     }
 }
 
@@ -1008,6 +1010,7 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
     const int P = op->p[0], PBP = (P + 1 + 3) / 4 * 4;
     std::vector<int> elem_q0[3];
     std::vector<double> band_uv[2];
+    std::vector<int> elem_uv[2];
     for (int d = 0; d < 3; d++) {
         const int nel = op->nel[d], nq = op->nqp[d];
         // element ownership of the points (first element p+1 points, last
@@ -1036,8 +1039,11 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
                                     d, f, q);
                 }
         std::vector<float> bandf(band.begin(), band.end());
-        if (d < 2) band_uv[d] = band;
-        YETI_TRY(upload_vec(ctx, st.elem[d], elem));
+        if (d < 2) {
+            band_uv[d] = band;
+            elem_uv[d] = elem;
+        }
+        if (d < 2) YETI_TRY(upload_vec(ctx, st.elem[d], elem));
         YETI_TRY(upload_vec(ctx, st.band64[d], band));
         YETI_TRY(upload_vec(ctx, st.band32[d], bandf));
     }
@@ -1058,7 +1064,6 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
                                   row * sizeof(double)) == 0;
             if (per) treg[d][t] |= 8;
         }
-        YETI_TRY(upload_vec(ctx, st.treg[d], treg[d]));
         st.ntile[d] = (int)tq0[d].size();
         YETI_TRY(upload_vec(ctx, st.tq0[d], tq0[d]));
         YETI_TRY(upload_vec(ctx, st.tnq[d], tnq[d]));
@@ -1084,36 +1089,68 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
     YETI_TRY(stream_prepare_kernels(op));
     int nsm = 0;
     YETI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-    // segments: (tile, element range) cut from the tile-major sequence so
-    // that every CTA gets about the same number of tile planes (a plane of a
-    // narrow tile costs a CTA about as much as a full one: the same stages,
-    // barriers and walks, with lanes idle)
+    // segments: (tile, plane range) cut from the tile-major sequence so that
+    // the CTAs get equal numbers of tile planes, give or take one (a plane
+    // of a narrow tile costs a CTA about as much as a full one: the same
+    // stages, barriers and walks, with lanes idle).  The cut falls between any
+    // two planes, also inside an element: a small patch is spread over as many
+    // CTAs as it has tile planes, and the boundary elements, which own p+1 and
+    // p+2 planes, hold no CTA longer than the others (8^3 p=2 FP64 23.7 -> 13.4
+    // us, 21x17x25 p=3 FP64 31.9 -> 23.7 us, 61x47x29 p=4 FP64 174 -> 154 us).
+    // On a full SM the CTA that was launched first runs ahead of the last one
+    // (117 against 130 us of the 64^3 p=3 FP32 apply, with equal planes), so
+    // with 16 planes per CTA or more (fewer cannot be cut that finely) the
+    // CTAs of each round of the SMs get 3 % less than those of the round
+    // before: 141 -> 138 us there, 128x128x32 p=4 FP32 321 -> 310 us; 2 % and
+    // 5 % measured 139.6 and 139.2 us, and at 11 planes (40^3 p=5) 3 % cost 5 %.
+    constexpr double kRoundLess = 0.03;
+    constexpr int kRoundPlanes = 16;
+    std::vector<int> elem_w;
+    for (int e = 0; e < op->nel[2]; e++)
+        elem_w.insert(elem_w.end(), elem_q0[2][e + 1] - elem_q0[2][e], e);
     for (int which = 0; which < 2; which++) {
-        // item (t, e) goes to CTA floor(work before it * ncta / total work);
-        // consecutive items of one CTA and one tile form a segment
         const int64_t total = (int64_t)ntiles * nqw;
-        const int64_t nitems = (int64_t)ntiles * op->nel[2];
-        const int ncta = (int)std::max<int64_t>(
-            1, std::min<int64_t>((int64_t)nsm * st.per_sm[which], nitems));
-        std::vector<int4> seg;
+        const int64_t ncta = std::min<int64_t>((int64_t)nsm * st.per_sm[which], total);
+        std::vector<WQSeg> seg;
         std::vector<int> cta_seg(ncta + 1, 0);
-        int64_t before = 0;
-        int last_cta = -1;
-        for (int t = 0; t < ntiles; t++) {
-            for (int e = 0; e < op->nel[2]; e++) {
-                const int c = (int)std::min<int64_t>(ncta - 1, before * ncta / total);
-                before += elem_q0[2][e + 1] - elem_q0[2][e];
-                if (c != last_cta || seg.empty() || seg.back().x != t) {
-                    for (int k = last_cta + 1; k <= c; k++) cta_seg[k] = (int)seg.size();
-                    seg.push_back(make_int4(t, e, e + 1, 0));
-                    last_cta = c;
-                } else {
-                    seg.back().z = e + 1;
-                }
-            }
+        // planes before CTA c: sum over the CTAs before it of 1 + less * ((per_sm - 1) / 2 - round)
+        const double less = total >= kRoundPlanes * ncta ? kRoundLess : 0.0;
+        std::vector<int64_t> cut(ncta + 1, total);
+        double sum = 0.0, all = 0.0;
+        auto share = [&](int64_t c) { return 1.0 + less * (0.5 * (st.per_sm[which] - 1) - (double)(c / nsm)); };
+        for (int64_t c = 0; c < ncta; c++) all += share(c);
+        for (int64_t c = 0; c < ncta; c++) {
+            cut[c] = (int64_t)std::floor((double)total * (sum / all) + 1e-6);
+            sum += share(c);
         }
-        for (int k = last_cta + 1; k <= ncta; k++) cta_seg[k] = (int)seg.size();
-        st.grid[which] = ncta;
+        for (int64_t c = 0; c < ncta; c++) {
+            const int64_t end = cut[c + 1];
+            for (int64_t i = cut[c]; i < end;) {
+                const int t = (int)(i / nqw), tu = t % st.ntile[0], tv = t / st.ntile[0];
+                WQSeg sg;
+                sg.coef = toff[t];
+                sg.pstride = pstride[t];
+                sg.qb = (int)(i % nqw);
+                sg.qe = (int)std::min<int64_t>(nqw, sg.qb + (end - i));
+                sg.eb = elem_w[sg.qb];
+                sg.qu0 = tq0[0][tu];
+                sg.qv0 = tq0[1][tv];
+                sg.nqu = (unsigned char)tnq[0][tu];
+                sg.nqv = (unsigned char)tnq[1][tv];
+                sg.regu = (unsigned char)treg[0][tu];
+                sg.regv = (unsigned char)treg[1][tv];
+                sg.fu0 = elem_uv[0][tq0[0][tu]];
+                sg.fv0 = elem_uv[1][tq0[1][tv]];
+                sg.neu = (unsigned char)(elem_uv[0][tq0[0][tu] + tnq[0][tu] - 1] - sg.fu0 + 1);
+                sg.nev = (unsigned char)(elem_uv[1][tq0[1][tv] + tnq[1][tv] - 1] - sg.fv0 + 1);
+                sg.nfu = (unsigned char)(sg.neu + P);
+                sg.nfv = (unsigned char)(sg.nev + P);
+                i += sg.qe - sg.qb;
+                seg.push_back(sg);
+            }
+            cta_seg[c + 1] = (int)seg.size();
+        }
+        st.grid[which] = (int)ncta;
         YETI_TRY(upload_vec(ctx, st.seg[which], seg));
         YETI_TRY(upload_vec(ctx, st.cta_seg[which], cta_seg));
     }
@@ -1187,16 +1224,8 @@ static int launch_stream(yeti_wq_op *op, const T *u, T *Ku, const int *done, cud
     a.Ku = Ku;
     a.done = done;
     a.coef = (f64 ? op->coef64 : op->coef32).template as<T>();
-    a.tile_off = st.tile_off.as<int64_t>();
-    a.tile_pstride = st.tile_pstride.as<int>();
-    for (int d = 0; d < 2; d++) {
-        a.tq0[d] = st.tq0[d].as<int>();
-        a.tnq[d] = st.tnq[d].as<int>();
-        a.treg[d] = st.treg[d].as<int>();
-        a.ntile[d] = st.ntile[d];
-    }
     for (int d = 0; d < 3; d++) {
-        a.elem[d] = st.elem[d].as<int>();
+        if (d < 2) a.elem[d] = st.elem[d].as<int>();
         a.band[d] = (f64 ? st.band64[d] : st.band32[d]).template as<T>();
         a.nfun[d] = op->n[d];
         a.cmask[d] = op->cmask[d];
@@ -1204,8 +1233,7 @@ static int launch_stream(yeti_wq_op *op, const T *u, T *Ku, const int *done, cud
     a.wq0 = st.wq0.as<int>();
     a.err = st.err.as<int>();
     a.wait_tries = st.wait_tries;
-    a.nqw = op->nqp[2];
-    a.seg = st.seg[which].as<int4>();
+    a.seg = st.seg[which].as<WQSeg>();
     a.cta_seg = st.cta_seg[which].as<int>();
     a.ncp = op->ncp;
     k_wq_apply_stream<T, P><<<st.grid[which], kThreads, st.smem[which], s>>>(a);
