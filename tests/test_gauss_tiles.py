@@ -1,0 +1,64 @@
+"""The stiffness and mass kernels' pair tiles and point chunks: element sizes
+with an odd and an even number of nodes, one tile and many, points in one
+chunk and in several, pair sums kept in shared memory (mass) and not, output
+arrays on 8-byte boundaries.  Bit-identical to the oracle, as in
+test_assembly.py and test_mass.py."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from yeti_b200.patches import cube_patch, u1_system_args
+from yeti_b200.stiffmtrx_elemstorage import SYSTEM_ARG_NAMES, sys_linmat_lindef_static
+
+# (nel, p): 8, 12, 27, 64, 125 and 210 nodes per element
+CASES = [((3, 2, 2), (1, 1, 1)), ((2, 3, 2), (2, 1, 1)), ((2, 2, 3), (2, 2, 2)),
+         ((2, 2, 1), (3, 3, 3)), ((2, 1, 1), (4, 4, 4)), ((1, 1, 2), (6, 5, 4))]
+
+
+def _args(nel, p):
+    return u1_system_args(cube_patch(nel, p, perturb=0.1, wrange=(0.8, 1.2), seed=4), E=2.1,
+                          nu=0.3, rho=7.8)
+
+
+def _mass_inputs(args):
+    d = dict(zip(SYSTEM_ARG_NAMES, args))
+    return [d[k] for k in ("activeElement", "nb_data", "COORDS3D", "IEN", "nb_elem_patch", "Nkv",
+                           "Ukv", "Nijk", "weight", "Jpqr", "ELT_TYPE", "PROPS", "JPROPS", "RHO",
+                           "TENSOR", "ind_dof_free", "nb_dof_free", "MCRD", "NBINT", "NNODE")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nel,p", CASES)
+def test_gpu_stiffness_and_mass_tiles_match_oracle(cuda_ok, nel, p):
+    from yeti_b200.massmtrx import build_cmassmatrix
+    args = _args(nel, p)
+    for got, ref in zip(sys_linmat_lindef_static(*args), oracle.sys_linmat_lindef_static(*args)):
+        np.testing.assert_array_equal(got, ref)
+    m = _mass_inputs(args)
+    for got, ref in zip(build_cmassmatrix(*m), oracle.build_cmassmatrix(m)):
+        np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.gpu
+def test_gpu_assembly_into_arrays_on_8_byte_boundaries(cuda_ok):
+    import torch
+    from yeti_b200 import _lib
+    from yeti_b200.stiffmtrx_elemstorage import pack_u1_model
+    args = _args((2, 2, 2), (2, 2, 2))
+    pm = pack_u1_model(*args)
+    n = pm.nb_data
+    k = torch.full((n + 2,), -1.0, dtype=torch.float64, device="cuda")
+    r = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    c, F = torch.zeros_like(r), torch.zeros(pm.nb_dof_tot, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx = _lib.default_context()
+    _lib.check(_lib.lib().yeti_assemble_u1_coo_ex(
+        ctx.handle, ctypes.byref(pm.struct), n, k[1:].data_ptr(), r[1:].data_ptr(),
+        c[1:].data_ptr(), F.data_ptr(), _lib.MEM_DEVICE, _lib.STIFF_PAIRS), "assemble")
+    ref = oracle.sys_linmat_lindef_static(*args)
+    np.testing.assert_array_equal(k[1:-1].cpu().numpy(), ref[0])
+    np.testing.assert_array_equal(r[1:].cpu().numpy(), ref[1])
+    np.testing.assert_array_equal(c[1:].cpu().numpy(), ref[2])
+    assert k[0] == -1.0 and k[-1] == -1.0

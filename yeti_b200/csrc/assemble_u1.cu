@@ -6,15 +6,15 @@
 // shap (shap.f90:21-180), stiffmatrix_byCP (stiffmatrix.F90:130-225),
 // material_lib (material_lib.f90:75-87) and shapPress (shapPress.f:18-262).
 //
-// Kernel design: one CTA per element.  Stage A: one thread per Gauss point
-// evaluates the rational basis derivatives dR/dx (3 x nnode) and the volume
-// weight into shared memory.  Stage B: one thread per control-point pair
-// (i <= j) accumulates the 3x3 block over the Gauss points and writes its 9
-// (or 6, diagonal) COO entries at the reference's slot positions, so the
-// writes of consecutive threads are contiguous.  Elements whose Gauss data do
-// not fit shared memory are processed in Gauss-point chunks (read-modify-write
-// of the element's own slots).  The load vector is a second kernel over the
-// elements that carry distributed loads.
+// Kernel design: one CTA per element.  Stage A evaluates the rational basis
+// derivatives dR/dx (3 x nnode) and the volume weight at the Gauss points into
+// shared memory.  Stage B: one thread per 2 x 2 tile of control-point pairs
+// accumulates the four 3x3 blocks over the Gauss points and writes them at the
+// reference's slot positions; the row and column indices are written by a
+// pass of their own with consecutive threads on consecutive slots.  Elements
+// whose Gauss data do not fit shared memory are processed in Gauss-point
+// chunks (read-modify-write of the element's own slots).  The load vector is
+// a second kernel over the elements that carry distributed loads.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -263,7 +263,7 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
 
 // ---------------------------------------------------------------- kernels
 struct StiffArgs {
-    int p0, p1, p2, nn, nq, qchunk;
+    int p0, p1, p2, nn, nq, ng, qchunk;
     const double *U0, *U1, *U2;
     const double *gauss;
     const double *coords;
@@ -332,21 +332,25 @@ __device__ inline void rational_derivs(
             }
 }
 
-// MatrixInv for 3x3 (operateurs.f:385-423); returns the determinant.
-__device__ inline double inv3(const double B[3][3], double A[3][3]) {
-    double det = B[0][1] * B[1][2] * B[2][0] - B[0][2] * B[1][1] * B[2][0] +
-                 B[0][2] * B[1][0] * B[2][1] - B[0][0] * B[1][2] * B[2][1] +
-                 B[0][0] * B[1][1] * B[2][2] - B[0][1] * B[1][0] * B[2][2];
-    A[0][0] = (B[1][1] * B[2][2] - B[1][2] * B[2][1]) / det;
-    A[0][1] = (B[0][2] * B[2][1] - B[0][1] * B[2][2]) / det;
-    A[0][2] = (B[0][1] * B[1][2] - B[0][2] * B[1][1]) / det;
-    A[1][0] = (B[1][2] * B[2][0] - B[1][0] * B[2][2]) / det;
-    A[1][1] = (B[0][0] * B[2][2] - B[0][2] * B[2][0]) / det;
-    A[1][2] = (B[0][2] * B[1][0] - B[0][0] * B[1][2]) / det;
-    A[2][0] = (B[1][0] * B[2][1] - B[1][1] * B[2][0]) / det;
-    A[2][1] = (B[0][1] * B[2][0] - B[0][0] * B[2][1]) / det;
-    A[2][2] = (B[0][0] * B[1][1] - B[0][1] * B[1][0]) / det;
-    return det;
+// Entry (r, c) = rc / 3, rc % 3 of the inverse of a 3x3 matrix (MatrixInv,
+// operateurs.f:385-423).
+__device__ inline double inv3_entry(const double B[3][3], int rc) {
+    const double det = B[0][1] * B[1][2] * B[2][0] - B[0][2] * B[1][1] * B[2][0] +
+                       B[0][2] * B[1][0] * B[2][1] - B[0][0] * B[1][2] * B[2][1] +
+                       B[0][0] * B[1][1] * B[2][2] - B[0][1] * B[1][0] * B[2][2];
+    double v = 0.0;
+    switch (rc) {
+        case 0: v = B[1][1] * B[2][2] - B[1][2] * B[2][1]; break;
+        case 1: v = B[0][2] * B[2][1] - B[0][1] * B[2][2]; break;
+        case 2: v = B[0][1] * B[1][2] - B[0][2] * B[1][1]; break;
+        case 3: v = B[1][2] * B[2][0] - B[1][0] * B[2][2]; break;
+        case 4: v = B[0][0] * B[2][2] - B[0][2] * B[2][0]; break;
+        case 5: v = B[0][2] * B[1][0] - B[0][0] * B[1][2]; break;
+        case 6: v = B[1][0] * B[2][1] - B[1][1] * B[2][0]; break;
+        case 7: v = B[0][1] * B[2][0] - B[0][0] * B[2][1]; break;
+        default: v = B[0][0] * B[1][1] - B[0][1] * B[1][0]; break;
+    }
+    return v / det;
 }
 
 // Parent-element Jacobian determinant (shap.f90:155-178).
@@ -360,24 +364,97 @@ __device__ inline double parent_det(const double J[3][3], const double *u1,
            A[0][1] * A[1][0] * A[2][2] - A[1][2] * A[2][1] * A[0][0];
 }
 
-// Shared-memory layout of one Gauss-point chunk of the stiffness and mass
-// kernels: per point the six 1-D rows (FN dFN FM dFM FL dFL, kMaxDeg1 each),
-// the nn rational numerators, 3 nn derivative values and kStiffQS scalars
-// (sx[3], 1/S, J then J^-1 [9], dv).
-__host__ __device__ inline size_t stiff_perq(int nn) {
-    return (size_t)6 * kMaxDeg1 + 4 * (size_t)nn + kStiffQS;
+// Shared memory of the stiffness and mass kernels (doubles): the element's
+// control points and weights, 1-D rows and node indices, then per point of a
+// chunk the derivative values (3 nnp and padding; nnp: nn rounded up to even,
+// so that a tile's two nodes are three aligned 16-byte loads) and kStiffQS
+// scalars (sx[3], 1/S, J[9], dv, and the rest of J^-1); the mass kernel has
+// kMassQS, and nn basis values more.
+constexpr int kStiffQS = 19, kMassQS = 15;
+__host__ __device__ inline int pad2(int n) { return (n + 1) & ~1; }
+__host__ __device__ inline size_t stiff_fixed(int nn, int ng) {
+    return (size_t)4 * pad2(nn) + pad2(basis_rows_doubles(ng)) + pad2(nn);
+}
+// derivative values of a point: even, and 2 mod 4, so that the same entry of
+// consecutive points falls on eight banks or more
+__host__ __device__ inline int stiff_ds(int nn) { return (3 * pad2(nn) + 1) / 4 * 4 + 2; }
+__host__ __device__ inline size_t stiff_perq(int nn) { return (size_t)stiff_ds(nn) + kStiffQS; }
+__host__ __device__ inline size_t mass_perq(int nn) { return (size_t)stiff_ds(nn) + kMassQS + pad2(nn); }
+
+// Scalar of a point that takes entry c of the inverse Jacobian.
+__host__ __device__ constexpr int inv_slot(int c) { return c < 4 ? c : c + 10; }
+
+// First slot of column node j's blocks, relative to the element's.
+__host__ __device__ inline int64_t slot_col(int j) { return 9LL * j * (j - 1) / 2 + 6LL * j; }
+
+// The slots of an element, a warp per column node j and consecutive lanes on
+// consecutive slots: visit(slot, i, j, row component, column component) for
+// the 9 j + 6 slots of the column (9 per node i < j with the row component
+// fastest, then the upper triangle of the diagonal block).
+template <class V>
+__device__ __forceinline__ void for_slots(int nn, int64_t base, V visit) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int j = warp; j < nn; j += nwarp) {
+        const int64_t jb = base + slot_col(j);
+        for (int sl = lane; sl < 9 * j + 6; sl += 32) {
+            int i = sl / 9, r = sl - 9 * i, ll, kk;
+            if (sl < 9 * j) {
+                ll = r / 3;
+                kk = r - 3 * ll;
+            } else {
+                i = j;
+                r = sl - 9 * j;
+                ll = r < 1 ? 0 : r < 3 ? 1 : 2;
+                kk = r - ll * (ll + 1) / 2;
+            }
+            visit(jb + sl, i, j, kk, ll);
+        }
+    }
 }
 
-__global__ void __launch_bounds__(256)
+// Tile t of the upper triangle of 2 x 2 tiles, column by column.
+__device__ __forceinline__ void tile_of(int t, int &ti, int &tj) {
+    tj = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while (tj * (tj + 1) / 2 > t) tj--;
+    while ((tj + 1) * (tj + 2) / 2 <= t) tj++;
+    ti = t - tj * (tj + 1) / 2;
+}
+
+// The 18 values of two consecutive blocks, by 16-byte stores.
+__device__ __forceinline__ void store18(double *o, const double (&v)[18]) {
+    if ((reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 18; i += 2) *reinterpret_cast<double2 *>(o + i) = make_double2(v[i], v[i + 1]);
+    } else {
+        o[0] = v[0];
+#pragma unroll
+        for (int i = 1; i < 17; i += 2) *reinterpret_cast<double2 *>(o + i) = make_double2(v[i], v[i + 1]);
+        o[17] = v[17];
+    }
+}
+
+// What bounds it: the FP64 pipe without contraction (a product and a sum are
+// two instructions).  A pair of nodes takes 48 of them per point, the nine
+// products of column node j with the moduli 9 more, which a 2 x 2 tile shares
+// between its two rows; a tile reads 13 values for four pairs where a thread
+// per pair read 7 for one.  Stage A keeps its 1-D rows once per element and
+// no numerators, so the 64 points of a p=3 element take 110 KB and two CTAs
+// share an SM.  Rows and columns go out in whole lines; written by the
+// pairs' threads, 36 bytes apart, each 4-byte store was an L2 transaction.
+// Measured on B200 against a thread per pair with one CTA per SM: 16^3 elements
+// of p=3 3.33 -> 2.16 ms (1.5 ms is the pipe's time at the highest clock), of
+// p=2 372 -> 301 us, 8^3 of p=4 2.90 -> 2.47 ms.
+__global__ void __launch_bounds__(512)
 k_u1_stiffness(StiffArgs a) {
-    extern __shared__ double smem[];
-    const int nn = a.nn;
+    extern __shared__ __align__(16) double smem[];
+    const int nn = a.nn, nnp = pad2(nn), ds = stiff_ds(nn);
     double *xe = smem;                      // 3*nn element CP coordinates
-    double *we = xe + 3 * nn;               // nn element weights
-    double *B1 = we + nn;                   // qchunk * 6 * kMaxDeg1
-    double *R0 = B1 + (size_t)a.qchunk * 6 * kMaxDeg1;   // qchunk * nn
-    double *dR = R0 + (size_t)a.qchunk * nn;             // qchunk * nn * 3
-    double *qs = dR + (size_t)a.qchunk * nn * 3;         // qchunk * kStiffQS
+    double *we = xe + 3 * nnp;              // nn element weights
+    double *rows = we + nnp;                // 1-D rows
+    int *nodes = reinterpret_cast<int *>(rows + pad2(basis_rows_doubles(a.ng)));
+    int *dof = nodes + nn;                  // first dof of each node
+    double *dR = smem + stiff_fixed(nn, a.ng);           // qchunk * ds
+    double *qs = dR + (size_t)a.qchunk * ds;             // qchunk * kStiffQS
     __shared__ double su1[3], su2[3];
     __shared__ int sni[3];
     const int e = blockIdx.x;
@@ -389,6 +466,7 @@ k_u1_stiffness(StiffArgs a) {
         xe[3 * i + 1] = a.coords[3 * cp + 1];
         xe[3 * i + 2] = a.coords[3 * cp + 2];
         we[i] = a.w[(size_t)e * nn + i];
+        dof[i] = 3 * cp;
     }
     if (tid < 3) {
         const double *U = tid == 0 ? a.U0 : (tid == 1 ? a.U1 : a.U2);
@@ -397,99 +475,135 @@ k_u1_stiffness(StiffArgs a) {
         su1[tid] = U[ni - 1];
         su2[tid] = U[ni];
     }
-    const int npairs = nn * (nn + 1) / 2;
+    const int nt = nnp / 2, ntiles = nt * (nt + 1) / 2;
     const int64_t base = a.slot[e];
     const double lam = a.lam, mu = a.mu, l2m = lam + 2.0 * mu;
     const int pd[3] = {a.p0, a.p1, a.p2};
     const double *Ud[3] = {a.U0, a.U1, a.U2};
+    __syncthreads();
+    basis_rows(pd, Ud, sni, su1, su2, a.gauss, a.ng, nn, rows, nodes);
+    for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+        a.krow[o] = dof[i] + kk;
+        a.kcol[o] = dof[j] + ll;
+    });
     for (int q0 = 0; q0 < a.nq; q0 += a.qchunk) {
         const int nqc = min(a.qchunk, a.nq - q0);
-        __syncthreads();
+        __syncthreads();   // the last chunk's values are used up
         // ---- stage A: basis derivatives at the chunk's Gauss points
-        basis_chunk(pd, Ud, sni, su1, su2, a.gauss, q0, nqc, nn, xe, we, B1, R0, nn, dR, 3 * nn, qs);
-        // A6: inverse Jacobian and the point's weight
-        for (int ql = tid; ql < nqc; ql += nth) {
+        basis_chunk(pd, rows, nodes, a.ng, q0, nqc, nn, xe, we, nullptr, 0, dR, ds, qs, kStiffQS);
+        // A5: the inverse Jacobian, an entry per thread (each forms the
+        // determinant), and the point's weight.  The entries take the slots
+        // of the sums, which are used up, and the spare ones
+        for (int t = tid; t < 10 * nqc; t += nth) {
+            const int rc = t / nqc, ql = t - rc * nqc;
             double *sq = qs + (size_t)ql * kStiffQS;
-            double J[3][3], Ji[3][3];
+            double J[3][3];
             for (int r = 0; r < 3; r++)
                 for (int c = 0; c < 3; c++) J[r][c] = sq[4 + 3 * r + c];
-            inv3(J, Ji);
-            sq[13] = a.gauss[4 * (q0 + ql)] * fabs(parent_det(J, su1, su2));
-            for (int r = 0; r < 3; r++)
-                for (int c = 0; c < 3; c++) sq[4 + 3 * r + c] = Ji[r][c];
+            if (rc == 9) sq[13] = a.gauss[4 * (q0 + ql)] * fabs(parent_det(J, su1, su2));
+            else sq[inv_slot(rc)] = inv3_entry(J, rc);
         }
         __syncthreads();
-        // A7: physical gradients dR/dx, one thread per (point, node)
-        for (int t = tid; t < nqc * nn; t += nth) {
-            const int ql = t / nn, n = t - ql * nn;
-            const double *Ji = qs + (size_t)ql * kStiffQS + 4;
-            double *d = dR + ((size_t)ql * nn + n) * 3;
-            const double d0 = d[0], d1 = d[1], d2 = d[2];
-            for (int c = 0; c < 3; c++) d[c] = d0 * Ji[c] + d1 * Ji[3 + c] + d2 * Ji[6 + c];
+        // A6: physical gradients dR/dx, a warp per point; the padding node's
+        // are zero
+        for (int ql = tid >> 5; ql < nqc; ql += nth >> 5) {
+            double Ji[9];
+#pragma unroll
+            for (int c = 0; c < 9; c++) Ji[c] = qs[(size_t)ql * kStiffQS + inv_slot(c)];
+            for (int n = tid & 31; n < nnp; n += 32) {
+                double *d = dR + (size_t)ql * ds + 3 * n;
+                const double d0 = d[0], d1 = d[1], d2 = d[2];
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+                    d[c] = n == nn ? 0.0 : d0 * Ji[c] + d1 * Ji[3 + c] + d2 * Ji[6 + c];
+            }
         }
         __syncthreads();
-        // ---- stage B: one thread per control-point pair (i <= j)
-        for (int t = tid; t < npairs; t += blockDim.x) {
-            int j = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-            while (j * (j + 1) / 2 > t) j--;
-            while ((j + 1) * (j + 2) / 2 <= t) j++;
-            const int i = t - j * (j + 1) / 2;
-            const int64_t jb = base + 9LL * j * (j - 1) / 2 + 6LL * j;
-            double K[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        // ---- stage B: one thread per 2 x 2 tile of pairs (i <= j)
+        for (int t = tid; t < ntiles; t += nth) {
+            int ti, tj;
+            tile_of(t, ti, tj);
+            // K[jj][9 ii + 3 l + k]: component (k, l) of pair (2 ti + ii, 2 tj + jj)
+            double K[2][18];
+#pragma unroll
+            for (int jj = 0; jj < 2; jj++)
+#pragma unroll
+                for (int c = 0; c < 18; c++) K[jj][c] = 0.0;
             if (q0 > 0) {
                 // resume the running sums of the earlier chunks (the stored
                 // diagonal of a diagonal block is halved; x2 is exact), so the
                 // points are added in one sequence as in the reference
-                if (i < j) {
-                    for (int ll = 0; ll < 3; ll++)
-                        for (int kk = 0; kk < 3; kk++) K[kk][ll] = a.kdata[jb + 9LL * i + 3 * ll + kk];
-                } else {
-                    for (int ll = 0; ll < 3; ll++)
-                        for (int kk = 0; kk <= ll; kk++) {
-                            const double v = a.kdata[jb + 9LL * j + ll * (ll + 1) / 2 + kk];
-                            K[kk][ll] = kk == ll ? v * 2.0 : v;
-                        }
+#pragma unroll
+                for (int jj = 0; jj < 2; jj++)
+#pragma unroll
+                    for (int ii = 0; ii < 2; ii++) {
+                        const int i = 2 * ti + ii, j = 2 * tj + jj;
+                        if (j >= nn || i > j) continue;
+                        const double *o = a.kdata + base + slot_col(j) + 9LL * i;
+#pragma unroll
+                        for (int ll = 0; ll < 3; ll++)
+#pragma unroll
+                            for (int kk = 0; kk < 3; kk++) {
+                                if (i < j) K[jj][9 * ii + 3 * ll + kk] = o[3 * ll + kk];
+                                else if (kk <= ll) {
+                                    const double v = o[ll * (ll + 1) / 2 + kk];
+                                    K[jj][9 * ii + 3 * ll + kk] = kk == ll ? v * 2.0 : v;
+                                }
+                            }
+                    }
+            }
+            const double2 *A = reinterpret_cast<const double2 *>(dR + 6 * ti);
+            const double2 *B = reinterpret_cast<const double2 *>(dR + 6 * tj);
+            for (int q = 0; q < nqc; q++, A += ds / 2, B += ds / 2) {
+                const double2 A0 = A[0], A1 = A[1], A2 = A[2], B0 = B[0], B1 = B[1], B2 = B[2];
+                const double av[2][3] = {{A0.x, A0.y, A1.x}, {A1.y, A2.x, A2.y}};
+                const double bv[2][3] = {{B0.x, B0.y, B1.x}, {B1.y, B2.x, B2.y}};
+                const double d = qs[(size_t)q * kStiffQS + 13];
+#pragma unroll
+                for (int jj = 0; jj < 2; jj++) {
+                    const double b0 = bv[jj][0], b1 = bv[jj][1], b2 = bv[jj][2];
+                    const double m0 = mu * b0, m1 = mu * b1, m2 = mu * b2;
+                    const double l0 = lam * b0, l1 = lam * b1, l2 = lam * b2;
+                    const double h0 = l2m * b0, h1 = l2m * b1, h2 = l2m * b2;
+#pragma unroll
+                    for (int ii = 0; ii < 2; ii++) {
+                        const double a0 = av[ii][0], a1 = av[ii][1], a2 = av[ii][2];
+                        double *k = K[jj] + 9 * ii;
+                        // B_i^T D B_j for isotropic D (stiffmatrix.F90:167-216)
+                        k[0] += (a0 * h0 + a1 * m1 + a2 * m2) * d;
+                        k[4] += (a1 * h1 + a0 * m0 + a2 * m2) * d;
+                        k[8] += (a2 * h2 + a0 * m0 + a1 * m1) * d;
+                        k[3] += (a0 * l1 + a1 * m0) * d;
+                        k[1] += (a1 * l0 + a0 * m1) * d;
+                        k[6] += (a0 * l2 + a2 * m0) * d;
+                        k[2] += (a2 * l0 + a0 * m2) * d;
+                        k[7] += (a1 * l2 + a2 * m1) * d;
+                        k[5] += (a2 * l1 + a1 * m2) * d;
+                    }
                 }
             }
-            for (int q = 0; q < nqc; q++) {
-                const double *A = dR + ((size_t)q * nn + i) * 3;
-                const double *B = dR + ((size_t)q * nn + j) * 3;
-                const double a0 = A[0], a1 = A[1], a2 = A[2];
-                const double b0 = B[0], b1 = B[1], b2 = B[2];
-                const double d = qs[(size_t)q * kStiffQS + 13];
-                // B_i^T D B_j for isotropic D (stiffmatrix.F90:167-216)
-                K[0][0] += (a0 * (l2m * b0) + a1 * (mu * b1) + a2 * (mu * b2)) * d;
-                K[1][1] += (a1 * (l2m * b1) + a0 * (mu * b0) + a2 * (mu * b2)) * d;
-                K[2][2] += (a2 * (l2m * b2) + a0 * (mu * b0) + a1 * (mu * b1)) * d;
-                K[0][1] += (a0 * (lam * b1) + a1 * (mu * b0)) * d;
-                K[1][0] += (a1 * (lam * b0) + a0 * (mu * b1)) * d;
-                K[0][2] += (a0 * (lam * b2) + a2 * (mu * b0)) * d;
-                K[2][0] += (a2 * (lam * b0) + a0 * (mu * b2)) * d;
-                K[1][2] += (a1 * (lam * b2) + a2 * (mu * b1)) * d;
-                K[2][1] += (a2 * (lam * b1) + a1 * (mu * b2)) * d;
-            }
-            const int dofi = 3 * ien[i], dofj = 3 * ien[j];
-            if (i < j) {
-                const int64_t s = jb + 9LL * i;
+#pragma unroll
+            for (int jj = 0; jj < 2; jj++) {
+                const int j = 2 * tj + jj;
+                if (j >= nn) continue;
+                double *o = a.kdata + base + slot_col(j) + 18LL * ti;
+                if (ti < tj) {
+                    store18(o, K[jj]);
+                    continue;
+                }
+                // the diagonal tile: (i, j) of the second column, then a
+                // diagonal block, its upper triangle with the diagonal halved
+                if (jj == 1) {
+#pragma unroll
+                    for (int c = 0; c < 9; c++) o[c] = K[1][c];
+                    o += 9;
+                }
+#pragma unroll
                 for (int ll = 0; ll < 3; ll++)
-                    for (int kk = 0; kk < 3; kk++) {
-                        const int64_t o = s + 3 * ll + kk;
-                        a.kdata[o] = K[kk][ll];
-                        if (q0 == 0) {
-                            a.krow[o] = dofi + kk;
-                            a.kcol[o] = dofj + ll;
-                        }
-                    }
-            } else {
-                const int64_t s = jb + 9LL * j;
-                for (int ll = 0; ll < 3; ll++)
+#pragma unroll
                     for (int kk = 0; kk <= ll; kk++) {
-                        const int64_t o = s + ll * (ll + 1) / 2 + kk;
-                        a.kdata[o] = (kk == ll) ? K[kk][ll] * 0.5 : K[kk][ll];
-                        if (q0 == 0) {
-                            a.krow[o] = dofj + kk;
-                            a.kcol[o] = dofj + ll;
-                        }
+                        const double v = K[jj][9 * jj + 3 * ll + kk];
+                        o[ll * (ll + 1) / 2 + kk] = kk == ll ? v * 0.5 : v;
                     }
             }
         }
@@ -501,10 +615,10 @@ k_u1_stiffness(StiffArgs a) {
 // with, per Gauss point, R and dvol = rho (w_q DetJac) (DetJac signed, as
 // shap returns it) in shared memory; one thread per node pair (i <= j)
 // accumulates (dvol R_j) R_i over the points in order onto the diagonal of
-// the 3x3 block and writes the block into the pair's COO slots (diagonal of
+// the 3x3 block, and the blocks go into the pairs' COO slots (diagonal of
 // the diagonal blocks halved, off-diagonal entries 0).
 struct MassArgs {
-    int p0, p1, p2, nn, nq, qchunk;
+    int p0, p1, p2, nn, nq, ng, qchunk, staged;
     const double *U0, *U1, *U2;
     const double *gauss;
     const double *coords;
@@ -517,15 +631,27 @@ struct MassArgs {
     int32_t *mrow, *mcol;
 };
 
+// What bounds it: the stores (16 bytes a slot against three FP64 operations
+// per pair and point).  With `staged` the pairs' sums stay in shared memory
+// over the chunks and are written as whole lines by consecutive threads;
+// elements whose pairs do not fit (more than kMassStaged bytes, degree 5 on)
+// write from the pairs' threads, 72 bytes apart.  13x9x11 elements of p=3 577 ->
+// 220 us (the stores alone 58 us at the copy rate; the rest is stage A's chain
+// of short steps), 16^3 of p=2 272 -> 137 us.
+constexpr size_t kMassStaged = 64 * 1024;
+
 __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
-    extern __shared__ double smem[];
-    const int nn = a.nn;
+    extern __shared__ __align__(16) double smem[];
+    const int nn = a.nn, nnp = pad2(nn), ds = stiff_ds(nn);
     double *xe = smem;                          // 3*nn element CP coordinates
-    double *we = xe + 3 * nn;                   // nn element weights
-    double *B1 = we + nn;                       // qchunk * 6 * kMaxDeg1
-    double *Rq = B1 + (size_t)a.qchunk * 6 * kMaxDeg1;   // qchunk * nn basis values
-    double *dR = Rq + (size_t)a.qchunk * nn;             // qchunk * nn * 3 (dR/dxi)
-    double *qs = dR + (size_t)a.qchunk * nn * 3;         // qchunk * kStiffQS
+    double *we = xe + 3 * nnp;                  // nn element weights
+    double *rows = we + nnp;                    // 1-D rows
+    int *nodes = reinterpret_cast<int *>(rows + pad2(basis_rows_doubles(a.ng)));
+    int *dof = nodes + nn;                  // first dof of each node
+    double *Rq = smem + stiff_fixed(nn, a.ng);           // qchunk * nnp basis values
+    double *dR = Rq + (size_t)a.qchunk * nnp;            // qchunk * ds (dR/dxi)
+    double *qs = dR + (size_t)a.qchunk * ds;             // qchunk * kMassQS
+    double *ms = qs + (size_t)a.qchunk * kMassQS;       // staged: pair sums
     __shared__ double su1[3], su2[3];
     __shared__ int sni[3];
     const int e = blockIdx.x;
@@ -537,6 +663,7 @@ __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
         xe[3 * i + 1] = a.coords[3 * cp + 1];
         xe[3 * i + 2] = a.coords[3 * cp + 2];
         we[i] = a.w[(size_t)e * nn + i];
+        dof[i] = 3 * cp;
     }
     if (tid < 3) {
         const double *U = tid == 0 ? a.U0 : (tid == 1 ? a.U1 : a.U2);
@@ -545,21 +672,32 @@ __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
         su1[tid] = U[ni - 1];
         su2[tid] = U[ni];
     }
-    const int npairs = nn * (nn + 1) / 2;
+    const int nt = nnp / 2, ntiles = nt * (nt + 1) / 2;
     const int64_t base = a.slot[e];
     const int pd[3] = {a.p0, a.p1, a.p2};
     const double *Ud[3] = {a.U0, a.U1, a.U2};
+    __syncthreads();
+    basis_rows(pd, Ud, sni, su1, su2, a.gauss, a.ng, nn, rows, nodes);
+    if (!a.staged)
+        for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+            a.mrow[o] = dof[i] + kk;
+            a.mcol[o] = dof[j] + ll;
+            if (kk != ll) a.mdata[o] = 0.0;
+        });
     for (int q0 = 0; q0 < a.nq; q0 += a.qchunk) {
         const int nqc = min(a.qchunk, a.nq - q0);
         __syncthreads();
         // ---- stage A: basis values and dvol at the chunk's Gauss points
-        basis_chunk(pd, Ud, sni, su1, su2, a.gauss, q0, nqc, nn, xe, we, B1, Rq, nn, dR, 3 * nn, qs);
-        for (int t = tid; t < nqc * nn; t += blockDim.x) {
-            const int ql = t / nn;
-            Rq[t] = Rq[t] * qs[(size_t)ql * kStiffQS + 3];
+        basis_chunk(pd, rows, nodes, a.ng, q0, nqc, nn, xe, we, Rq, nnp, dR, ds, qs, kMassQS);
+        for (int ql = tid >> 5; ql < nqc; ql += blockDim.x >> 5) {
+            const double inv = qs[(size_t)ql * kMassQS + 3];
+            for (int n = tid & 31; n < nnp; n += 32) {
+                double &R = Rq[(size_t)ql * nnp + n];
+                R = n < nn ? R * inv : 0.0;
+            }
         }
         for (int ql = tid; ql < nqc; ql += blockDim.x) {
-            double *sq = qs + (size_t)ql * kStiffQS;
+            double *sq = qs + (size_t)ql * kMassQS;
             double J[3][3];
             for (int r = 0; r < 3; r++)
                 for (int c = 0; c < 3; c++) J[r][c] = sq[4 + 3 * r + c];
@@ -567,47 +705,58 @@ __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
             sq[13] = a.rho * dvol;
         }
         __syncthreads();
-        // ---- stage B: one thread per control-point pair (i <= j)
-        for (int t = tid; t < npairs; t += blockDim.x) {
-            int j = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-            while (j * (j + 1) / 2 > t) j--;
-            while ((j + 1) * (j + 2) / 2 <= t) j++;
-            const int i = t - j * (j + 1) / 2;
-            const int64_t jb = base + 9LL * j * (j - 1) / 2 + 6LL * j;
-            // resume the running sum of the earlier chunks (a diagonal
+        // ---- stage B: one thread per 2 x 2 tile of pairs (i <= j)
+        for (int t = tid; t < ntiles; t += blockDim.x) {
+            int ti, tj;
+            tile_of(t, ti, tj);
+            double m[2][2] = {{0.0, 0.0}, {0.0, 0.0}};   // [jj][ii]
+            auto each = [&](auto visit) {
+#pragma unroll
+                for (int jj = 0; jj < 2; jj++)
+#pragma unroll
+                    for (int ii = 0; ii < 2; ii++) {
+                        const int i = 2 * ti + ii, j = 2 * tj + jj;
+                        if (j < nn && i <= j) visit(m[jj][ii], i, j);
+                    }
+            };
+            // resume the running sums of the earlier chunks (a diagonal
             // block's stored value is halved; x2 is exact)
-            double m = 0.0;
-            if (q0 > 0) m = i < j ? a.mdata[jb + 9LL * i] : a.mdata[jb + 9LL * j] * 2.0;
+            if (q0 > 0)
+                each([&](double &v, int i, int j) {
+                    if (a.staged) v = ms[j * (j + 1) / 2 + i];
+                    else v = a.mdata[base + slot_col(j) + 9LL * i] * (i < j ? 1.0 : 2.0);
+                });
             for (int q = 0; q < nqc; q++) {
-                const double t1 = qs[(size_t)q * kStiffQS + 13] * Rq[(size_t)q * nn + j];
-                m += t1 * Rq[(size_t)q * nn + i];
+                const double2 ri = *reinterpret_cast<const double2 *>(Rq + (size_t)q * nnp + 2 * ti);
+                const double2 rj = *reinterpret_cast<const double2 *>(Rq + (size_t)q * nnp + 2 * tj);
+                const double d = qs[(size_t)q * kMassQS + 13];
+                const double t0 = d * rj.x, t1 = d * rj.y;
+                m[0][0] += t0 * ri.x;
+                m[0][1] += t0 * ri.y;
+                m[1][0] += t1 * ri.x;
+                m[1][1] += t1 * ri.y;
             }
-            const int dofi = 3 * ien[i], dofj = 3 * ien[j];
-            if (i < j) {
-                const int64_t s = jb + 9LL * i;
-                for (int ll = 0; ll < 3; ll++)
-                    for (int kk = 0; kk < 3; kk++) {
-                        const int64_t o = s + 3 * ll + kk;
-                        a.mdata[o] = kk == ll ? m : 0.0;
-                        if (q0 == 0) {
-                            a.mrow[o] = dofi + kk;
-                            a.mcol[o] = dofj + ll;
-                        }
-                    }
-            } else {
-                const int64_t s = jb + 9LL * j;
-                for (int ll = 0; ll < 3; ll++)
-                    for (int kk = 0; kk <= ll; kk++) {
-                        const int64_t o = s + ll * (ll + 1) / 2 + kk;
-                        a.mdata[o] = kk == ll ? m * 0.5 : 0.0;
-                        if (q0 == 0) {
-                            a.mrow[o] = dofj + kk;
-                            a.mcol[o] = dofj + ll;
-                        }
-                    }
-            }
+            each([&](double &v, int i, int j) {
+                if (a.staged) {
+                    ms[j * (j + 1) / 2 + i] = v;
+                    return;
+                }
+                double *o = a.mdata + base + slot_col(j) + 9LL * i;
+                for (int ll = 0; ll < 3; ll++) {
+                    if (i < j) o[4 * ll] = v;
+                    else o[ll * (ll + 1) / 2 + ll] = v * 0.5;
+                }
+            });
         }
     }
+    if (!a.staged) return;
+    __syncthreads();
+    for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+        const double v = ms[j * (j + 1) / 2 + i];
+        a.mdata[o] = kk != ll ? 0.0 : i < j ? v : v * 0.5;
+        a.mrow[o] = dof[i] + kk;
+        a.mcol[o] = dof[j] + ll;
+    });
 }
 
 // Distributed loads (UELMAT.f90:121-223), deterministic and in the reference's
@@ -818,6 +967,10 @@ __global__ void k_u1_rhs_gather(int64_t ndof, const int64_t *ptr,
     F[dof] = acc;
 }
 
+// Shared memory of a CTA when n share an SM (228 KB, 1 KB of it reserved per
+// CTA, and the kernels' static arrays).
+constexpr size_t sm_share(int n) { return 228 * 1024 / n - 1536; }
+
 static bool in_list(const int64_t *l, int64_t n, int64_t v) {
     for (int64_t i = 0; i < n; i++)
         if (l[i] == v) return true;
@@ -908,14 +1061,19 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
     for (size_t ip = 0; ip < M.patches.size(); ip++) {
         U1Patch &P = M.patches[ip];
         if (!P.nactive) continue;
-        const size_t fixed = sizeof(double) * 4 * P.nn;
+        const size_t fixed = sizeof(double) * stiff_fixed(P.nn, P.ng);
         const size_t perq = sizeof(double) * stiff_perq(P.nn);
         YETI_CHECK(fixed + perq <= smem_cap, YETI_EUNSUPPORTED,
                    "element with %d nodes does not fit shared memory", P.nn);
         int qchunk = (int)std::min<size_t>(P.nq, (smem_cap - fixed) / perq);
+        // a thread per tile: 256 where several CTAs share an SM (their
+        // points fit half of its memory), else 512 of the one CTA
+        const int nt = pad2(P.nn) / 2, ntiles = nt * (nt + 1) / 2;
+        const int most = fixed + perq * qchunk <= sm_share(2) ? 256 : 512;
+        const int threads = std::min(most, std::max(64, (ntiles + 31) / 32 * 32));
         StiffArgs a;
         a.p0 = P.p[0]; a.p1 = P.p[1]; a.p2 = P.p[2];
-        a.nn = P.nn; a.nq = P.nq; a.qchunk = qchunk;
+        a.nn = P.nn; a.nq = P.nq; a.ng = P.ng; a.qchunk = qchunk;
         a.U0 = P.knots.as<double>();
         a.U1 = a.U0 + P.nkv[0];
         a.U2 = a.U1 + P.nkv[1];
@@ -939,7 +1097,7 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
                 int64_t n = std::min<int64_t>(left, 1 << 30);
                 StiffArgs b = a;
                 b.ien += off * P.nn; b.w += off * P.nn; b.span += off * 3; b.slot += off;
-                k_u1_stiffness<<<(unsigned)n, 256, smem, ctx->stream>>>(b);
+                k_u1_stiffness<<<(unsigned)n, threads, smem, ctx->stream>>>(b);
                 count_launches(1);
                 YETI_CUDA(cudaGetLastError());
                 left -= n; off += n;
@@ -1137,14 +1295,23 @@ YETI_API int yeti_assemble_u1_mass_coo(yeti_ctx *ctx, const yeti_u1_model *m,
     for (size_t ip = 0; ip < M.patches.size(); ip++) {
         U1Patch &P = M.patches[ip];
         if (!P.nactive) continue;
-        const size_t fixed = sizeof(double) * 4 * P.nn;
-        const size_t perq = sizeof(double) * stiff_perq(P.nn);
+        const size_t pairs = sizeof(double) * ((size_t)P.nn * (P.nn + 1) / 2);
+        const bool staged = pairs <= kMassStaged;
+        const size_t fixed = sizeof(double) * stiff_fixed(P.nn, P.ng) + (staged ? pairs : 0);
+        const size_t perq = sizeof(double) * mass_perq(P.nn);
         YETI_CHECK(fixed + perq <= smem_cap, YETI_EUNSUPPORTED,
                    "element with %d nodes does not fit shared memory", P.nn);
-        const int qchunk = (int)std::min<size_t>(P.nq, (smem_cap - fixed) / perq);
+        // points per chunk: staged sums cost nothing between chunks, and
+        // stage A is a chain of short steps, so the chunk is cut for four
+        // CTAs per SM where that leaves it eight points, else for two
+        size_t cap = smem_cap;
+        if (staged && fixed + perq <= sm_share(2)) cap = sm_share(2);
+        if (staged && fixed + 8 * perq <= sm_share(4)) cap = sm_share(4);
+        const int most = (int)std::min<size_t>(P.nq, (cap - fixed) / perq);
+        const int qchunk = (P.nq + (P.nq + most - 1) / most - 1) / ((P.nq + most - 1) / most);
         MassArgs a;
         a.p0 = P.p[0]; a.p1 = P.p[1]; a.p2 = P.p[2];
-        a.nn = P.nn; a.nq = P.nq; a.qchunk = qchunk;
+        a.nn = P.nn; a.nq = P.nq; a.ng = P.ng; a.qchunk = qchunk; a.staged = staged;
         a.U0 = P.knots.as<double>();
         a.U1 = a.U0 + P.nkv[0];
         a.U2 = a.U1 + P.nkv[1];

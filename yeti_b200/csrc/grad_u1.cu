@@ -121,14 +121,14 @@ __host__ __device__ inline PtLayout pt_layout(int nn, int nadj, int nbody) {
 
 // Shared memory of one element: xe, ue, uae, we, then the point records
 // (PtLayout) of one chunk of pchunk points, then the basis scratch
-// (kBasisB1 + kStiffQS per point of the chunk), the external- and
+// (1-D rows, node indices, kBasisQS per point of the chunk), the external- and
 // internal-work accumulators of the (control point, component) tasks and
 // the term buffer of stage B (qchunk points).
 __host__ __device__ inline size_t grad_smem_doubles(int nn, int pchunk, int nadj, const PtLayout &L,
-                                                    size_t face, int qchunk) {
+                                                    size_t face, int qchunk, int ng) {
     const size_t vol = (size_t)pchunk * L.size;
     return (size_t)(6 + 3 * nadj) * nn + nn + (vol > face ? vol : face) +
-           (size_t)pchunk * (kBasisB1 + kStiffQS) + (size_t)2 * 3 * nn * nadj +
+           basis_rows_doubles(ng) + (nn + 1) / 2 + (size_t)pchunk * kBasisQS + (size_t)2 * 3 * nn * nadj +
            (size_t)3 * nn * qchunk * 3 * nadj;
 }
 
@@ -185,14 +185,18 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
     const size_t face = (size_t)a.ng * a.ng * (4 * nn + 11 + 3 * nadj);
     const int pc = a.pchunk;
     const size_t vol = (size_t)pc * L.size;
-    double *B1 = pts + (vol > face ? vol : face);
-    double *qs = B1 + (size_t)pc * kBasisB1;
-    double *ge_s = qs + (size_t)pc * kStiffQS;
+    double *rows = pts + (vol > face ? vol : face);
+    int *nodes = reinterpret_cast<int *>(rows + basis_rows_doubles(a.ng));
+    double *qs = rows + basis_rows_doubles(a.ng) + (nn + 1) / 2;
+    double *ge_s = qs + (size_t)pc * kBasisQS;
     double *gi_s = ge_s + (size_t)3 * nn * nadj;   // 3 nn nadj accumulators
     double *terms = gi_s + (size_t)3 * nn * nadj;  // 3 nn qchunk 3 nadj terms
     const double lambda = a.E * a.nu / (1.0 + a.nu) / (1.0 - 2.0 * a.nu);
     const double mu = a.E / 2.0 / (1.0 + a.nu);
     for (int t = tid; t < 3 * nn * nadj; t += nth) gi_s[t] = ge_s[t] = 0.0;
+    const int pd[3] = {a.p0, a.p1, a.p2};
+    const double *Ud[3] = {a.U0, a.U1, a.U2};
+    basis_rows(pd, Ud, sni, su1, su2, a.gauss, a.ng, nn, rows, nodes);
     // The points are taken in chunks of pc (their records in shared memory);
     // every accumulator continues over the chunks in point order, so the
     // sums are the same sequences as over all points at once.
@@ -200,17 +204,13 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
         const int np = min(pc, a.nq - p0);
         __syncthreads();
         // ---------------- stage A: per volume point of the chunk
-        {
-            const int pd[3] = {a.p0, a.p1, a.p2};
-            const double *Ud[3] = {a.U0, a.U1, a.U2};
-            // R numerators and dR/dxi into the point records, dx/dxi into qs
-            basis_chunk(pd, Ud, sni, su1, su2, a.gauss, p0, np, nn, xe, we, B1, pts + L.R, L.size,
-                        pts + L.dR, L.size, qs);
-        }
+        // R numerators and dR/dxi into the point records, dx/dxi into qs
+        basis_chunk(pd, rows, nodes, a.ng, p0, np, nn, xe, we, pts + L.R, L.size, pts + L.dR, L.size,
+                    qs, kBasisQS);
         for (int t = tid; t < np * nn; t += nth) {
             const int q = t / nn, n = t - q * nn;
             double *R = pts + (size_t)q * L.size + L.R;
-            R[n] = R[n] * qs[(size_t)q * kStiffQS + 3];
+            R[n] = R[n] * qs[(size_t)q * kBasisQS + 3];
         }
         if (a.compute_int) {
             // the gradients of the state and of the adjoints: ordered sums over
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
             const double *R = P + L.R;
             double AI[3][3];
             for (int i = 0; i < 3; i++)
-                for (int c = 0; c < 3; c++) AI[i][c] = qs[(size_t)q * kStiffQS + 4 + 3 * c + i];
+                for (int c = 0; c < 3; c++) AI[i][c] = qs[(size_t)q * kBasisQS + 4 + 3 * c + i];
             double AxA[3][3];
             gcross(AI[0], AI[1], AxA[2]);
             const double Area = gdot(AxA[2], AI[2]);
@@ -733,11 +733,11 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         // chunk that does (at least the term buffer's)
         int pchunk = P.nq;
         while (pchunk > qchunk &&
-               sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, qchunk) > (size_t)smem_optin)
+               sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, qchunk, P.ng) > (size_t)smem_optin)
             pchunk--;
         g.qchunk = std::min(qchunk, pchunk);
         g.pchunk = pchunk;
-        const size_t smem = sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, g.qchunk);
+        const size_t smem = sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, g.qchunk, P.ng);
         YETI_CHECK(smem <= (size_t)smem_optin, YETI_EUNSUPPORTED,
                    "shape gradient: element needs %zu bytes of shared memory", smem);
         YETI_TRY(set_smem_optin((const void *)k_u1_grad, ctx->device, smem, "shape gradient element"));
