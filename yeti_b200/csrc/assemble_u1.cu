@@ -172,6 +172,7 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
     out.patches.clear();
     out.patches.resize(m->nb_patch);
     out.nb_cp = m->nb_cp;
+    UploadPack pack;
     int64_t jelem = 0, ukv_off = 0, ien_off = 0, count = 0;
     for (int64_t ip = 0; ip < m->nb_patch; ip++) {
         U1Patch &P = out.patches[ip];
@@ -182,10 +183,9 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
         P.nelem = m->nb_elem_patch[ip];
         P.elem_begin = jelem;
         P.nn = (int)m->nnode[ip];
-        bool any_active = false;
-        for (int64_t e = 0; e < P.nelem; e++)
-            if (m->active[jelem + e] == 1) any_active = true;
-        if (any_active) {
+        int64_t nact = 0;
+        for (int64_t e = 0; e < P.nelem; e++) nact += m->active[jelem + e] == 1;
+        if (nact) {
             YETI_CHECK(!m->is_u1 || m->is_u1[ip], YETI_EUNSUPPORTED,
                        "patch %lld: only U1/THREED solid elements are on this "
                        "path", (long long)ip + 1);
@@ -213,10 +213,14 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
         P.rho = m->rho ? m->rho[ip] : 0.0;
         P.nb_data_elem = 9LL * P.nn * (P.nn - 1) / 2 + 6LL * P.nn;
         const int nn = P.nn;
-        std::vector<int32_t> ien, span, gid;
-        std::vector<double> w;
+        std::vector<int32_t> ien(nact * nn), span(nact * 3), gid;
+        std::vector<double> w(nact * nn);
+        P.act.reserve(nact);
+        P.slot.reserve(nact);
+        gid.reserve(nact);
         for (int64_t e = 0; e < P.nelem; e++, jelem++) {
             if (m->active[jelem] != 1) continue;
+            const int64_t k = (int64_t)P.act.size();
             P.act.push_back(jelem);
             P.slot.push_back(count);
             count += P.nb_data_elem;
@@ -226,29 +230,29 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
                 YETI_CHECK(cp >= 1 && cp <= m->nb_cp, YETI_EINVAL,
                            "IEN entry %lld of element %lld out of range",
                            (long long)cp, (long long)jelem + 1);
-                ien.push_back((int32_t)(cp - 1));
-                w.push_back(m->weight[ien_off + e * nn + a]);
+                ien[k * nn + a] = (int32_t)(cp - 1);
+                w[k * nn + a] = m->weight[ien_off + e * nn + a];
             }
             for (int d = 0; d < 3; d++) {
                 int64_t ni = m->nijk[3 * jelem + d];
                 YETI_CHECK(ni >= P.p[d] + 1 && ni <= P.nkv[d] - P.p[d] - 1,
                            YETI_EINVAL, "Nijk of element %lld out of range",
                            (long long)jelem + 1);
-                span.push_back((int32_t)ni);
+                span[k * 3 + d] = (int32_t)ni;
             }
         }
         P.nactive = (int64_t)P.act.size();
         int nk = P.nkv[0] + P.nkv[1] + P.nkv[2];
         if (P.nactive) {
-            YETI_TRY(upload(ctx, P.knots, m->ukv + ukv_off, nk));
+            pack.add(P.knots, m->ukv + ukv_off, nk);
             std::vector<double> g;
             gauss_volume_host(P.ng, g);
-            YETI_TRY(upload(ctx, P.gauss, g.data(), g.size()));
-            YETI_TRY(upload(ctx, P.ien, ien.data(), ien.size()));
-            YETI_TRY(upload(ctx, P.w, w.data(), w.size()));
-            YETI_TRY(upload(ctx, P.span, span.data(), span.size()));
-            YETI_TRY(upload(ctx, P.slotd, P.slot.data(), P.slot.size()));
-            YETI_TRY(upload(ctx, P.gid, gid.data(), gid.size()));
+            pack.add(P.gauss, g);
+            pack.add(P.ien, ien);
+            pack.add(P.w, w);
+            pack.add(P.span, span);
+            pack.add(P.slotd, P.slot);
+            pack.add(P.gid, gid);
         }
         ukv_off += nk;
         ien_off += P.nelem * nn;
@@ -257,8 +261,8 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
                "sum of nb_elem_patch (%lld) != nb_elem (%lld)",
                (long long)jelem, (long long)m->nb_elem);
     out.nb_data = count;
-    YETI_TRY(upload(ctx, out.coords, m->coords, (size_t)3 * m->nb_cp));
-    return YETI_OK;
+    pack.add(out.coords, m->coords, (size_t)3 * m->nb_cp);
+    return pack.commit(ctx, out.arena);
 }
 
 // ---------------------------------------------------------------- kernels
@@ -971,12 +975,6 @@ __global__ void k_u1_rhs_gather(int64_t ndof, const int64_t *ptr,
 // CTA, and the kernels' static arrays).
 constexpr size_t sm_share(int n) { return 228 * 1024 / n - 1536; }
 
-static bool in_list(const int64_t *l, int64_t n, int64_t v) {
-    for (int64_t i = 0; i < n; i++)
-        if (l[i] == v) return true;
-    return false;
-}
-
 }  // namespace yeti
 
 using namespace yeti;
@@ -1055,6 +1053,7 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
     std::vector<Loaded> loaded;
     std::vector<PatchRhs> patch_erhs;
     int64_t erhs_total = 0;
+    const LoadMarks marks(m, [](int64_t ty) { return ty == 101 || ty == 102 || (ty > 9 && ty < 100); });
     std::vector<int64_t> ien_offset(M.patches.size(), 0);
     for (size_t ip = 1; ip < M.patches.size(); ip++)
         ien_offset[ip] = ien_offset[ip - 1] + M.patches[ip - 1].nelem * M.patches[ip - 1].nn;
@@ -1109,13 +1108,12 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
         int max_body = 0;
         for (int64_t le = 0; le < P.nactive; le++) {
             const int64_t jel = P.act[le] + 1;   // 1-based element number
-            int64_t k2 = 0, cinfo = 0;
+            int64_t cinfo = 0;
             size_t before = terms.size();
             int nbody = 0;
             for (int64_t il = 0; il < m->nb_load; il++) {
-                int64_t nt = m->load_target_nbelem[il], ty = m->jdltype[il];
-                if ((ty == 101 || ty == 102 || (ty > 9 && ty < 100)) &&
-                    in_list(m->inddload + k2, nt, jel)) {
+                const int64_t ty = m->jdltype[il];
+                if (marks.on(il, jel)) {
                     LoadTerm T;
                     memset(&T, 0, sizeof(T));
                     T.mag = m->adlmag[il];
@@ -1140,7 +1138,6 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
                     }
                     terms.push_back(T);
                 }
-                k2 += nt;
                 cinfo += m->nb_load_addinfos ? m->nb_load_addinfos[il] : 0;
             }
             if (terms.size() > before) {
@@ -1160,19 +1157,18 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
                 gauss_face_host(P.ng, f, tmp);
                 std::copy(tmp.begin(), tmp.end(), gf.begin() + (f - 1) * 4 * P.ng * P.ng);
             }
-            DevBuf &dgf = newbuf();
-            YETI_TRY(upload(ctx, dgf, gf.data(), gf.size()));
-            DevBuf &del = newbuf();
-            YETI_TRY(upload(ctx, del, elems.data(), elems.size()));
-            DevBuf &dtp = newbuf();
-            YETI_TRY(upload(ctx, dtp, tptr.data(), tptr.size()));
-            DevBuf &dtm = newbuf();
-            YETI_TRY(upload(ctx, dtm, terms.data(), terms.size()));
+            DevBuf &arena = newbuf(), &dgf = newbuf(), &del = newbuf(), &dtp = newbuf(), &dtm = newbuf();
+            UploadPack lpack;
+            lpack.add(dgf, gf);
+            lpack.add(del, elems);
+            lpack.add(dtp, tptr);
+            lpack.add(dtm, terms);
             DevBuf *dnd = nullptr;
             if (m->nodal_dist && m->nb_n_dist > 0) {
                 dnd = &newbuf();
-                YETI_TRY(upload(ctx, *dnd, m->nodal_dist, (size_t)m->nb_n_dist * m->nb_cp));
+                lpack.add(*dnd, m->nodal_dist, (size_t)m->nb_n_dist * m->nb_cp);
             }
+            YETI_TRY(lpack.commit(ctx, arena));
             DevBuf &der = newbuf();
             YETI_TRY(der.alloc(ctx, sizeof(double) * 3 * P.nn * elems.size()));
             patch_erhs.push_back({&der, loaded.size() - elems.size()});
@@ -1216,25 +1212,28 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
                                       cudaMemcpyDeviceToDevice, ctx->stream));
             off += (int64_t)(pe.buf->bytes / sizeof(double));
         }
-        std::vector<int64_t> cnt(ndof + 1, 0), idx;
-        std::vector<std::vector<int64_t>> lists(ndof);
-        for (auto &L : loaded) {
-            const U1Patch &P = M.patches[L.patch];
-            const int64_t jel = P.act[L.local];
-            const int64_t ien_base = ien_offset[L.patch] + (jel - P.elem_begin) * P.nn;
-            for (int n = 0; n < P.nn; n++) {
-                int64_t cp = m->ien[ien_base + n] - 1;
-                for (int d = 0; d < 3; d++) lists[3 * cp + d].push_back(L.off + 3 * n + d);
+        // CSR of the element entries of each dof, elements in order: count,
+        // then fill in the same loop order
+        std::vector<int64_t> cnt(ndof + 1, 0);
+        auto walk = [&](auto &&visit) {
+            for (auto &L : loaded) {
+                const U1Patch &P = M.patches[L.patch];
+                const int64_t jel = P.act[L.local];
+                const int64_t ien_base = ien_offset[L.patch] + (jel - P.elem_begin) * P.nn;
+                for (int n = 0; n < P.nn; n++)
+                    for (int d = 0; d < 3; d++)
+                        visit(3 * (m->ien[ien_base + n] - 1) + d, L.off + 3 * n + d);
             }
-        }
-        for (int64_t i = 0; i < ndof; i++) {
-            cnt[i + 1] = cnt[i] + (int64_t)lists[i].size();
-            idx.insert(idx.end(), lists[i].begin(), lists[i].end());
-        }
-        DevBuf &dptr = newbuf();
-        YETI_TRY(upload(ctx, dptr, cnt.data(), cnt.size()));
-        DevBuf &didx = newbuf();
-        YETI_TRY(upload(ctx, didx, idx.data(), idx.size()));
+        };
+        walk([&](int64_t dof, int64_t) { cnt[dof + 1]++; });
+        for (int64_t i = 0; i < ndof; i++) cnt[i + 1] += cnt[i];
+        std::vector<int64_t> idx(cnt[ndof]), fill(cnt.begin(), cnt.end() - 1);
+        walk([&](int64_t dof, int64_t off) { idx[fill[dof]++] = off; });
+        DevBuf &garena = newbuf(), &dptr = newbuf(), &didx = newbuf();
+        UploadPack gpack;
+        gpack.add(dptr, cnt);
+        gpack.add(didx, idx);
+        YETI_TRY(gpack.commit(ctx, garena));
         k_u1_rhs_gather<<<(unsigned)((ndof + 255) / 256), 256, 0, ctx->stream>>>(
             ndof, dptr.as<int64_t>(), didx.as<int64_t>(), dall.as<double>(), f_);
         count_launches(1);

@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
@@ -55,6 +56,22 @@ struct yeti_ctx {
     // allocate with cudaMallocAsync / cudaFreeAsync on `stream` (no implicit
     // device synchronisation; for contexts driven by the serving loop)
     bool stream_ordered = false;
+    // Freed blocks kept for the next allocations (dev_alloc): a call's
+    // scratch costs a list lookup instead of cudaMalloc and cudaFree, which
+    // took 2 to 4 ms of a Gauss call or an operator setup.  Blocks of a size
+    // class are interchangeable; each carries an event recorded on the
+    // context's stream when it was freed, which another stream waits for
+    // before it takes the block.  At most kPoolBytes are kept; they are given
+    // back with the context, and earlier when an allocation fails or the HBM
+    // budget needs the room.
+    struct PoolBlock {
+        void *ptr;
+        cudaEvent_t freed;
+        cudaStream_t stream;   // where `freed` was recorded (identity only)
+    };
+    std::mutex pool_mu;
+    std::multimap<size_t, PoolBlock> pool;
+    size_t pool_bytes = 0;
     // device-time accounting of the element kernels (yeti_ctx_set_timing)
     bool timing = false;
     std::mutex timing_mu;
@@ -63,19 +80,29 @@ struct yeti_ctx {
 
 namespace yeti {
 
-// Device allocation charged against the context budget.
+constexpr size_t kPoolBytes = size_t(256) << 20;   // most a context keeps of freed blocks
+constexpr size_t kPoolBlock = size_t(64) << 20;    // largest block it keeps
+
+// Device allocation charged against the context budget.  A block may come
+// from the context's pool: its last user's work has been enqueued on the
+// context's stream of that time (or is done), so all work on a buffer must
+// be enqueued on the context's stream before the buffer is freed.
 int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes);
 void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes);
+// Give the pool's blocks back to the device.
+void pool_release(yeti_ctx *ctx);
 
-// RAII device buffer owned by a context.
+// RAII device buffer owned by a context, or a view of a part of another one
+// (owned == false).
 struct DevBuf {
     yeti_ctx *ctx = nullptr;
     void *ptr = nullptr;
     size_t bytes = 0;
+    bool owned = true;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : ctx(o.ctx), ptr(o.ptr), bytes(o.bytes) {
+    DevBuf(DevBuf &&o) noexcept : ctx(o.ctx), ptr(o.ptr), bytes(o.bytes), owned(o.owned) {
         o.ptr = nullptr;
         o.bytes = 0;
     }
@@ -85,6 +112,7 @@ struct DevBuf {
             ctx = o.ctx;
             ptr = o.ptr;
             bytes = o.bytes;
+            owned = o.owned;
             o.ptr = nullptr;
             o.bytes = 0;
         }
@@ -98,10 +126,17 @@ struct DevBuf {
         if (rc == YETI_OK) bytes = n;
         return rc;
     }
+    void view(void *p, size_t n) {
+        release();
+        ptr = p;
+        bytes = n;
+        owned = false;
+    }
     void release() {
-        if (ptr) dev_free(ctx, ptr, bytes);
+        if (ptr && owned) dev_free(ctx, ptr, bytes);
         ptr = nullptr;
         bytes = 0;
+        owned = true;
     }
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
@@ -115,6 +150,38 @@ int upload(yeti_ctx *ctx, DevBuf &buf, const T *host, size_t n) {
                                   cudaMemcpyHostToDevice, ctx->stream));
     return YETI_OK;
 }
+
+// Host arrays uploaded together: add() copies them into one host buffer,
+// commit() allocates `arena`, makes one copy and turns the arrays' buffers into
+// views of it (arena must outlive them).
+class UploadPack {
+    struct Item {
+        DevBuf *buf;
+        size_t off, bytes;
+    };
+    std::vector<Item> items;
+    std::vector<char> host;
+
+public:
+    template <class T>
+    void add(DevBuf &buf, const T *data, size_t n) {
+        const size_t off = (host.size() + 255) & ~size_t(255), bytes = n * sizeof(T);
+        host.resize(off + bytes + 16);
+        if (bytes) memcpy(host.data() + off, data, bytes);
+        items.push_back({&buf, off, bytes});
+    }
+    template <class T>
+    void add(DevBuf &buf, const std::vector<T> &v) {
+        add(buf, v.data(), v.size());
+    }
+    int commit(yeti_ctx *ctx, DevBuf &arena) {
+        YETI_TRY(upload(ctx, arena, host.data(), host.size()));
+        for (const Item &it : items) it.buf->view(arena.as<char>() + it.off, it.bytes);
+        items.clear();
+        host.clear();
+        return YETI_OK;
+    }
+};
 
 // Guard that makes ctx->device current for the scope.
 struct DeviceGuard {

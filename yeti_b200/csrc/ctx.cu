@@ -23,6 +23,45 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return YETI_ECUDA;
 }
 
+// Size class of a pooled block: bytes rounded up to an eighth of its power of
+// two (512 bytes at least).
+static size_t pool_class(size_t bytes) {
+    size_t step = 512;
+    while (step * 16 <= bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+}
+
+// The caller holds pool_mu.
+static void pool_release_locked(yeti_ctx *ctx) {
+    for (auto &kv : ctx->pool) {
+        cudaEventDestroy(kv.second.freed);
+        cudaFree(kv.second.ptr);
+    }
+    ctx->pool.clear();
+    ctx->pool_bytes = 0;
+}
+
+void pool_release(yeti_ctx *ctx) {
+    std::lock_guard<std::mutex> lock(ctx->pool_mu);
+    pool_release_locked(ctx);
+}
+
+// A block of the class from the pool, or nullptr.
+static void *pool_take(yeti_ctx *ctx, size_t cls) {
+    std::lock_guard<std::mutex> lock(ctx->pool_mu);
+    auto it = ctx->pool.find(cls);
+    if (it == ctx->pool.end()) return nullptr;
+    const yeti_ctx::PoolBlock b = it->second;
+    if (b.stream != ctx->stream && cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    ctx->pool.erase(it);
+    ctx->pool_bytes -= cls;
+    cudaEventDestroy(b.freed);
+    return b.ptr;
+}
+
 int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) bytes = 16;
@@ -31,8 +70,26 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
                   ctx->bytes_in_use.load(), bytes, ctx->hbm_budget);
         return YETI_ENOMEM;
     }
-    cudaError_t e = ctx->stream_ordered ? cudaMallocAsync(ptr, bytes, ctx->stream)
-                                        : cudaMalloc(ptr, bytes);
+    cudaError_t e = cudaSuccess;
+    if (ctx->stream_ordered) {
+        e = cudaMallocAsync(ptr, bytes, ctx->stream);
+    } else {
+        const size_t cls = pool_class(bytes);
+        *ptr = pool_take(ctx, cls);
+        if (!*ptr) {
+            {
+                std::lock_guard<std::mutex> lock(ctx->pool_mu);
+                if (ctx->hbm_budget && ctx->bytes_in_use + ctx->pool_bytes + bytes > ctx->hbm_budget)
+                    pool_release_locked(ctx);
+            }
+            e = cudaMalloc(ptr, cls);
+            if (e != cudaSuccess) {
+                (void)cudaGetLastError();
+                pool_release(ctx);
+                e = cudaMalloc(ptr, cls);
+            }
+        }
+    }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         set_error("cudaMalloc of %zu bytes failed: %s", bytes,
@@ -44,11 +101,29 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     return YETI_OK;
 }
 
+// Keep the block for the next dev_alloc of its class if there is room.
+static bool pool_put(yeti_ctx *ctx, void *ptr, size_t cls) {
+    if (cls > kPoolBlock) return false;
+    std::lock_guard<std::mutex> lock(ctx->pool_mu);
+    if (ctx->pool_bytes + cls > kPoolBytes) return false;
+    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->stream};
+    if (cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventRecord(b.freed, ctx->stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (b.freed) cudaEventDestroy(b.freed);
+        return false;
+    }
+    ctx->pool.emplace(cls, b);
+    ctx->pool_bytes += cls;
+    return true;
+}
+
 void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes) {
     if (!ptr) return;
+    if (!bytes) bytes = 16;
     if (ctx && ctx->stream_ordered) cudaFreeAsync(ptr, ctx->stream);
-    else cudaFree(ptr);
-    if (ctx) ctx->bytes_in_use -= (bytes ? bytes : 16);
+    else if (!ctx || !pool_put(ctx, ptr, pool_class(bytes))) cudaFree(ptr);
+    if (ctx) ctx->bytes_in_use -= bytes;
 }
 
 static std::atomic<uint64_t> g_launches{0};
@@ -115,6 +190,7 @@ YETI_API int yeti_ctx_create(int device, size_t hbm_budget_bytes,
 YETI_API int yeti_ctx_destroy(yeti_ctx *ctx) {
     if (!ctx) return YETI_OK;
     DeviceGuard g(ctx->device);
+    pool_release(ctx);
     if (ctx->own_stream) {
         cudaStreamSynchronize(ctx->own_stream);
         cudaStreamDestroy(ctx->own_stream);

@@ -584,12 +584,6 @@ __global__ void k_grad_gather(int64_t n, const int64_t *ptr, const int64_t *idx,
     ge[t] = ae;
 }
 
-static bool in_list_g(const int64_t *l, int64_t n, int64_t v) {
-    for (int64_t i = 0; i < n; i++)
-        if (l[i] == v) return true;
-    return false;
-}
-
 }  // namespace yeti
 
 using namespace yeti;
@@ -613,12 +607,8 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
     const double *sol_d = sol, *adj_d = adj;
     double *gi_d = gwint, *ge_d = gwext;
     if (mem == YETI_MEM_HOST) {
-        YETI_TRY(upload(ctx, dsol, sol, (size_t)3 * ncp));
-        YETI_TRY(upload(ctx, dadj, adj, (size_t)nout));
         YETI_TRY(dgi.alloc(ctx, nout * sizeof(double)));
         YETI_TRY(dge.alloc(ctx, nout * sizeof(double)));
-        sol_d = dsol.as<double>();
-        adj_d = dadj.as<double>();
         gi_d = dgi.as<double>();
         ge_d = dge.as<double>();
     }
@@ -632,18 +622,29 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         keep.emplace_back(new DevBuf());
         return *keep.back();
     };
-    DevBuf dj, da, dinfo, dnd;
+    DevBuf larena, dj, da, dinfo, dnd;
+    UploadPack lpack;
     std::vector<int32_t> jdl(m->nb_load > 0 ? m->nb_load : 1, 0);
     for (int64_t i = 0; i < m->nb_load; i++) jdl[i] = (int32_t)m->jdltype[i];
-    YETI_TRY(upload(ctx, dj, jdl.data(), jdl.size()));
+    lpack.add(dj, jdl);
     std::vector<double> adl(m->nb_load > 0 ? m->nb_load : 1, 0.0);
     for (int64_t i = 0; i < m->nb_load; i++) adl[i] = m->adlmag[i];
-    YETI_TRY(upload(ctx, da, adl.data(), adl.size()));
+    lpack.add(da, adl);
     std::vector<double> inf(m->len_load_addinfos > 0 ? m->len_load_addinfos : 1, 0.0);
     for (int64_t i = 0; i < m->len_load_addinfos; i++) inf[i] = m->load_addinfos[i];
-    YETI_TRY(upload(ctx, dinfo, inf.data(), inf.size()));
+    lpack.add(dinfo, inf);
     if (m->nodal_dist && m->nb_n_dist > 0)
-        YETI_TRY(upload(ctx, dnd, m->nodal_dist, (size_t)m->nb_n_dist * m->nb_cp));
+        lpack.add(dnd, m->nodal_dist, (size_t)m->nb_n_dist * m->nb_cp);
+    if (mem == YETI_MEM_HOST) {
+        lpack.add(dsol, sol, (size_t)3 * ncp);
+        lpack.add(dadj, adj, (size_t)nout);
+    }
+    YETI_TRY(lpack.commit(ctx, larena));
+    if (mem == YETI_MEM_HOST) {
+        sol_d = dsol.as<double>();
+        adj_d = dadj.as<double>();
+    }
+    const LoadMarks marks(m, [](int64_t ty) { return ty == 101 || (ty > 9 && ty < 100); });
     // element contributions, in global element order
     struct Done { int patch; int64_t local; int64_t off; };
     std::vector<Done> done;
@@ -661,17 +662,12 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         int max_body = 0;
         for (int64_t le = 0; le < P.nactive; le++) {
             const int64_t jel = P.act[le] + 1;
-            int64_t k2 = 0;
             int nb = 0;
-            for (int64_t il = 0; il < m->nb_load; il++) {
-                const int64_t nt = m->load_target_nbelem[il], ty = m->jdltype[il];
-                if ((ty == 101 || (ty > 9 && ty < 100)) && in_list_g(m->inddload + k2, nt, jel)) {
+            for (int64_t il = 0; il < m->nb_load; il++)
+                if (marks.on(il, jel)) {
                     terms.push_back((int32_t)il);
-                    nb += ty == 101;
-                    if (ty == 4 % 10 && 0) {}
+                    nb += m->jdltype[il] == 101;
                 }
-                k2 += nt;
-            }
             YETI_CHECK(nb <= 8, YETI_EUNSUPPORTED, "more than 8 centrifugal loads on one element");
             max_body = std::max(max_body, nb);
             elems.push_back((int32_t)le);
@@ -684,15 +680,14 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
             gauss_face_host(P.ng, f, tmp);
             std::copy(tmp.begin(), tmp.end(), gf.begin() + (f - 1) * 4 * P.ng * P.ng);
         }
-        DevBuf &dgf = newbuf();
-        YETI_TRY(upload(ctx, dgf, gf.data(), gf.size()));
-        DevBuf &del = newbuf();
-        YETI_TRY(upload(ctx, del, elems.data(), elems.size()));
-        DevBuf &dtp = newbuf();
-        YETI_TRY(upload(ctx, dtp, tptr.data(), tptr.size()));
-        DevBuf &dtm = newbuf();
+        DevBuf &arena = newbuf(), &dgf = newbuf(), &del = newbuf(), &dtp = newbuf(), &dtm = newbuf();
+        UploadPack epack;
+        epack.add(dgf, gf);
+        epack.add(del, elems);
+        epack.add(dtp, tptr);
         if (terms.empty()) terms.push_back(0);
-        YETI_TRY(upload(ctx, dtm, terms.data(), terms.size()));
+        epack.add(dtm, terms);
+        YETI_TRY(epack.commit(ctx, arena));
         DevBuf &bi = newbuf();
         DevBuf &be = newbuf();
         YETI_TRY(bi.alloc(ctx, sizeof(double) * nadj * 3 * P.nn * elems.size()));
@@ -779,10 +774,11 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
     for (int64_t i = 0; i < nout; i++) ptr[i + 1] += ptr[i];
     std::vector<int64_t> idx(std::max<int64_t>(ptr[nout], 1), 0), fill(ptr.begin(), ptr.end() - 1);
     walk([&](int64_t o, int64_t e) { idx[fill[o]++] = e; });
-    DevBuf &dptr = newbuf();
-    DevBuf &didx = newbuf();
-    YETI_TRY(upload(ctx, dptr, ptr.data(), ptr.size()));
-    YETI_TRY(upload(ctx, didx, idx.data(), idx.size()));
+    DevBuf &garena = newbuf(), &dptr = newbuf(), &didx = newbuf();
+    UploadPack gpack;
+    gpack.add(dptr, ptr);
+    gpack.add(didx, idx);
+    YETI_TRY(gpack.commit(ctx, garena));
     k_grad_gather<<<(unsigned)((nout + 255) / 256), 256, 0, s>>>(
         nout, dptr.as<int64_t>(), didx.as<int64_t>(), ai.as<double>(), ae.as<double>(), gi_d, ge_d);
     count_launches(1);

@@ -21,6 +21,7 @@ struct U1Patch {
     int64_t nb_data_elem = 0;
     std::vector<int64_t> act;   // global ids (0-based) of active elements
     std::vector<int64_t> slot;  // COO slot offset of each active element
+    // views of U1Model::arena
     DevBuf knots;   // U_1 | U_2 | U_3
     DevBuf gauss;   // 4 * nq  (weight, t1, t2, t3)
     DevBuf ien;     // nactive * nn, int32 0-based CP index
@@ -31,6 +32,7 @@ struct U1Patch {
 };
 
 struct U1Model {
+    DevBuf arena;            // holds the arrays of the patches and coords
     std::vector<U1Patch> patches;
     DevBuf coords;           // 3 * nb_cp
     int64_t nb_cp = 0;
@@ -46,5 +48,30 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out);
 int launch_u1_stiffness_sf(yeti_ctx *ctx, const U1Patch &P, const double *coords,
                            double lam, double mu, double *kdata, int32_t *krow,
                            int32_t *kcol, size_t smem_cap);
+
+// Which elements carry a distributed or body load, per load: on(il, jel) for
+// load il and 1-based element jel.
+class LoadMarks {
+    std::vector<std::vector<char>> mark;   // empty: not such a load
+
+public:
+    // takes(type): the loads of interest
+    template <class F>
+    LoadMarks(const yeti_u1_model *m, F takes) : mark(m->nb_load > 0 ? m->nb_load : 0) {
+        int64_t k = 0;
+        for (int64_t il = 0; il < m->nb_load; il++) {
+            const int64_t n = m->load_target_nbelem[il];
+            if (takes(m->jdltype[il])) {
+                mark[il].assign(m->nb_elem + 1, 0);
+                for (int64_t i = 0; i < n; i++) {
+                    const int64_t e = m->inddload[k + i];
+                    if (e >= 1 && e <= m->nb_elem) mark[il][e] = 1;
+                }
+            }
+            k += n;
+        }
+    }
+    bool on(int64_t il, int64_t jel) const { return !mark[il].empty() && mark[il][jel]; }
+};
 
 }  // namespace yeti

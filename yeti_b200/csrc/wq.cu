@@ -742,6 +742,7 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
                    "yeti_wq_setup: weight %d is %g", i, weights[i]);
     // 1-D rules, block partition, tiles
     WQRule1D R[3];
+    UploadPack pack;
     for (int d = 0; d < 3; d++) {
         YETI_CHECK(wq_rule_1d(p[d], nel[d], R[d]) == 0, YETI_EINVAL,
                    "yeti_wq_setup: WQ rule failed");
@@ -753,14 +754,14 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
         }
         op->NF[d] = NF;
         op->NQ[d] = NQ;
-        YETI_TRY(upload(ctx, op->blkd[d], op->blk[d].data(), op->blk[d].size()));
+        pack.add(op->blkd[d], op->blk[d]);
         std::vector<double> t6, t4;
         build_tiles<double>(R[d], op->blk[d], NF, NQ, t6, &t4);
-        YETI_TRY(upload(ctx, op->tiles64[d], t6.data(), t6.size()));
+        pack.add(op->tiles64[d], t6);
         std::vector<float> f6;
         build_tiles<float>(R[d], op->blk[d], NF, NQ, f6, nullptr);
-        YETI_TRY(upload(ctx, op->tiles32[d], f6.data(), f6.size()));
-        YETI_TRY(upload(ctx, op->dtiles[d], t4.data(), t4.size()));
+        pack.add(op->tiles32[d], f6);
+        pack.add(op->dtiles[d], t4);
     }
     const int nb[3] = {(int)op->blk[0].size(), (int)op->blk[1].size(), (int)op->blk[2].size()};
     op->nblocks = (int64_t)nb[0] * nb[1] * nb[2];
@@ -772,7 +773,8 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
         qoff[b + 1] = qoff[b] + (int64_t)op->blk[0][bu].nq * op->blk[1][bv].nq * op->blk[2][bw].nq;
     }
     op->nqp_total = qoff[op->nblocks];
-    YETI_TRY(upload(ctx, op->qoff, qoff.data(), qoff.size()));
+    pack.add(op->qoff, qoff);
+    YETI_TRY(pack.commit(ctx, op->tables));
     // geometry -> coefficients
     DevBuf dcps, dw, flags;
     YETI_TRY(upload(ctx, dcps, cps, (size_t)3 * ncp));
@@ -877,7 +879,10 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
 YETI_API int yeti_wq_destroy(yeti_wq_op *op) {
     if (!op) return YETI_OK;
     DeviceGuard guard(op->ctx->device);
-    cudaStreamSynchronize(op->ctx->stream);
+    // the operator's memory goes back to the context's pool: wait for its
+    // work on every stream the context has had since
+    if (op->ctx->stream_ordered) cudaStreamSynchronize(op->ctx->stream);
+    else cudaDeviceSynchronize();
     delete op;
     return YETI_OK;
 }

@@ -67,6 +67,7 @@ struct WQStreamPlan {
     int per_sm[2] = {0, 0};
     size_t smem[2] = {0, 0};
     int64_t ncoef = 0;
+    DevBuf tables;           // holds the arrays below
     DevBuf elem[2], band64[3], band32[3], wq0, tq0[2], tnq[2];
     DevBuf tile_off, tile_pstride, seg[2], cta_seg[2];
     DevBuf err;              // int: a kernel's bounded wait gave up
@@ -187,6 +188,7 @@ struct yeti_wq_op {
     double E = 0, nu = 0;
     std::vector<yeti::BlkInfo> blk[3];
     int NF[3] = {0, 0, 0}, NQ[3] = {0, 0, 0};
+    yeti::DevBuf tables;    // holds the arrays of blkd .. qoff
     yeti::DevBuf blkd[3];
     yeti::DevBuf tiles64[3], tiles32[3], dtiles[3];
     yeti::DevBuf qoff;

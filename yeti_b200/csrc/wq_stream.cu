@@ -921,11 +921,6 @@ static void make_tiles(const std::vector<int> &elem_q0, int nel, std::vector<int
     if (last_begin < nel) add(last_begin, nel);
 }
 
-template <class T>
-static int upload_vec(yeti_ctx *ctx, DevBuf &b, const std::vector<T> &v) {
-    return upload(ctx, b, v.data(), v.size());
-}
-
 // Copy the coefficients from the element-block layout of the setup kernels
 // into the tile/plane layout of the streaming kernel.
 template <class T>
@@ -1008,6 +1003,7 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
     yeti_ctx *ctx = op->ctx;
     WQStreamPlan &st = op->st;
     const int P = op->p[0], PBP = (P + 1 + 3) / 4 * 4;
+    UploadPack pack;
     std::vector<int> elem_q0[3];
     std::vector<double> band_uv[2];
     std::vector<int> elem_uv[2];
@@ -1043,11 +1039,11 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
             band_uv[d] = band;
             elem_uv[d] = elem;
         }
-        if (d < 2) YETI_TRY(upload_vec(ctx, st.elem[d], elem));
-        YETI_TRY(upload_vec(ctx, st.band64[d], band));
-        YETI_TRY(upload_vec(ctx, st.band32[d], bandf));
+        if (d < 2) pack.add(st.elem[d], elem);
+        pack.add(st.band64[d], band);
+        pack.add(st.band32[d], bandf);
     }
-    YETI_TRY(upload_vec(ctx, st.wq0, elem_q0[2]));
+    pack.add(st.wq0, elem_q0[2]);
     std::vector<int> tq0[2], tnq[2], treg[2];
     for (int d = 0; d < 2; d++) {
         make_tiles(elem_q0[d], op->nel[d], tq0[d], tnq[d], treg[d], d == 0 ? kTQ : kTV);
@@ -1065,8 +1061,8 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
             if (per) treg[d][t] |= 8;
         }
         st.ntile[d] = (int)tq0[d].size();
-        YETI_TRY(upload_vec(ctx, st.tq0[d], tq0[d]));
-        YETI_TRY(upload_vec(ctx, st.tnq[d], tnq[d]));
+        pack.add(st.tq0[d], tq0[d]);
+        pack.add(st.tnq[d], tnq[d]);
     }
     // coefficient layout: tile-major, then w plane, then entry, then point
     const int ntiles = st.ntile[0] * st.ntile[1];
@@ -1080,8 +1076,8 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
         toff[t + 1] = toff[t] + (int64_t)nqw * pstride[t];
     }
     st.ncoef = toff[ntiles];
-    YETI_TRY(upload_vec(ctx, st.tile_off, toff));
-    YETI_TRY(upload_vec(ctx, st.tile_pstride, pstride));
+    pack.add(st.tile_off, toff);
+    pack.add(st.tile_pstride, pstride);
     YETI_TRY(st.err.alloc(ctx, sizeof(int)));
     YETI_CUDA(cudaMemsetAsync(st.err.ptr, 0, sizeof(int), ctx->stream));
 
@@ -1151,10 +1147,10 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
             cta_seg[c + 1] = (int)seg.size();
         }
         st.grid[which] = (int)ncta;
-        YETI_TRY(upload_vec(ctx, st.seg[which], seg));
-        YETI_TRY(upload_vec(ctx, st.cta_seg[which], cta_seg));
+        pack.add(st.seg[which], seg);
+        pack.add(st.cta_seg[which], cta_seg);
     }
-    return YETI_OK;
+    return pack.commit(ctx, st.tables);
 }
 
 template <class T>
@@ -1164,7 +1160,8 @@ static int permute_one(yeti_wq_op *op, const DevBuf &src, DevBuf &dst) {
     YETI_TRY(dst.alloc(ctx, st.ncoef * sizeof(T)));
     YETI_CUDA(cudaMemsetAsync(dst.ptr, 0, st.ncoef * sizeof(T), ctx->stream));
     // per-direction maps of the setup layout: point -> (block, local index)
-    DevBuf blk[3], loc[3], nq1[3], ptrs;
+    DevBuf blk[3], loc[3], nq1[3], maps, ptrs;
+    UploadPack pack;
     const int *hp[9];
     for (int d = 0; d < 3; d++) {
         std::vector<int> b(op->nqp[d]), l(op->nqp[d]), n(op->blk[d].size());
@@ -1176,9 +1173,12 @@ static int permute_one(yeti_wq_op *op, const DevBuf &src, DevBuf &dst) {
                 l[B.q0 + q] = q;
             }
         }
-        YETI_TRY(upload_vec(ctx, blk[d], b));
-        YETI_TRY(upload_vec(ctx, loc[d], l));
-        YETI_TRY(upload_vec(ctx, nq1[d], n));
+        pack.add(blk[d], b);
+        pack.add(loc[d], l);
+        pack.add(nq1[d], n);
+    }
+    YETI_TRY(pack.commit(ctx, maps));
+    for (int d = 0; d < 3; d++) {
         hp[d] = blk[d].as<int>();
         hp[3 + d] = loc[d].as<int>();
         hp[6 + d] = nq1[d].as<int>();
