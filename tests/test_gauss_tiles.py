@@ -62,3 +62,19 @@ def test_gpu_assembly_into_arrays_on_8_byte_boundaries(cuda_ok):
     np.testing.assert_array_equal(r[1:].cpu().numpy(), ref[1])
     np.testing.assert_array_equal(c[1:].cpu().numpy(), ref[2])
     assert k[0] == -1.0 and k[-1] == -1.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nadj", [1, 2, 3, 4])
+@pytest.mark.parametrize("nel,p", [((3, 2, 2), (2, 2, 2)), ((2, 1, 2), (3, 4, 2))])
+def test_gpu_gradient_of_one_to_four_adjoints_matches_oracle(cuda_ok, nadj, nel, p):
+    """The kernel for one adjoint and the one for several, points in one chunk
+    and in several."""
+    from yeti_b200.gradient import grad_from_system_args
+    args = _args(nel, p)
+    rng = np.random.default_rng(nadj)
+    sol = 0.01 * rng.standard_normal((3, args[2].shape[1]))
+    adj = 0.01 * rng.standard_normal((nadj, 3, args[2].shape[1]))
+    for got, ref in zip(grad_from_system_args(args, sol, adj),
+                        oracle.grad_lin_elast_work(args, sol, adj)):
+        np.testing.assert_array_equal(got, ref)

@@ -11,15 +11,14 @@
 // v = P x Q (normal pressure, shapPress.f face ordering) or e_t |A x B|
 // (fixed direction), differentiated through the face tangents.
 //
-// Kernel design: one CTA per active element.  Stage A: one thread per
-// quadrature point computes the basis, covariant frame, metrics, strains and
-// stresses of the state and adjoint fields into shared memory (all the
-// points when their records fit, else chunk by chunk, every sum continued
-// across the chunks in point order).  Stage B: one
-// thread per control point accumulates its (nadj x 3) derivative over the
-// points in order.  A second kernel sums element contributions per control
-// point in element order (deterministic).  Compiled without FMA contraction
-// and following the reference's operation order.
+// Kernel design: one CTA per active element.  Stage A computes per quadrature
+// point the basis, covariant frame, metrics, strains and stresses of the state
+// and adjoint fields into shared memory, chunk by chunk of points, every sum
+// continued across the chunks in point order.  Stage B: one thread per
+// (control point, component) accumulates its derivatives over the points in
+// order.  A second kernel sums element contributions per control point in
+// element order (deterministic).  Compiled without FMA contraction and
+// following the reference's operation order.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -31,12 +30,18 @@
 namespace yeti {
 
 constexpr int kGradMaxAdj = 4;
+constexpr int kGradThreads = 512;   // threads per SM of k_u1_grad<1> (128 registers each)
 
-__device__ __constant__ int c_vi[6] = {0, 1, 2, 0, 0, 1};
-__device__ __constant__ int c_vj[6] = {0, 1, 2, 1, 2, 2};
+// Voigt pairs (11, 22, 33, 12, 13, 23) as compile-time functions: the loops
+// over them are unrolled, so that the 3x3 and 6x6 tensors stay in registers
+// (with the pairs in constant memory every access went through local memory).
+__host__ __device__ constexpr int voigt_i(int ij) { return ij < 3 ? ij : ij == 5 ? 1 : 0; }
+__host__ __device__ constexpr int voigt_j(int ij) { return ij < 3 ? ij : ij == 3 ? 1 : 2; }
+// Entry (i, j) of a symmetric 3x3 matrix held as its Voigt entries.
+__host__ __device__ constexpr int voigt(int i, int j) { return i == j ? i : i + j + 2; }
 
 struct GradArgs {
-    int p0, p1, p2, nn, nq, ng, nadj, qchunk, pchunk;
+    int p0, p1, p2, nn, nq, ng, nadj, pchunk;
     int compute_int, compute_ext, include_surface;
     const double *U0, *U1, *U2;
     const double *gauss;      // volume rule (4 * nq)
@@ -121,15 +126,13 @@ __host__ __device__ inline PtLayout pt_layout(int nn, int nadj, int nbody) {
 
 // Shared memory of one element: xe, ue, uae, we, then the point records
 // (PtLayout) of one chunk of pchunk points, then the basis scratch
-// (1-D rows, node indices, kBasisQS per point of the chunk), the external- and
-// internal-work accumulators of the (control point, component) tasks and
-// the term buffer of stage B (qchunk points).
+// (1-D rows, node indices, kBasisQS per point of the chunk) and the external-
+// and internal-work accumulators of the (control point, component) tasks.
 __host__ __device__ inline size_t grad_smem_doubles(int nn, int pchunk, int nadj, const PtLayout &L,
-                                                    size_t face, int qchunk, int ng) {
+                                                    size_t face, int ng) {
     const size_t vol = (size_t)pchunk * L.size;
     return (size_t)(6 + 3 * nadj) * nn + nn + (vol > face ? vol : face) +
-           basis_rows_doubles(ng) + (nn + 1) / 2 + (size_t)pchunk * kBasisQS + (size_t)2 * 3 * nn * nadj +
-           (size_t)3 * nn * qchunk * 3 * nadj;
+           basis_rows_doubles(ng) + (nn + 1) / 2 + (size_t)pchunk * kBasisQS + (size_t)2 * 3 * nn * nadj;
 }
 
 // gradUELMAT1adj (gradUELMAT_solid.f90:18-479) of one element per CTA.
@@ -141,9 +144,20 @@ __host__ __device__ inline size_t grad_smem_doubles(int nn, int pchunk, int nadj
 // dAAE, dC and the accumulated gradient -- depends on that component alone,
 // so each task performs exactly the operations the reference performs for
 // its component, in the same order, and the results keep their bits.
-__global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
+// What bounds it: the FP64 pipe in stage B (about 800 operations per point and
+// task; 0.19 ms for 32x32x2 elements of p=2 at its highest rate) and the
+// chain of short steps of stage A.  The tensors of a task live in registers;
+// the points are a loop of the task's thread, so nothing is passed between
+// threads, and small CTAs (96 threads at p=2, five per SM) run each
+// other's stages A and B at the same time.  Measured on B200 against a thread
+// per (task, point) with the Voigt pairs in constant memory, whose tensors
+// went through local memory and its terms through shared memory: 32x32x2 of
+// p=2 1284 -> 350 us, 6^3 of p=3 1160 -> 277 us, 4^3 of p=4 2297 -> 567 us.
+// NA: adjoints the loops are unrolled for (nadj of them are present).
+template <int NA>
+__global__ void __launch_bounds__(256, NA == 1 ? 2 : 1) k_u1_grad(GradArgs a) {
     extern __shared__ double sm[];
-    const int nn = a.nn, nadj = a.nadj;
+    const int nn = a.nn, nadj = NA == 1 ? 1 : a.nadj;
     const int e = a.elems[blockIdx.x];
     double *xe = sm;                    // 3*nn coords
     double *ue = xe + 3 * nn;           // 3*nn state
@@ -190,7 +204,6 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
     double *qs = rows + basis_rows_doubles(a.ng) + (nn + 1) / 2;
     double *ge_s = qs + (size_t)pc * kBasisQS;
     double *gi_s = ge_s + (size_t)3 * nn * nadj;   // 3 nn nadj accumulators
-    double *terms = gi_s + (size_t)3 * nn * nadj;  // 3 nn qchunk 3 nadj terms
     const double lambda = a.E * a.nu / (1.0 + a.nu) / (1.0 - 2.0 * a.nu);
     const double mu = a.E / 2.0 / (1.0 + a.nu);
     for (int t = tid; t < 3 * nn * nadj; t += nth) gi_s[t] = ge_s[t] = 0.0;
@@ -253,64 +266,59 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
             P[L.dj] = detJac;
             if (a.compute_int) {
                 double AAI[3][3], AAE[3][3];
+#pragma unroll
                 for (int i = 0; i < 3; i++)
+#pragma unroll
                     for (int j = 0; j < 3; j++) AAI[i][j] = gdot(AI[i], AI[j]);
                 ginv3(AAI, AAE);
+                // H is symmetric: the reference copies its upper triangle
                 double H[6][6];
+#pragma unroll
                 for (int kl = 0; kl < 6; kl++) {
-                    const int k = c_vi[kl], l = c_vj[kl];
+                    const int k = voigt_i(kl), l = voigt_j(kl);
+#pragma unroll
                     for (int ij = 0; ij <= kl; ij++) {
-                        const int i = c_vi[ij], j = c_vj[ij];
+                        const int i = voigt_i(ij), j = voigt_j(ij);
                         H[ij][kl] = lambda * AAE[i][j] * AAE[k][l] +
                                     mu * (AAE[i][k] * AAE[j][l] + AAE[i][l] * AAE[j][k]);
+                        H[kl][ij] = H[ij][kl];
                     }
                 }
-                for (int kl = 1; kl < 6; kl++)
-                    for (int r = kl; r < 6; r++) H[r][kl - 1] = H[kl - 1][r];
-                double dU[3][3];
-                for (int i = 0; i < 3; i++)
-                    for (int c = 0; c < 3; c++) dU[i][c] = P[L.dU + 3 * i + c];
-                double strain[6], stress[6];
-                for (int ij = 0; ij < 6; ij++) {
-                    const int i = c_vi[ij], j = c_vj[ij];
-                    if (i == j) strain[ij] = gdot(AI[i], dU[i]);
-                    else strain[ij] = gdot(AI[i], dU[j]) + gdot(AI[j], dU[i]);
-                }
-                for (int ii = 0; ii < 6; ii++) {
-                    double s = 0.0;
-                    for (int jj = 0; jj < 6; jj++) s = s + H[ii][jj] * strain[jj];
-                    stress[ii] = s;
-                }
-                for (int i = 0; i < 3; i++)
-                    for (int c = 0; c < 3; c++) P[L.AAE + 3 * i + c] = AAE[i][c];
-                for (int ij = 0; ij < 6; ij++) {
-                    P[L.strain + ij] = strain[ij];
-                    P[L.stress + ij] = stress[ij];
-                }
-                for (int k = 0; k < nadj; k++) {
-                    double dA[3][3];
+                // strain and stress of a displacement gradient
+                auto strains = [&](const double *dv, double *e, double *t) {
+                    double dU[3][3], strain[6];
+#pragma unroll
                     for (int i = 0; i < 3; i++)
-                        for (int c = 0; c < 3; c++) dA[i][c] = P[L.dUA + 9 * k + 3 * i + c];
-                    double sA[6], tA[6];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) dU[i][c] = dv[3 * i + c];
+#pragma unroll
                     for (int ij = 0; ij < 6; ij++) {
-                        const int i = c_vi[ij], j = c_vj[ij];
-                        if (i == j) sA[ij] = gdot(AI[i], dA[i]);
-                        else sA[ij] = gdot(AI[i], dA[j]) + gdot(AI[j], dA[i]);
+                        const int i = voigt_i(ij), j = voigt_j(ij);
+                        if (i == j) strain[ij] = gdot(AI[i], dU[i]);
+                        else strain[ij] = gdot(AI[i], dU[j]) + gdot(AI[j], dU[i]);
+                        e[ij] = strain[ij];
                     }
+#pragma unroll
                     for (int ii = 0; ii < 6; ii++) {
                         double s = 0.0;
-                        for (int jj = 0; jj < 6; jj++) s = s + H[ii][jj] * sA[jj];
-                        tA[ii] = s;
+#pragma unroll
+                        for (int jj = 0; jj < 6; jj++) s = s + H[ii][jj] * strain[jj];
+                        t[ii] = s;
                     }
-                    for (int ij = 0; ij < 6; ij++) {
-                        P[L.sA + 6 * k + ij] = sA[ij];
-                        P[L.tA + 6 * k + ij] = tA[ij];
-                    }
+                };
+                strains(P + L.dU, P + L.strain, P + L.stress);
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) P[L.AAE + 3 * i + c] = AAE[i][c];
+                for (int k = 0; k < nadj; k++)
+                    strains(P + L.dUA + 9 * k, P + L.sA + 6 * k, P + L.tA + 6 * k);
+                for (int k = 0; k < nadj; k++) {
+                    double work = 0.0;
+#pragma unroll
+                    for (int ij = 0; ij < 6; ij++) work = work + P[L.sA + 6 * k + ij] * P[L.stress + ij];
+                    P[L.work + k] = work;
                 }
-                for (int k = 0; k < nadj; k++) P[L.work + k] = 0.0;
-                for (int ij = 0; ij < 6; ij++)
-                    for (int k = 0; k < nadj; k++)
-                        P[L.work + k] = P[L.work + k] + P[L.sA + 6 * k + ij] * stress[ij];
             }
             if (a.compute_ext && nbody > 0) {
                 for (int k = 0; k < nadj; k++)
@@ -344,87 +352,92 @@ __global__ void __launch_bounds__(256) k_u1_grad(GradArgs a) {
             }
         }
         __syncthreads();
-        // ---------------- stage B: interior work, per (control point, component,
-        // point) in parallel.  Each thread forms the three terms the reference
-        // subtracts from the gradient at its point (work dJ detJ, the
-        // stress-times-strain-variation term, the material-variation term); one
-        // thread per (control point, component) then subtracts them in point
-        // order, the reference's order, so the sums keep their bits.  Points are
-        // taken in chunks of a.qchunk (the term buffer).
+        // ---------------- stage B: interior work, a thread per (control point,
+        // component) over the chunk's points in order: the three terms the
+        // reference subtracts from the gradient at a point (work dJ detJ, the
+        // stress-times-strain-variation term, the material-variation term)
         if (a.compute_int) {
-            for (int q0 = 0; q0 < np; q0 += a.qchunk) {
-                const int nqc = min(a.qchunk, np - q0);
-                __syncthreads();
-                for (int t = tid; t < 3 * nn * nqc; t += nth) {
-                    const int task = t / nqc, ql = t - task * nqc, q = q0 + ql;
-                    const int cp = task / 3, c = task - 3 * cp;
+            for (int task = tid; task < 3 * nn; task += nth) {
+                const int cp = task / 3, c = task - 3 * cp;
+                double g[NA];
+#pragma unroll
+                for (int k = 0; k < NA; k++) g[k] = k < nadj ? gi_s[task * nadj + k] : 0.0;
+                for (int q = 0; q < np; q++) {
                     const double *P = pts + (size_t)q * L.size;
                     const double *dr = P + L.dR + 3 * cp;
                     const double Area = P[L.area], detJac = P[L.dj];
                     const double *AxA = P + L.AxA;
                     const double *AI = P + L.AI, *AAE = P + L.AAE;
                     const double *stress = P + L.stress, *strain = P + L.strain, *dU = P + L.dU;
-                    double *tt = terms + ((size_t)task * a.qchunk + ql) * 3 * nadj;
+                    const double d0 = dr[0], d1 = dr[1], d2 = dr[2];
+                    const double drv[3] = {d0, d1, d2};
                     double dJ = 0.0;
-                    for (int i = 0; i < 3; i++) dJ = dJ + AxA[3 * i + c] * dr[i];
-                    for (int k = 0; k < nadj; k++) tt[3 * k] = P[L.work + k] * dJ * detJac;
-                    for (int k = 0; k < nadj; k++) {
-                        const double *d = P + L.dUA + 9 * k;
+#pragma unroll
+                    for (int i = 0; i < 3; i++) dJ = dJ + AxA[3 * i + c] * drv[i];
+                    // sum of t[ij] times the strain variation of dv
+                    auto variation = [&](const double *t, const double *dv) {
+                        const double v[3] = {dv[c], dv[3 + c], dv[6 + c]};
                         double ev = 0.0;
+#pragma unroll
                         for (int ij = 0; ij < 6; ij++) {
-                            const int i = c_vi[ij], j = c_vj[ij];
-                            if (i == j) ev = ev + stress[ij] * d[3 * i + c] * dr[i];
-                            else ev = ev + stress[ij] * d[3 * i + c] * dr[j] + stress[ij] * d[3 * j + c] * dr[i];
+                            const int i = voigt_i(ij), j = voigt_j(ij);
+                            if (i == j) ev = ev + t[ij] * v[i] * drv[i];
+                            else ev = ev + t[ij] * v[i] * drv[j] + t[ij] * v[j] * drv[i];
                         }
-                        tt[3 * k + 1] = ev * Area * detJac;
+                        return ev;
+                    };
+                    double vA[NA];
+#pragma unroll
+                    for (int k = 0; k < NA; k++) {
+                        if (k >= nadj) continue;
+                        g[k] = g[k] - P[L.work + k] * dJ * detJac;
+                        g[k] = g[k] - variation(stress, P + L.dUA + 9 * k) * Area * detJac;
+                        vA[k] = variation(P + L.tA + 6 * k, dU);
                     }
-                    double dAAI[3][3], dAAE[3][3];
+                    // AAE and dAAI are symmetric to the bit (their entries (i, j)
+                    // and (j, i) are the same products and sums), dAAE is not:
+                    // its two triangles add the same terms in other orders
+                    double E[6], dI[6], dE[3][3];
+#pragma unroll
+                    for (int ij = 0; ij < 6; ij++) {
+                        const int i = voigt_i(ij), j = voigt_j(ij);
+                        E[ij] = AAE[3 * i + j];
+                        dI[ij] = drv[i] * AI[3 * j + c] + AI[3 * i + c] * drv[j];
+                    }
+#pragma unroll
                     for (int j = 0; j < 3; j++)
-                        for (int i = 0; i < 3; i++) dAAI[i][j] = dr[i] * AI[3 * j + c] + AI[3 * i + c] * dr[j];
-                    for (int i = 0; i < 3; i++)
-                        for (int j = 0; j < 3; j++) dAAE[i][j] = 0.0;
-                    for (int j = 0; j < 3; j++)
-                        for (int i = 0; i < 3; i++)
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            double v = 0.0;
+#pragma unroll
                             for (int l = 0; l < 3; l++)
+#pragma unroll
                                 for (int k = 0; k < 3; k++)
-                                    dAAE[i][j] = dAAE[i][j] - AAE[3 * i + k] * AAE[3 * l + j] * dAAI[k][l];
-                    double vA[kGradMaxAdj];
-                    for (int k = 0; k < nadj; k++) {
-                        const double *tA = P + L.tA + 6 * k;
-                        double ev = 0.0;
-                        for (int ij = 0; ij < 6; ij++) {
-                            const int i = c_vi[ij], j = c_vj[ij];
-                            if (i == j) ev = ev + tA[ij] * dU[3 * i + c] * dr[i];
-                            else ev = ev + tA[ij] * dU[3 * i + c] * dr[j] + tA[ij] * dU[3 * j + c] * dr[i];
+                                    v = v - E[voigt(i, k)] * E[voigt(l, j)] * dI[voigt(k, l)];
+                            dE[i][j] = v;
                         }
-                        vA[k] = ev;
-                    }
+#pragma unroll
                     for (int kl = 0; kl < 6; kl++) {
-                        const int k = c_vi[kl], l = c_vj[kl];
+                        const int k = voigt_i(kl), l = voigt_j(kl);
+#pragma unroll
                         for (int ij = 0; ij < 6; ij++) {
-                            const int i = c_vi[ij], j = c_vj[ij];
+                            const int i = voigt_i(ij), j = voigt_j(ij);
                             const double dC =
-                                lambda * dAAE[i][j] * AAE[3 * k + l] + lambda * AAE[3 * i + j] * dAAE[k][l] +
-                                mu * dAAE[i][k] * AAE[3 * j + l] + mu * AAE[3 * i + k] * dAAE[j][l] +
-                                mu * dAAE[i][l] * AAE[3 * j + k] + mu * AAE[3 * i + l] * dAAE[j][k];
-                            for (int kk = 0; kk < nadj; kk++)
-                                vA[kk] = vA[kk] + dC * strain[ij] * P[L.sA + 6 * kk + kl];
+                                lambda * dE[i][j] * E[voigt(k, l)] + lambda * E[voigt(i, j)] * dE[k][l] +
+                                mu * dE[i][k] * E[voigt(j, l)] + mu * E[voigt(i, k)] * dE[j][l] +
+                                mu * dE[i][l] * E[voigt(j, k)] + mu * E[voigt(i, l)] * dE[j][k];
+#pragma unroll
+                            for (int kk = 0; kk < NA; kk++)
+                                if (kk < nadj) vA[kk] = vA[kk] + dC * strain[ij] * P[L.sA + 6 * kk + kl];
                         }
                     }
-                    for (int k = 0; k < nadj; k++) tt[3 * k + 2] = vA[k] * Area * detJac;
+#pragma unroll
+                    for (int k = 0; k < NA; k++)
+                        if (k < nadj) g[k] = g[k] - vA[k] * Area * detJac;
                 }
-                __syncthreads();
-                for (int task = tid; task < 3 * nn; task += nth)
-                    for (int k = 0; k < nadj; k++) {
-                        double g = gi_s[task * nadj + k];
-                        for (int ql = 0; ql < nqc; ql++) {
-                            const double *tt = terms + ((size_t)task * a.qchunk + ql) * 3 * nadj + 3 * k;
-                            g = g - tt[0];
-                            g = g - tt[1];
-                            g = g - tt[2];
-                        }
-                        gi_s[task * nadj + k] = g;
-                    }
+#pragma unroll
+                for (int k = 0; k < NA; k++)
+                    if (k < nadj) gi_s[task * nadj + k] = g[k];
             }
         }
         // ---------------- stage B': body-load work, one task per (control
@@ -612,10 +625,12 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         gi_d = dgi.as<double>();
         ge_d = dge.as<double>();
     }
-    int smem_optin = 0;
+    int smem_optin = 0, nsm = 0;
+    YETI_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     YETI_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     cudaFuncAttributes fattr;
-    YETI_CUDA(cudaFuncGetAttributes(&fattr, k_u1_grad));
+    const auto kernel = nadj == 1 ? k_u1_grad<1> : k_u1_grad<kGradMaxAdj>;
+    YETI_CUDA(cudaFuncGetAttributes(&fattr, kernel));
     smem_optin -= (int)fattr.sharedSizeBytes;   // the kernel's static shared memory
     std::vector<std::unique_ptr<DevBuf>> keep;
     auto newbuf = [&keep]() -> DevBuf & {
@@ -721,23 +736,25 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         g.ege = be.as<double>();
         const PtLayout L = pt_layout(P.nn, (int)nadj, max_body);
         const size_t face = (size_t)P.ng * P.ng * (4 * P.nn + 11 + 3 * nadj);
-        // term buffer of stage B: up to 6144 doubles (48 KB), whole chunks of points
-        const int qchunk = (int)std::max<int64_t>(
-            1, std::min<int64_t>(P.nq, 6144 / (9 * (int64_t)P.nn * nadj)));
-        // point records: all the points when they fit, else the largest
-        // chunk that does (at least the term buffer's)
+        // a thread per (control point, component); point records in chunks
+        // (every sum continues over them) cut for as many CTAs per SM as the
+        // registers allow, but of eight points at least
+        const int threads = std::min(256, std::max(96, (3 * P.nn + 31) / 32 * 32));
+        const int ctas = std::max<int>(1, std::min<int64_t>(kGradThreads / threads, (P.nactive + nsm - 1) / nsm));
+        auto bytes = [&](int n) {
+            return sizeof(double) * grad_smem_doubles(P.nn, n, (int)nadj, L, face, P.ng);
+        };
         int pchunk = P.nq;
-        while (pchunk > qchunk &&
-               sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, qchunk, P.ng) > (size_t)smem_optin)
-            pchunk--;
-        g.qchunk = std::min(qchunk, pchunk);
+        while (pchunk > std::min(8, P.nq) && bytes(pchunk) > (size_t)228 * 1024 / ctas - 1536) pchunk--;
+        while (pchunk > 1 && bytes(pchunk) > (size_t)smem_optin) pchunk--;
+        pchunk = (P.nq + (P.nq + pchunk - 1) / pchunk - 1) / ((P.nq + pchunk - 1) / pchunk);
         g.pchunk = pchunk;
-        const size_t smem = sizeof(double) * grad_smem_doubles(P.nn, pchunk, (int)nadj, L, face, g.qchunk, P.ng);
+        const size_t smem = bytes(pchunk);
         YETI_CHECK(smem <= (size_t)smem_optin, YETI_EUNSUPPORTED,
                    "shape gradient: element needs %zu bytes of shared memory", smem);
-        YETI_TRY(set_smem_optin((const void *)k_u1_grad, ctx->device, smem, "shape gradient element"));
+        YETI_TRY(set_smem_optin((const void *)kernel, ctx->device, smem, "shape gradient element"));
         KernelTimer timer(ctx, "k_u1_grad");
-        k_u1_grad<<<(unsigned)elems.size(), 256, smem, s>>>(g);
+        kernel<<<(unsigned)elems.size(), threads, smem, s>>>(g);
         count_launches(1);
         YETI_CUDA(cudaGetLastError());
     }
