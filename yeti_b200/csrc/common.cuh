@@ -81,7 +81,7 @@ struct yeti_ctx {
 namespace yeti {
 
 constexpr size_t kPoolBytes = size_t(256) << 20;   // most a context keeps of freed blocks
-constexpr size_t kPoolBlock = size_t(64) << 20;    // largest block it keeps
+constexpr size_t kPoolBlock = size_t(128) << 20;   // largest block it keeps
 
 // Device allocation charged against the context budget.  A block may come
 // from the context's pool: its last user's work has been enqueued on the

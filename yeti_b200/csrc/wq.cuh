@@ -88,16 +88,28 @@ struct CGScal {
 // c, the separable operator sum_d a[c][d] K_d (x) M (x) M on the component's
 // free box, inverted through the generalised eigenpairs K_d U = M_d U Lambda
 // of the 1-D WQ matrices; optionally scaled by sqrt(diag(P) / diag(K)).
+// Tilings of the passes (wq_fd.cu): units of rows / columns (nA) in ntA or
+// nsplit tiles, units of lines / rows (nL); ctas -1: not possible.
+struct FdTile {
+    int ntA, nA, nL, ctas, threads;
+    size_t smem;
+};
+struct FdPlane {
+    int nsplit, nA, nL, ctas, threads;
+    size_t smem;
+};
 struct WQFdPlan {
     int variant = -1;          // YETI_PCG_FD bits it was built for (-1: none)
     int lo[3][3], m[3][3];     // free box per [component][direction]
-    int64_t goff[3][3];        // U (fwd) at goff, U^T (bwd) at goff + m*m
+    int64_t goff[2][3][3];     // [FP64, FP32]: U (fwd) at goff, then U^T (bwd)
     int64_t doff[3][3];        // a[c][d] * lambda_d
     bool scaled = false;
     DevBuf g64, g32, d64, d32, s64, s32;   // matrices, eigenvalues, scaling
     DevBuf t64, t32;           // two intermediate vectors
     DevBuf parts;              // partials of the r.z reduction
     int max_grid = 0;
+    FdTile tile[2][4][3];      // [FP64, FP32][u, v, w, fused w][component]
+    FdPlane plane[2][3];
 };
 // FD reduction modes of the last (u, backward) pass.
 enum FdRed { FD_NONE = 0, FD_ITER = 1, FD_START = 2, FD_REPLACE = 3 };

@@ -23,8 +23,9 @@
 // Device work per application: six passes of dense 1-D products along u, v,
 // w (forward with U^T, the eigenvalue division fused into the w pass, then
 // backward with U).  Each pass is a small-K GEMM over the lines of the box,
-// tiled in shared memory (16-deep K chunks, 4x4 register tiles); the
-// vectors (a few MB) stay in L2 between passes.
+// its operands staged whole in shared memory; the vectors (a few MB) stay in
+// L2 between passes.  FP64 runs on the FP64 matrix instructions, FP32 on
+// packed FMAs over 8x8 register tiles (struct FdGemm).
 #include <algorithm>
 #include <cmath>
 #include <deque>
@@ -39,8 +40,7 @@
 namespace yeti {
 
 constexpr int kFdThreads = 256;
-constexpr int kFdTA = 128;     // max output rows per CTA
-constexpr int kFdTL = 128;     // max lines per CTA
+constexpr int kFdTL = 256;     // max lines per CTA
 constexpr int kFdMaxM = 512;   // largest 1-D free size accepted
 constexpr size_t kFdSmem = 200 * 1024;   // staged G and line tiles per CTA
 
@@ -188,147 +188,254 @@ struct FdArgs {
     const int *done;
     CGScal *cg;
     double *parts;
-    int red;
+    int red, vec;      // vec: lines can be copied in 16-byte pieces
     int n[3];
     int64_t ncp;
     int lo[3][3], m[3][3];
     int64_t goff[3];   // per component, for this pass
     int64_t goff2[3];  // fused w pass: the backward matrix
     int64_t doff[3][3];
-    int nag[3], nlg[3], ntA[3], cta_end[3];
+    int nA[3], nL[3], ntA[3], cta_end[3];
 };
 
-// Tiles of one pass for one component: ntA tiles of TA = 4 nag output rows
-// times tiles of TL = 4 nlg lines, the whole contraction (m rows of G and of
-// the lines) staged in shared memory.  The fused w pass (two G matrices)
-// needs one row tile.  Lines per CTA are cut until the pass has at least two
-// CTAs per SM (148 SMs) so that no SM idles behind a neighbour with twice
-// its work.
-struct FdTile {
-    int ntA, nag, nlg, ctas, threads;
-    size_t smem;
-};
-static FdTile fd_tile(int m, int64_t nlines, size_t esize, bool fused) {
-    FdTile t;
-    const int ng = fused ? 2 : 1;
-    t.ntA = fused ? 1 : (m + kFdTA - 1) / kFdTA;
-    auto bytes = [&](int nag, int nlg) {
-        return (size_t)m * (ng * 4 * nag + 4 * nlg + 4) * esize;
-    };
-    auto ctas = [&](int ntA, int nlg) {
-        return ntA * (int)((nlines + 4 * nlg - 1) / (4 * nlg));
-    };
-    for (;;) {
-        t.nag = ((m + t.ntA - 1) / t.ntA + 3) / 4;
-        // the most lines per CTA that still give the pass (three components)
-        // two CTAs per SM
-        int nlg = std::min(kFdTL / 4, kFdThreads / t.nag);
-        while (nlg > 4 && ctas(t.ntA, nlg) < (2 * 148 + 2) / 3) nlg--;
-        while (nlg > 4 && bytes(t.nag, nlg) > kFdSmem) nlg--;
-        t.nlg = nlg;
-        if (bytes(t.nag, nlg) <= kFdSmem || fused) break;
-        t.ntA++;
-    }
-    t.smem = bytes(t.nag, t.nlg);
-    t.ctas = ctas(t.ntA, t.nlg);
-    t.threads = (t.nag * t.nlg + 31) / 32 * 32;
-    if (fused && t.smem > kFdSmem) t.ctas = -1;   // not possible: separate passes
-    return t;
-}
+// The product of a pass on staged operands: out[a][l] = sum_k G[k][a] x(k, l)
+// for the CTA's rows a < kRow nA and lines l < kLine nL, G at Gs[k ldg + a] and x at
+// Xs[k ldx + l] (LK = false) or Xs[l ldx + k] (LK = true); K, rows and lines
+// beyond the data are zero in shared memory.  run() gives the calling
+// thread's outputs to visit, eight at a time, after all have been formed:
+// visit(a, l, v) with the rows, lines and values of the eight (FP32: two
+// groups of four consecutive lines, LK: rows).  `between` runs first (a
+// barrier, when visit overwrites an operand).
+template <class T> struct FdGemm;
 
-template <class T> struct Vec4;
-template <> struct Vec4<float> {
-    static __device__ __forceinline__ void ld(const float *p, float v[4]) {
-        const float4 q = *reinterpret_cast<const float4 *>(p);
-        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+// FP32: a thread per 4 rows (4 ag ..) x 8 lines (LK: lg + nL j; else 4 lg .. and
+// 4 (nL + lg) ..); consecutive threads take consecutive outputs in memory:
+// lines, LK: rows.  The 32 FMAs of a warp take 8 cycles of the SM, the 16-byte
+// loads that feed them 12 wavefronts (4x4 tiles: 8 for 4).  8x8 tiles balance
+// the two (16 and 16), but leave 64^3 elements five warps per SM, which the
+// latency of a step then bounds: 26 us for the plane pass against 22 us.
+template <>
+struct FdGemm<float> {
+    static constexpr int kRow = 4, kLine = 8;   // rows / lines per unit of nA / nL
+    __host__ __device__ static int threads(int nA, int nL) { return (nA * nL + 31) / 32 * 32; }
+    __host__ __device__ static int ldg(int nA) { return 4 * nA; }
+    __host__ __device__ static int ldx(int m, int nL, bool lk) {
+        // LK: a multiple of 4 floats, odd in units of 4 (bank groups of 8 lanes)
+        return lk ? ((m + 3) / 4 | 1) * 4 : 8 * nL;
     }
-};
-template <> struct Vec4<double> {
-    static __device__ __forceinline__ void ld(const double *p, double v[4]) {
-        const double2 q0 = *reinterpret_cast<const double2 *>(p);
-        const double2 q1 = *reinterpret_cast<const double2 *>(p + 2);
-        v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-    }
-};
 
-template <class T>
-__device__ __forceinline__ void fma44(T acc[4][4], const T g[4], const T x[4]) {
+    template <bool LK, class B, class V>
+    static __device__ __forceinline__ void run(const float *Gs, int ldg, const float *Xs, int ldx,
+                                               int m4, int nA, int nL, B between, V visit) {
+        const int t0 = LK ? nA : nL, fast = threadIdx.x % t0, slow = threadIdx.x / t0;
+        const int lg = LK ? slow : fast, ag = LK ? fast : slow;
+        const bool act = slow < (LK ? nL : nA);
+        // LK: rows in pairs, acc[line][row / 2]; else lines in pairs,
+        // acc[line / 2 + 4 (row / 2)][row % 2]
+        float2 acc[8][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+        for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
+        auto ld = [](const float *p) { return *reinterpret_cast<const float4 *>(p); };
+        if (act && LK) {
+            const float *g0 = Gs + 4 * ag, *xp = Xs + lg * ldx;
+            const int js = nL * ldx;
+            for (int k = 0; k < m4; k += 4) {
+                float4 x4[8], g[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] += g[i] * x[j];
-}
-
-// FP32: the 4x4 tile as pairs of columns on packed FP32x2 FMAs (each lane
-// of a pair is the scalar FMA acc += g x, so the sums keep their bits).
-__device__ __forceinline__ void fma44_2(float2 acc[4][2], const float g[4], const float2 x[2]) {
+                for (int j = 0; j < 8; j++) x4[j] = ld(xp + j * js + k);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float2 gg = make_float2(g[i], g[i]);
-        acc[i][0] = __ffma2_rn(gg, x[0], acc[i][0]);
-        acc[i][1] = __ffma2_rn(gg, x[1], acc[i][1]);
-    }
-}
-
-// acc[i][j] = sum_{k < m} gp[k ldg + i] xp[k ldx + j], the next row's
-// operands loaded while the current row's products issue.
-__device__ __forceinline__ void fd_contract(const float *gp, int ldg, const float *xp, int ldx,
-                                            int m, float acc[4][4]) {
-    float2 a2[4][2];
+                for (int kk = 0; kk < 4; kk++) g[kk] = ld(g0 + (k + kk) * ldg);
 #pragma unroll
-    for (int i = 0; i < 4; i++) a2[i][0] = a2[i][1] = make_float2(0.f, 0.f);
-    float g0[4], g1[4];
-    float2 x0[2], x1[2];
-    auto ldx2 = [](const float *p, float2 v[2]) {
-        const float4 q = *reinterpret_cast<const float4 *>(p);
-        v[0] = make_float2(q.x, q.y);
-        v[1] = make_float2(q.z, q.w);
-    };
-    Vec4<float>::ld(gp, g0);
-    ldx2(xp, x0);
-    int k = 0;
-    for (; k + 1 < m; k += 2) {
-        Vec4<float>::ld(gp + (k + 1) * ldg, g1);
-        ldx2(xp + (k + 1) * ldx, x1);
-        fma44_2(a2, g0, x0);
-        if (k + 2 < m) {
-            Vec4<float>::ld(gp + (k + 2) * ldg, g0);
-            ldx2(xp + (k + 2) * ldx, x0);
+                for (int kk = 0; kk < 4; kk++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float x = kk == 0 ? x4[j].x : kk == 1 ? x4[j].y : kk == 2 ? x4[j].z : x4[j].w;
+                        acc[j][0] = __ffma2_rn(make_float2(g[kk].x, g[kk].y), make_float2(x, x), acc[j][0]);
+                        acc[j][1] = __ffma2_rn(make_float2(g[kk].z, g[kk].w), make_float2(x, x), acc[j][1]);
+                    }
+            }
         }
-        fma44_2(a2, g1, x1);
-    }
-    if (k < m) fma44_2(a2, g0, x0);
+        if (act && !LK) {
+            const float *g0 = Gs + 4 * ag, *x0 = Xs + 4 * lg, *x1 = x0 + 4 * nL;
+#pragma unroll 4
+            for (int k = 0; k < m4; k++) {
+                const float4 g = ld(g0 + k * ldg), xa = ld(x0 + k * ldx), xb = ld(x1 + k * ldx);
+                const float2 x[4] = {{xa.x, xa.y}, {xa.z, xa.w}, {xb.x, xb.y}, {xb.z, xb.w}};
+                const float gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        acc[i][0] = a2[i][0].x;
-        acc[i][1] = a2[i][0].y;
-        acc[i][2] = a2[i][1].x;
-        acc[i][3] = a2[i][1].y;
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        acc[j + 4 * (i / 2)][i % 2] =
+                            __ffma2_rn(make_float2(gv[i], gv[i]), x[j], acc[j + 4 * (i / 2)][i % 2]);
+            }
+        }
+        between();
+        if (!act) return;
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+            int a[8], l[8];
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                // LK: lines 2 o, 2 o + 1 with four rows each; else row o with its lines
+                const int i = LK ? e % 4 : o, j = LK ? 2 * o + e / 4 : e;
+                a[e] = 4 * ag + i;
+                l[e] = LK ? lg + nL * j : (j < 4 ? 4 * lg : 4 * (nL + lg) - 4) + j;
+                const float2 p = LK ? acc[j][i / 2] : acc[j / 2 + 4 * (i / 2)][i % 2];
+                v[e] = (LK ? i : j) & 1 ? p.y : p.x;
+            }
+            visit(a, l, v);
+        }
     }
+};
+
+// d += a b on the FP64 matrix instruction (8x4 times 4x8): lane holds
+// a[lane / 4][lane % 4], b[lane % 4][lane / 4] and d[lane / 4][2 (lane % 4) + {0, 1}].
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
 }
 
-template <class T>
-__device__ __forceinline__ void fd_contract(const T *gp, int ldg, const T *xp, int ldx, int m,
-                                            T acc[4][4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = T(0);
-    T g0[4], x0[4], g1[4], x1[4];
-    Vec4<T>::ld(gp, g0);
-    Vec4<T>::ld(xp, x0);
-    int k = 0;
-    for (; k + 1 < m; k += 2) {
-        Vec4<T>::ld(gp + (k + 1) * ldg, g1);
-        Vec4<T>::ld(xp + (k + 1) * ldx, x1);
-        fma44(acc, g0, x0);
-        if (k + 2 < m) {
-            Vec4<T>::ld(gp + (k + 2) * ldg, g0);
-            Vec4<T>::ld(xp + (k + 2) * ldx, x0);
-        }
-        fma44(acc, g1, x1);
+// FP64: a warp per block of 16 rows x 16 lines, blocks dealt out in turn
+// (at most kBlocks per warp).  Bound by the FP64 pipe: the four matrix
+// instructions of four k take 16 cycles of the SM, their eight wavefronts of
+// operands 8; a 4x4 register tile on scalar FMAs took 16 wavefronts for 8
+// cycles of FMAs.  Leading dimensions are 4 or 12 modulo 16 doubles, so that the
+// 4 x 4 doubles a half warp reads lie on distinct banks.  Measured on B200
+// (u + v + w + v + u of one application): 64^3 p=3 177 -> 80 us, 21x17x25 p=3 (two
+// plane passes and w) 42 -> 18 us; FP32 128x128x32 p=4 218 -> 138 us.
+template <>
+struct FdGemm<double> {
+    static constexpr int kRow = 16, kLine = 16, kBlocks = 4;
+    __host__ __device__ static int threads(int nA, int nL) {
+        const int w = nA * nL;
+        return 32 * (w <= 8 ? w : 8);
     }
-    if (k < m) fma44(acc, g0, x0);
+    __host__ __device__ static int ldg(int nA) { return 16 * nA + 4; }
+    __host__ __device__ static int ldx(int m, int nL, bool lk) {
+        const int m4 = (m + 3) / 4 * 4;
+        return !lk ? 16 * nL + 4 : m4 % 8 ? m4 : m4 + 4;
+    }
+
+    template <bool LK, class B, class V>
+    static __device__ __forceinline__ void run(const double *Gs, int ldg, const double *Xs, int ldx,
+                                               int m4, int nA, int nL, B between, V visit) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+        const int r = lane >> 2, q = lane & 3;
+        double acc[kBlocks][2][2][2];
+#pragma unroll
+        for (int b = 0; b < kBlocks; b++) {
+            const int blk = warp + b * nwarp;
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) acc[b][i][j][0] = acc[b][i][j][1] = 0.0;
+            if (blk >= nA * nL) continue;
+            const int ab = blk / nL, lb = blk - ab * nL;
+            const double *g = Gs + q * ldg + 16 * ab + r;
+            const double *x = LK ? Xs + (16 * lb + r) * ldx + q : Xs + q * ldx + 16 * lb + r;
+            const int xj = LK ? 8 * ldx : 8, xk = LK ? 1 : ldx;
+#pragma unroll 4
+            for (int k = 0; k < m4; k += 4) {
+                const double a0 = g[k * ldg], a1 = g[k * ldg + 8];
+                const double b0 = x[k * xk], b1 = x[k * xk + xj];
+                dmma(acc[b][0][0], a0, b0);
+                dmma(acc[b][0][1], a0, b1);
+                dmma(acc[b][1][0], a1, b0);
+                dmma(acc[b][1][1], a1, b1);
+            }
+        }
+        between();
+#pragma unroll
+        for (int b = 0; b < kBlocks; b++) {
+            const int blk = warp + b * nwarp;
+            if (blk >= nA * nL) continue;
+            const int ab = blk / nL, lb = blk - ab * nL;
+            int a[8], l[8];
+            double v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const int i = e >> 2, j = e >> 1 & 1;
+                a[e] = 16 * ab + 8 * i + r;
+                l[e] = 16 * lb + 8 * j + 2 * q + (e & 1);
+                v[e] = acc[b][i][j][e & 1];
+            }
+            visit(a, l, v);
+        }
+    }
+};
+// Largest number of units nA nL of a CTA.
+template <class T>
+constexpr int kFdUnits = sizeof(T) == 4 ? kFdThreads : 8 * FdGemm<double>::kBlocks;
+
+// Least threads of a CTA.  FP64 CTAs of small patches have a few blocks only:
+// the other warps help to stage the operands (21x17x25 p=3: plane pass 5.9 ->
+// 5.3 us, w pass 7.4 -> 6.6 us); in FP32 they cost the 64^3 plane pass 1 us.
+template <class T>
+constexpr int kFdLeast = sizeof(T) == 4 ? 32 : kFdThreads;
+
+// m rounded up to whole steps of the contractions.
+__host__ __device__ inline int fd_m4(int m) { return (m + 3) / 4 * 4; }
+// Leading dimension of the 1-D matrices in global memory: that of a staged
+// matrix with all its rows in one tile, so that it is copied as one run.
+template <class T>
+__host__ __device__ inline int fd_ldm(int m) {
+    return FdGemm<T>::ldg((m + FdGemm<T>::kRow - 1) / FdGemm<T>::kRow);
+}
+// Elements of such a matrix (zero rows up to fd_m4(m)).
+template <class T>
+__host__ __device__ inline int64_t fd_matrix(int m) {
+    return (int64_t)fd_m4(m) * fd_ldm<T>(m);
+}
+
+// Tiles of one pass for one component: nA units of rows (ntA row tiles) and
+// nL units of lines per CTA, the whole contraction staged in shared memory.
+// The fused w pass (two G matrices) needs one row tile.  Of the tilings
+// that fit, the one whose busiest SM has the least work (units, in whole
+// warps) is taken, counting the CTAs that share an SM; ties go to the larger
+// tile, which reads G less often.
+template <class T>
+static FdTile fd_tile(int m, int64_t nlines, bool lk, bool fused) {
+    using Gm = FdGemm<T>;
+    const int m4 = fd_m4(m), units = (m + Gm::kRow - 1) / Gm::kRow;
+    FdTile best;
+    best.ctas = -1;
+    double best_cost = 0.0;
+    for (int ntA = 1; ntA <= (fused ? 1 : units); ntA++) {
+        const int nA = (units + ntA - 1) / ntA;
+        for (int nL = 1; nL * Gm::kLine <= kFdTL && nA * nL <= kFdUnits<T>; nL++) {
+            FdTile t;
+            t.ntA = ntA;
+            t.nA = nA;
+            t.nL = nL;
+            const size_t g = (size_t)m4 * Gm::ldg(nA) * (fused ? 2 : 1);
+            const int ldx = Gm::ldx(m, nL, lk);
+            const size_t x = lk ? (size_t)nL * Gm::kLine * ldx
+                                : (size_t)(fused ? std::max(m4, nA * Gm::kRow) : m4) * ldx;
+            t.smem = (g + x) * sizeof(T);
+            if (t.smem > kFdSmem) continue;
+            t.threads = Gm::threads(nA, nL);
+            t.ctas = ntA * (int)((nlines + nL * Gm::kLine - 1) / (nL * Gm::kLine));
+            // three components share the SMs
+            const double per_sm = std::ceil(3.0 * t.ctas / 148.0);
+            const double resident = std::max(1.0, std::min(std::floor(227.0 * 1024 / (t.smem + 8192)),
+                                                           std::floor(512.0 / t.threads)));
+            const double work = sizeof(T) == 4 ? t.threads / 32 : nA * nL;
+            // units on the busiest SM (four schedulers take them in
+            // fours); a round of CTAs also pays its loads
+            const double rounds = std::ceil(per_sm / resident);
+            const double cost = std::ceil(per_sm * work / 4.0) * 4.0 + rounds * 2.0;
+            if (best.ctas < 0 || cost < best_cost - 1e-9 ||
+                (cost < best_cost + 1e-9 && nA * nL > best.nA * best.nL)) {
+                best = t;
+                best_cost = cost;
+            }
+        }
+        if (best.ctas > 0 && ntA >= 4) break;
+    }
+    return best;   // ctas -1: not possible
 }
 
 // Asynchronous global -> shared copy of one element (cp.async, sm_80+);
@@ -339,6 +446,84 @@ __device__ __forceinline__ void cp_elem(T *sdst, const T *gsrc, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(saddr), "l"(gsrc),
                  "n"((int)sizeof(T)), "r"(valid ? (int)sizeof(T) : 0)
                  : "memory");
+}
+// 16 bytes (both addresses 16-byte aligned), of which the first n elements
+// are read and the rest written as zero.
+template <class T>
+__device__ __forceinline__ void cp_vec(T *sdst, const T *gsrc, int n) {
+    const unsigned saddr = (unsigned)__cvta_generic_to_shared(sdst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(gsrc),
+                 "r"(n * (int)sizeof(T))
+                 : "memory");
+}
+// Four consecutive values; aligned: one 16-byte store.
+__device__ __forceinline__ void store4(float *o, const float *v, bool aligned) {
+    if (aligned) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+    else
+#pragma unroll
+        for (int e = 0; e < 4; e++) o[e] = v[e];
+}
+__device__ __forceinline__ void store4(double *o, const double *v, bool) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = v[e];
+}
+
+// The last step of a pass for eight outputs of a thread at idx (-1: none):
+// EPI 2 scales, adds to r.z and sets p.  Loads first: the stores that follow
+// would each be waited for.  Four consecutive outputs (FP32) go out as one
+// store where they are aligned.
+template <class T, int EPI>
+__device__ __forceinline__ void fd_write(const FdArgs<T> &a, const int64_t (&idx)[8], T (&v)[8],
+                                         double &rz) {
+    if (EPI == 2) {
+        T sv[8], rv[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            sv[e] = a.s && idx[e] >= 0 ? __ldg(a.s + idx[e]) : T(1);
+            rv[e] = a.red != FD_NONE && idx[e] >= 0 ? __ldg(a.r + idx[e]) : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            if (a.s) v[e] *= sv[e];
+            if (a.red != FD_NONE && idx[e] >= 0) rz += (double)rv[e] * (double)v[e];
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+        const bool run = sizeof(T) == 4 && idx[h] >= 0 && idx[h + 3] == idx[h] + 3 && idx[h + 1] == idx[h] + 1;
+        if (run) {
+            store4(a.out + idx[h], v + h, (reinterpret_cast<uintptr_t>(a.out + idx[h]) & 15) == 0);
+            if (EPI == 2 && a.red == FD_START)
+                store4(a.p + idx[h], v + h, (reinterpret_cast<uintptr_t>(a.p + idx[h]) & 15) == 0);
+        } else {
+#pragma unroll
+            for (int e = h; e < h + 4; e++) {
+                if (idx[e] < 0) continue;
+                a.out[idx[e]] = v[e];
+                if (EPI == 2 && a.red == FD_START) a.p[idx[e]] = v[e];
+            }
+        }
+    }
+}
+
+// Columns a0 .. a0 + n of a 1-D matrix into Gs[k ldg + a], k < fd_m4(m); zero
+// beyond the data, in 16-byte pieces, consecutive threads on consecutive
+// ones (the whole matrix as one run).
+template <class T>
+__device__ __forceinline__ void stage_matrix(T *Gs, int ldg, const T *G, int m, int a0, int n) {
+    constexpr int VEC = 16 / sizeof(T);
+    const int ldm = fd_ldm<T>(m);
+    if (a0 == 0 && ldg == ldm) {
+        const int tot = fd_m4(m) * ldm;
+        for (int t = threadIdx.x * VEC; t < tot; t += blockDim.x * VEC) cp_vec(Gs + t, G + t, VEC);
+        return;
+    }
+    const int nv = n / VEC, tot = fd_m4(m) * nv;
+    for (int t = threadIdx.x; t < tot; t += blockDim.x) {
+        const int k = t / nv, a = (t - k * nv) * VEC;
+        const bool in = a0 + a < ldm;
+        cp_vec(Gs + k * ldg + a, in ? G + (int64_t)k * ldm + a0 + a : G, in ? VEC : 0);
+    }
 }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
@@ -372,143 +557,115 @@ __device__ __forceinline__ void fd_finish_rz(const FdArgs<T> &a, double rz, doub
 // reduction mode; EPI 3 (AX == 2, one row tile): forward product, division
 // by Lambda and backward product in one CTA, the intermediate kept in shared
 // memory.  The G columns and the lines are staged by cp.async (all copies in
-// flight at once), then contracted from shared memory.
+// flight at once): lines along u as they lie in memory (LK), the others with
+// the lines consecutive.
 template <class T, int AX, int EPI>
-__global__ void __launch_bounds__(kFdThreads) k_fd_pass(FdArgs<T> a) {
+__global__ void __launch_bounds__(kFdThreads, sizeof(T) == 4 ? 3 : 2) k_fd_pass(FdArgs<T> a) {
+    using Gm = FdGemm<T>;
+    constexpr bool LK = AX == 0;
     extern __shared__ __align__(16) unsigned char fd_smem[];
     __shared__ int64_t lb[kFdTL];
-    __shared__ int2 lc[kFdTL];   // (i1, i2) of a line
+    __shared__ T ll12[kFdTL];    // EPI 1, 3: the line's part of Lambda
     __shared__ double sh[32];
     if (a.done && *a.done) return;
     int b = blockIdx.x, c = 0;
     while (c < 2 && b >= a.cta_end[c]) c++;
     if (c > 0) b -= a.cta_end[c - 1];
     constexpr int D1 = AX == 0 ? 1 : 0, D2 = AX == 2 ? 1 : 2;
-    const int nag = a.nag[c], nlg = a.nlg[c], ntA = a.ntA[c];
-    const int m = a.m[c][AX], m1 = a.m[c][D1], m2 = a.m[c][D2];
-    const int64_t nlines = (int64_t)m1 * m2;
-    const int TA = 4 * nag, TL = 4 * nlg, TLp = TL + 4;
-    T *Gs = reinterpret_cast<T *>(fd_smem);    // [m][TA]
-    T *G2 = Gs + (size_t)m * TA;               // EPI 3: [m][TA]
-    T *Xs = EPI == 3 ? G2 + (size_t)m * TA : G2;   // [m][TLp]
+    const int nA = a.nA[c], nL = a.nL[c], ntA = a.ntA[c];
+    const int m = a.m[c][AX], m1 = a.m[c][D1], m2 = a.m[c][D2], m4 = fd_m4(m);
+    const int nlines = m1 * m2;
+    const int TA = Gm::kRow * nA, TL = Gm::kLine * nL, ldg = Gm::ldg(nA), ldx = Gm::ldx(m, nL, LK);
+    T *Gs = reinterpret_cast<T *>(fd_smem);
+    T *G2 = Gs + (size_t)m4 * ldg;                     // EPI 3
+    T *Xs = EPI == 3 ? G2 + (size_t)m4 * ldg : G2;
     const int a0 = (b % ntA) * TA;
-    const int64_t l0 = (int64_t)(b / ntA) * TL;
+    const int l0 = (b / ntA) * TL;
     const int64_t st[3] = {1, (int64_t)a.n[0], (int64_t)a.n[0] * a.n[1]};
     const int64_t sk = st[AX];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nthr = blockDim.x, nwarp = nthr >> 5;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    stage_matrix(Gs, ldg, a.g + a.goff[c], m, a0, TA);
+    if (EPI == 3) stage_matrix(G2, ldg, a.g + a.goff2[c], m, 0, TA);
     for (int ll = tid; ll < TL; ll += nthr) {
-        const int64_t l = l0 + ll;
+        const int l = l0 + ll;
         int64_t base = -1;
         int i1 = 0, i2 = 0;
         if (l < nlines) {
-            i1 = (int)(l % m1);
-            i2 = (int)(l / m1);
+            i2 = l / m1;
+            i1 = l - i2 * m1;
             base = c * a.ncp + (int64_t)a.lo[c][AX] * sk + (int64_t)(a.lo[c][D1] + i1) * st[D1] +
                    (int64_t)(a.lo[c][D2] + i2) * st[D2];
         }
         lb[ll] = base;
-        lc[ll] = make_int2(i1, i2);
-    }
-    // G columns a0 .. a0 + TA of every row k (a warp per row)
-    const T *G = a.g + a.goff[c];
-    for (int k = warp; k < m; k += nwarp) {
-        const T *src = G + (int64_t)k * m;
-        for (int aa = lane; aa < TA; aa += 32) {
-            const int col = a0 + aa;
-            cp_elem(Gs + k * TA + aa, col < m ? src + col : G, col < m);
-        }
-    }
-    if (EPI == 3) {
-        const T *Gb = a.g + a.goff2[c];
-        for (int k = warp; k < m; k += nwarp) {
-            const T *src = Gb + (int64_t)k * m;
-            for (int aa = lane; aa < TA; aa += 32)
-                cp_elem(G2 + k * TA + aa, aa < m ? src + aa : Gb, aa < m);
-        }
+        if (EPI == 1 || EPI == 3)
+            ll12[ll] = base >= 0 ? a.dsc[a.doff[c][D1] + i1] + a.dsc[a.doff[c][D2] + i2] : T(1);
     }
     __syncthreads();   // lb
-    if (AX == 0) {
-        // lines are contiguous: a warp per line, lanes along k
-        for (int ll = warp; ll < TL; ll += nwarp) {
+    constexpr int VEC = 16 / sizeof(T);
+    if (LK) {
+        // lines are contiguous: a warp per line, in 16-byte pieces when every
+        // line begins on one
+        for (int ll = tid >> 5; ll < TL; ll += nthr >> 5) {
             const int64_t base = lb[ll];
-            for (int k = lane; k < m; k += 32)
-                cp_elem(Xs + k * TLp + ll, base >= 0 ? a.in + base + k : a.in, base >= 0);
+            const T *src = base >= 0 ? a.in + base : a.in;
+            if (a.vec)
+                for (int k = (tid & 31) * VEC; k < m4; k += 32 * VEC)
+                    cp_vec(Xs + ll * ldx + k, src + k, base >= 0 ? min(VEC, m - k) : 0);
+            else
+                for (int k = tid & 31; k < m4; k += 32)
+                    cp_elem(Xs + ll * ldx + k, k < m ? src + k : src, base >= 0 && k < m);
+        }
+    } else if (a.vec) {
+        // row k of the tile is contiguous along the lines of a run, and the
+        // runs are whole 16-byte pieces
+        const int nv = TL / VEC;
+        for (int t = tid; t < nv * m4; t += nthr) {
+            const int k = t / nv, ll = (t - k * nv) * VEC;
+            const int64_t base = lb[ll];
+            const bool in = base >= 0 && k < m;
+            cp_vec(Xs + k * ldx + ll, in ? a.in + base + (int64_t)k * sk : a.in, in ? VEC : 0);
         }
     } else {
-        // row k of the tile is contiguous along the lines: a warp per row
-        for (int k = warp; k < m; k += nwarp) {
-            for (int ll = lane; ll < TL; ll += 32) {
-                const int64_t base = lb[ll];
-                cp_elem(Xs + k * TLp + ll, base >= 0 ? a.in + base + (int64_t)k * sk : a.in,
-                        base >= 0);
-            }
+        for (int t = tid; t < TL * m4; t += nthr) {
+            const int k = t / TL, ll = t - k * TL;
+            const int64_t base = lb[ll];
+            const bool in = base >= 0 && k < m;
+            cp_elem(Xs + k * ldx + ll, in ? a.in + base + (int64_t)k * sk : a.in, in);
         }
     }
     cp_wait_all();
     __syncthreads();
-    int ag, lg;
-    if (AX == 0) {
-        ag = tid % nag;
-        lg = tid / nag;
-    } else {
-        lg = tid % nlg;
-        ag = tid / nlg;
-    }
-    const bool act = tid < nag * nlg;
-    T acc[4][4];
-    if (act) fd_contract(Gs + 4 * ag, TA, Xs + 4 * lg, TLp, m, acc);
-    if (EPI == 3) {
-        // divide by Lambda, park the eigen-space values in Xs, contract back
-        __syncthreads();
-        if (act) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int e = 4 * ag + i;
-                if (e >= m) continue;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int ll = 4 * lg + j;
-                    const int2 q = lc[ll];
-                    const T lam = a.dsc[a.doff[c][0] + q.x] + a.dsc[a.doff[c][1] + q.y] +
-                                  a.dsc[a.doff[c][2] + e];
-                    Xs[e * TLp + ll] = lb[ll] >= 0 ? acc[i][j] / lam : T(0);
-                }
-            }
-        }
-        __syncthreads();
-        if (act) fd_contract(G2 + 4 * ag, TA, Xs + 4 * lg, TLp, m, acc);
-    }
     double rz = 0.0;
-    if (act) {
+    // Lambda of (row e, line ll); AX == 2: (lambda_u + lambda_v) + lambda_w
+    static_assert(AX == 2 || (EPI != 1 && EPI != 3), "the division belongs to the w pass");
+    auto lambda = [&](int e, int ll) { return ll12[ll] + __ldg(a.dsc + a.doff[c][2] + e); };
+    auto write = [&](const int (&row)[8], const int (&ll)[8], T (&v)[8]) {
+        int64_t idx[8];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int row = a0 + 4 * ag + i;
-            if (row >= m) continue;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int ll = 4 * lg + j;
-                const int64_t base = lb[ll];
-                if (base < 0) continue;
-                const int64_t idx = base + (int64_t)row * sk;
-                T v = acc[i][j];
-                if (EPI == 1) {
-                    int e3[3];
-                    e3[AX] = row;
-                    e3[D1] = lc[ll].x;
-                    e3[D2] = lc[ll].y;
-                    const T lam = a.dsc[a.doff[c][0] + e3[0]] + a.dsc[a.doff[c][1] + e3[1]] +
-                                  a.dsc[a.doff[c][2] + e3[2]];
-                    v = v / lam;
-                }
-                if (EPI == 2) {
-                    if (a.s) v *= a.s[idx];
-                    if (a.red != FD_NONE) rz += (double)a.r[idx] * (double)v;
-                    if (a.red == FD_START) a.p[idx] = v;
-                }
-                a.out[idx] = v;
-            }
+        for (int e = 0; e < 8; e++) {
+            const int64_t base = lb[ll[e]];
+            idx[e] = a0 + row[e] < m && base >= 0 ? base + (int64_t)(a0 + row[e]) * sk : -1;
+            if (EPI == 1 && idx[e] >= 0) v[e] = v[e] / lambda(a0 + row[e], ll[e]);
         }
+        fd_write<T, EPI>(a, idx, v, rz);
+    };
+    auto nothing = [] {};
+    if constexpr (EPI == 3) {
+        // divide by Lambda, park the eigen-space values in Xs, contract back
+        Gm::template run<false>(
+            Gs, ldg, Xs, ldx, m4, nA, nL, [] { __syncthreads(); },
+            [&](const int (&row)[8], const int (&ll)[8], T (&v)[8]) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    if (row[e] >= m4) continue;
+                    const bool in = row[e] < m && lb[ll[e]] >= 0;
+                    Xs[row[e] * ldx + ll[e]] = in ? v[e] / lambda(row[e], ll[e]) : T(0);
+                }
+            });
+        __syncthreads();
+        Gm::template run<false>(G2, ldg, Xs, ldx, m4, nA, nL, nothing, write);
+    } else {
+        Gm::template run<LK>(Gs, ldg, Xs, ldx, m4, nA, nL, nothing, write);
     }
     if (EPI != 2 || a.red == FD_NONE) return;
     fd_finish_rz(a, rz, sh);
@@ -518,86 +675,65 @@ __global__ void __launch_bounds__(kFdThreads) k_fd_pass(FdArgs<T> a) {
 // (rows v, columns u of the component's free box),
 //     T[v][a] = sum_i X[v][i] Gu[i][a],   Y[b][a] = sum_j Gv[j][b] T[j][a],
 // forward (Gu = U_u, Gv = U_v; in positions, out eigen indices) or backward
-// (Gu = U_u^T, Gv = U_v^T).  The plane, Gu's columns of the CTA's column
-// split, Gv and T stay in shared memory.  goff: Gu, goff2: Gv; ntA: column
-// splits, nag: 4-column groups per split, nlg: 4-row groups (ceil(m_v / 4)).
-// EPI 2 as k_fd_pass.
+// (Gu = U_u^T, Gv = U_v^T).  The plane (rows as they lie in memory), Gu's
+// columns of the CTA's column split, Gv and T stay in shared memory.  goff:
+// Gu, goff2: Gv; ntA: column splits, nA: units of columns per split, nL: units
+// of rows.  EPI 2 as k_fd_pass.
 template <class T, int EPI>
-__global__ void __launch_bounds__(kFdThreads) k_fd_plane(FdArgs<T> a) {
+__global__ void __launch_bounds__(kFdThreads, sizeof(T) == 4 ? 3 : 2) k_fd_plane(FdArgs<T> a) {
+    using Gm = FdGemm<T>;
     extern __shared__ __align__(16) unsigned char fd_smem[];
     __shared__ double sh[32];
     if (a.done && *a.done) return;
     int b = blockIdx.x, c = 0;
     while (c < 2 && b >= a.cta_end[c]) c++;
     if (c > 0) b -= a.cta_end[c - 1];
-    const int mu = a.m[c][0], mv = a.m[c][1];
-    const int nsplit = a.ntA[c], nag = a.nag[c], nvg = a.nlg[c];
-    const int TA = 4 * nag, ldv = 4 * nvg + 4, ldb = 4 * nvg;
+    const int mu = a.m[c][0], mv = a.m[c][1], mu4 = fd_m4(mu), mv4 = fd_m4(mv);
+    const int nsplit = a.ntA[c], nA = a.nA[c], nL = a.nL[c];
     const int sp = b % nsplit, kw = b / nsplit;
-    const int a0 = sp * TA;
-    T *Xt = reinterpret_cast<T *>(fd_smem);   // [mu][ldv]: X transposed
-    T *Gu = Xt + (size_t)mu * ldv;            // [mu][TA]
-    T *Gv = Gu + (size_t)mu * TA;             // [mv][ldb]
-    T *Tm = Gv + (size_t)mv * ldb;            // [mv][TA]
+    const int TA = Gm::kRow * nA, TB = Gm::kLine * nL, a0 = sp * TA;
+    const int ldx = Gm::ldx(mu, nL, true), ldu = Gm::ldg(nA), ldv = Gm::ldg(TB / Gm::kRow),
+              ldt = Gm::ldx(mv, TA / Gm::kLine, false);
+    T *Xs = reinterpret_cast<T *>(fd_smem);       // [TB][ldx]: X[v][i]
+    T *Gu = Xs + (size_t)TB * ldx;                // [mu4][ldu]
+    T *Gv = Gu + (size_t)mu4 * ldu;               // [mv4][ldv]
+    T *Tm = Gv + (size_t)mv4 * ldv;               // [TB][ldt]: T[v][a]
     const int64_t nu = a.n[0], nv = a.n[1];
     const int64_t plane = c * a.ncp + (int64_t)(a.lo[c][2] + kw) * nu * nv +
                           (int64_t)a.lo[c][1] * nu + a.lo[c][0];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarp = blockDim.x >> 5;
-    // the plane, a warp per row v (contiguous along u); rows mv .. 4 nvg zero
-    for (int v = warp; v < 4 * nvg; v += nwarp) {
-        const T *src = a.in + plane + (int64_t)v * nu;
-        for (int i = lane; i < mu; i += 32)
-            cp_elem(Xt + i * ldv + v, v < mv ? src + i : a.in, v < mv);
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    // the plane, a warp per row v (contiguous along u); rows mv .. TB zero
+    constexpr int VEC = 16 / sizeof(T);
+    for (int v = tid >> 5; v < TB; v += nthr >> 5) {
+        const T *src = v < mv ? a.in + plane + v * nu : a.in;
+        if (a.vec)
+            for (int i = (tid & 31) * VEC; i < mu4; i += 32 * VEC)
+                cp_vec(Xs + v * ldx + i, src + i, v < mv ? min(VEC, mu - i) : 0);
+        else
+            for (int i = tid & 31; i < mu4; i += 32)
+                cp_elem(Xs + v * ldx + i, i < mu ? src + i : src, v < mv && i < mu);
     }
-    const T *G = a.g + a.goff[c];
-    for (int i = warp; i < mu; i += nwarp)
-        for (int aa = lane; aa < TA; aa += 32) {
-            const int col = a0 + aa;
-            cp_elem(Gu + i * TA + aa, col < mu ? G + (int64_t)i * mu + col : G, col < mu);
-        }
-    const T *H = a.g + a.goff2[c];
-    for (int j = warp; j < mv; j += nwarp)
-        for (int bb = lane; bb < ldb; bb += 32)
-            cp_elem(Gv + j * ldb + bb, bb < mv ? H + (int64_t)j * mv + bb : H, bb < mv);
+    stage_matrix(Gu, ldu, a.g + a.goff[c], mu, a0, TA);
+    stage_matrix(Gv, ldv, a.g + a.goff2[c], mv, 0, TB);
     cp_wait_all();
     __syncthreads();
-    const int ag = tid % nag, vg = tid / nag;
-    const bool act = vg < nvg;
-    T acc[4][4];
-    if (act) {
-        fd_contract(Xt + 4 * vg, ldv, Gu + 4 * ag, TA, mu, acc);
+    Gm::template run<true>(Gu, ldu, Xs, ldx, mu4, nA, nL, [] {},
+                           [&](const int (&col)[8], const int (&v)[8], T (&t)[8]) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int v = 4 * vg + i;
-            if (v < mv)
-#pragma unroll
-                for (int j = 0; j < 4; j++) Tm[v * TA + 4 * ag + j] = acc[i][j];
-        }
-    }
+                               for (int e = 0; e < 8; e++) Tm[v[e] * ldt + col[e]] = t[e];
+                           });
     __syncthreads();
     double rz = 0.0;
-    if (act) {
-        fd_contract(Gv + 4 * vg, ldb, Tm + 4 * ag, TA, mv, acc);
+    Gm::template run<false>(Gv, ldv, Tm, ldt, mv4, TB / Gm::kRow, TA / Gm::kLine, [] {},
+                            [&](const int (&row)[8], const int (&col)[8], T (&v)[8]) {
+                                int64_t idx[8];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int row = 4 * vg + i;
-            if (row >= mv) continue;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int col = a0 + 4 * ag + j;
-                if (4 * ag + j >= TA || col >= mu) continue;
-                const int64_t idx = plane + (int64_t)row * nu + col;
-                T v = acc[i][j];
-                if (EPI == 2) {
-                    if (a.s) v *= a.s[idx];
-                    if (a.red != FD_NONE) rz += (double)a.r[idx] * (double)v;
-                    if (a.red == FD_START) a.p[idx] = v;
-                }
-                a.out[idx] = v;
-            }
-        }
-    }
+                                for (int e = 0; e < 8; e++)
+                                    idx[e] = row[e] < mv && a0 + col[e] < mu
+                                                 ? plane + (int64_t)row[e] * nu + a0 + col[e]
+                                                 : -1;
+                                fd_write<T, EPI>(a, idx, v, rz);
+                            });
     if (EPI != 2 || a.red == FD_NONE) return;
     fd_finish_rz(a, rz, sh);
 }
@@ -633,32 +769,32 @@ __global__ void k_fd_scaling(const double *diagK, const double *kdmd, double *s6
 
 // ------------------------------------------------------------------ plan
 // Tiling of the fused plane pass for one component: column splits of the
-// u products (each CTA recomputes nothing, it reads the whole plane), at
-// most 256 threads, the staged plane, Gu columns, Gv and T within kFdSmem,
-// and splits added while the pass (three components) has fewer than two
-// CTAs per SM.  ctas = -1: does not fit (the line passes run instead).
-struct FdPlane {
-    int nsplit, nag, nvg, ctas, threads;
-    size_t smem;
-};
-static FdPlane fd_plane_tile(int mu, int mv, int mw, size_t esize) {
-    FdPlane t;
-    t.nvg = (mv + 3) / 4;
-    t.ctas = -1;
-    const int ldv = 4 * t.nvg + 4, ldb = 4 * t.nvg;
-    bool ok = false;
-    for (t.nsplit = 1; t.nsplit <= mu; t.nsplit++) {
-        t.nag = ((mu + t.nsplit - 1) / t.nsplit + 3) / 4;
-        const int TA = 4 * t.nag;
-        t.smem = ((size_t)mu * ldv + (size_t)mu * TA + (size_t)mv * ldb + (size_t)mv * TA) * esize;
-        if (t.nag * t.nvg > kFdThreads || t.smem > kFdSmem) continue;
-        ok = true;
-        if (3 * mw * t.nsplit >= 2 * 148 || t.nag <= 2) break;
+// u products (each CTA recomputes nothing, it reads the whole plane), with
+// the staged plane, Gu columns, Gv and T within kFdSmem, and splits added while
+// the pass (three components) has fewer CTAs than SMs.  ctas = -1: does not
+// fit (the line passes run instead).
+template <class T>
+static FdPlane fd_plane_tile(int mu, int mv, int mw) {
+    using Gm = FdGemm<T>;
+    // rows and lines change roles between the products: whole units of both
+    constexpr int per = std::max(1, Gm::kLine / Gm::kRow);
+    const int units = (mu + Gm::kRow - 1) / Gm::kRow;
+    FdPlane t, best;
+    best.ctas = -1;
+    t.nL = (mv + Gm::kLine - 1) / Gm::kLine;
+    const int TB = Gm::kLine * t.nL;
+    for (t.nsplit = 1; t.nsplit <= units; t.nsplit++) {
+        t.nA = ((units + t.nsplit - 1) / t.nsplit + per - 1) / per * per;
+        t.smem = ((size_t)TB * Gm::ldx(mu, t.nL, true) + (size_t)fd_m4(mu) * Gm::ldg(t.nA) +
+                  (size_t)fd_m4(mv) * Gm::ldg(TB / Gm::kRow) +
+                  (size_t)TB * Gm::ldx(mv, t.nA * Gm::kRow / Gm::kLine, false)) * sizeof(T);
+        if (t.nA * t.nL > kFdUnits<T> || t.smem > kFdSmem) continue;
+        t.ctas = mw * t.nsplit;
+        t.threads = std::max(Gm::threads(t.nA, t.nL), kFdLeast<T>);
+        best = t;
+        if (3 * t.ctas >= 148) break;
     }
-    if (!ok) return t;
-    t.ctas = mw * t.nsplit;
-    t.threads = (t.nag * t.nvg + 31) / 32 * 32;
-    return t;
+    return best;
 }
 
 template <class T>
@@ -807,6 +943,42 @@ __global__ void k_fd_diag_coef_blk(const double *coef, const int64_t *qoff,
             for (int k = 0; k < 3; k++)
                 out[(int64_t)(3 * c + k) * n + g] = base[(int64_t)sym9(3 * c + k, 3 * c + k) * nqb];
     }
+}
+
+// U, then U^T (m x m, row-major), appended to g in the layout of the passes.
+template <class T>
+static void add_matrices(const std::vector<double> &U, int m, std::vector<T> &g, int64_t &off) {
+    const int ldm = fd_ldm<T>(m);
+    off = (int64_t)g.size();
+    g.resize(g.size() + 2 * fd_matrix<T>(m), T(0));
+    T *u = &g[off], *ut = u + fd_matrix<T>(m);
+    for (int i = 0; i < m; i++)
+        for (int j = 0; j < m; j++)
+            u[(size_t)i * ldm + j] = ut[(size_t)j * ldm + i] = (T)U[(size_t)i * m + j];
+}
+
+// The tilings of every pass; returns the most CTAs of a pass (partials of its
+// reduction).
+template <class T>
+static int fd_plan_tiles(WQFdPlan &F) {
+    const int w = sizeof(T) == 4;
+    int most = 0;
+    for (int ps = 0; ps < 4; ps++) {   // u, v, w, fused w
+        const int ax = std::min(ps, 2);
+        int tot = 0;
+        for (int c = 0; c < 3; c++) {
+            F.tile[w][ps][c] = fd_tile<T>(F.m[c][ax], (int64_t)F.m[c][ax == 0 ? 1 : 0] *
+                                                          F.m[c][ax == 2 ? 1 : 2], ax == 0, ps == 3);
+            tot += std::max(0, F.tile[w][ps][c].ctas);
+        }
+        most = std::max(most, tot);
+    }
+    int tot = 0;
+    for (int c = 0; c < 3; c++) {
+        F.plane[w][c] = fd_plane_tile<T>(F.m[c][0], F.m[c][1], F.m[c][2]);
+        tot += std::max(0, F.plane[w][c].ctas);
+    }
+    return std::max(most, tot);
 }
 
 int wq_fd_prepare(yeti_wq_op *op, int variant, bool f32) {
@@ -995,27 +1167,26 @@ int wq_fd_prepare(yeti_wq_op *op, int variant, bool f32) {
                    "fast diagonalisation: separable operator of component %d is singular", c);
     }
     // device tables: G (U then U^T) per (c, d); a * lambda; 1-D diagonals
-    std::vector<double> g, dsc, kdmd;
+    std::vector<double> g64, dsc, kdmd;
+    std::vector<float> g32;
     for (int c = 0; c < 3; c++)
         for (int d = 0; d < 3; d++) {
             const int m = F.m[c][d];
             const Eig &e = *E[c][d];
-            F.goff[c][d] = (int64_t)g.size();
-            g.insert(g.end(), e.U.begin(), e.U.end());
-            for (int i = 0; i < m; i++)
-                for (int j = 0; j < m; j++) g.push_back(e.U[(size_t)j * m + i]);
+            add_matrices<double>(e.U, m, g64, F.goff[0][c][d]);
+            if (f32) add_matrices<float>(e.U, m, g32, F.goff[1][c][d]);
             F.doff[c][d] = (int64_t)dsc.size();
             for (int i = 0; i < m; i++) dsc.push_back(acoef[c][d] * e.lam[i]);
             for (int i = 0; i < m; i++) kdmd.push_back(e.kd[i]);
             for (int i = 0; i < m; i++) kdmd.push_back(e.md[i]);
         }
-    YETI_TRY(upload(ctx, F.g64, g.data(), g.size()));
+    YETI_TRY(upload(ctx, F.g64, g64.data(), g64.size()));
     YETI_TRY(upload(ctx, F.d64, dsc.data(), dsc.size()));
     F.g32.release();
     F.d32.release();
     if (f32) {
-        std::vector<float> gf(g.begin(), g.end()), df(dsc.begin(), dsc.end());
-        YETI_TRY(upload(ctx, F.g32, gf.data(), gf.size()));
+        std::vector<float> df(dsc.begin(), dsc.end());
+        YETI_TRY(upload(ctx, F.g32, g32.data(), g32.size()));
         YETI_TRY(upload(ctx, F.d32, df.data(), df.size()));
     }
     // scaling vector
@@ -1048,25 +1219,8 @@ int wq_fd_prepare(yeti_wq_op *op, int variant, bool f32) {
     YETI_TRY(F.t64.alloc(ctx, 2 * op->ndof * sizeof(double)));
     F.t32.release();
     if (f32) YETI_TRY(F.t32.alloc(ctx, 2 * op->ndof * sizeof(float)));
-    int maxg = 0;
-    for (int ax = 0; ax < 3; ax++)
-        for (int fused = 0; fused < 2; fused++) {
-            int tot = 0;
-            for (int c = 0; c < 3; c++) {
-                const int64_t nl = (int64_t)F.m[c][(ax == 0) ? 1 : 0] * F.m[c][(ax == 2) ? 1 : 2];
-                for (size_t es : {sizeof(double), sizeof(float)})
-                    tot += std::max(0, fd_tile(F.m[c][ax], nl, es, fused).ctas);
-            }
-            maxg = std::max(maxg, tot);
-        }
-    for (size_t es : {sizeof(double), sizeof(float)}) {
-        int tot = 0;
-        for (int c = 0; c < 3; c++)
-            tot += std::max(0, fd_plane_tile(F.m[c][0], F.m[c][1], F.m[c][2], es).ctas);
-        maxg = std::max(maxg, tot);
-    }
-    F.max_grid = maxg;
-    YETI_TRY(F.parts.alloc(ctx, (size_t)maxg * sizeof(double)));
+    F.max_grid = std::max(fd_plan_tiles<double>(F), fd_plan_tiles<float>(F));
+    YETI_TRY(F.parts.alloc(ctx, (size_t)F.max_grid * sizeof(double)));
     // the tables were uploaded (and, on a stream-ordered context,
     // allocated) on the context's stream; solves may run on other streams
     YETI_CUDA(cudaStreamSynchronize(s));
@@ -1093,24 +1247,30 @@ static int fd_pass(yeti_wq_op *op, FdArgs<T> a, bool bwd, cudaStream_t s) {
     const WQFdPlan &F = op->fd;
     int tot = 0, threads = 32;
     size_t smem = 0;
+    // 16-byte copies of the lines: rows begin on 16 bytes, and where lines are
+    // consecutive their runs along u are whole pieces
+    constexpr int VEC = 16 / sizeof(T);
+    bool vec = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0 && op->n[0] % VEC == 0;
     for (int c = 0; c < 3; c++) {
         const int m = F.m[c][AX];
-        const int64_t nl = (int64_t)F.m[c][AX == 0 ? 1 : 0] * F.m[c][AX == 2 ? 1 : 2];
-        const FdTile t = fd_tile(m, nl, sizeof(T), EPI == 3);
+        const FdTile &t = F.tile[sizeof(T) == 4][EPI == 3 ? 3 : AX][c];
         YETI_CHECK(t.ctas > 0, YETI_EINVAL, "fast diagonalisation: no tiling for m=%d", m);
-        a.nag[c] = t.nag;
-        a.nlg[c] = t.nlg;
+        a.nA[c] = t.nA;
+        a.nL[c] = t.nL;
         a.ntA[c] = t.ntA;
         tot += t.ctas;
         a.cta_end[c] = tot;
-        a.goff[c] = F.goff[c][AX] + (bwd ? (int64_t)m * m : 0);
-        a.goff2[c] = F.goff[c][AX] + (int64_t)m * m;
+        const int64_t off = F.goff[sizeof(T) == 4][c][AX];
+        a.goff[c] = off + (bwd ? fd_matrix<T>(m) : 0);
+        a.goff2[c] = off + fd_matrix<T>(m);
         smem = std::max(smem, t.smem);
-        threads = std::max(threads, t.threads);
+        threads = std::max(std::max(threads, t.threads), kFdLeast<T>);
+        vec = vec && (AX == 0 || F.m[c][0] % VEC == 0) && F.lo[c][0] % VEC == 0;
     }
-    // every component's tile fits `threads` (nag nlg <= threads).  The
-    // shared-memory opt-in (the 48 KB default covers static plus dynamic
-    // memory) is set by wq_fd_prepare on this device, outside any capture
+    a.vec = vec;
+    // every component's units fit `threads`.  The shared-memory opt-in (the
+    // 48 KB default covers static plus dynamic memory) is set by
+    // wq_fd_prepare on this device, outside any capture
     k_fd_pass<T, AX, EPI><<<tot, threads, smem, s>>>(a);
     count_launches(1);
     return YETI_OK;
@@ -1122,32 +1282,38 @@ static int fd_plane(yeti_wq_op *op, FdArgs<T> a, bool bwd, cudaStream_t s) {
     const WQFdPlan &F = op->fd;
     int tot = 0, threads = 32;
     size_t smem = 0;
+    constexpr int VEC = 16 / sizeof(T);
+    bool vec = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0 && op->n[0] % VEC == 0;
     for (int c = 0; c < 3; c++) {
         const int mu = F.m[c][0], mv = F.m[c][1];
-        const FdPlane t = fd_plane_tile(mu, mv, F.m[c][2], sizeof(T));
+        const FdPlane &t = F.plane[sizeof(T) == 4][c];
         YETI_CHECK(t.ctas > 0, YETI_EINVAL, "fast diagonalisation: plane %dx%d does not fit", mu, mv);
         a.ntA[c] = t.nsplit;
-        a.nag[c] = t.nag;
-        a.nlg[c] = t.nvg;
+        a.nA[c] = t.nA;
+        a.nL[c] = t.nL;
         tot += t.ctas;
         a.cta_end[c] = tot;
-        a.goff[c] = F.goff[c][0] + (bwd ? (int64_t)mu * mu : 0);
-        a.goff2[c] = F.goff[c][1] + (bwd ? (int64_t)mv * mv : 0);
+        const int64_t *off = F.goff[sizeof(T) == 4][c];
+        a.goff[c] = off[0] + (bwd ? fd_matrix<T>(mu) : 0);
+        a.goff2[c] = off[1] + (bwd ? fd_matrix<T>(mv) : 0);
         smem = std::max(smem, t.smem);
         threads = std::max(threads, t.threads);
+        vec = vec && F.lo[c][0] % VEC == 0;
     }
+    a.vec = vec;
     k_fd_plane<T, EPI><<<tot, threads, smem, s>>>(a);
     count_launches(1);
     return YETI_OK;
 }
 
 // The fused plane pass pays off when its tile leaves room for two CTAs per
-// SM (measured at 64^3: FP32, 57 KB, 24 us against 2 x 16.5 us for the two
-// line passes; FP64, 114 KB, one CTA per SM, 63 us against 2 x 29 us).
+// SM (64^3: FP32, 79 KB, 22 us against two line passes of 13 us or more each;
+// FP64, 158 KB, one CTA per SM, takes the line passes, 12.4 us each).
 constexpr size_t kFdPlaneSmem = 100 * 1024;
-static bool fd_planes_fit(const WQFdPlan &F, size_t esize) {
+template <class T>
+static bool fd_planes_fit(const WQFdPlan &F) {
     for (int c = 0; c < 3; c++) {
-        const FdPlane t = fd_plane_tile(F.m[c][0], F.m[c][1], F.m[c][2], esize);
+        const FdPlane &t = F.plane[sizeof(T) == 4][c];
         if (t.ctas <= 0 || t.smem > kFdPlaneSmem) return false;
     }
     return true;
@@ -1155,11 +1321,10 @@ static bool fd_planes_fit(const WQFdPlan &F, size_t esize) {
 
 // The w pass can run fused (forward, division, backward in one CTA) when
 // every component's w tile is a single row tile that fits.
-static bool fd_w_fused(const WQFdPlan &F, size_t esize) {
-    for (int c = 0; c < 3; c++) {
-        if (F.m[c][2] > kFdTA) return false;
-        if (fd_tile(F.m[c][2], (int64_t)F.m[c][0] * F.m[c][1], esize, true).ctas <= 0) return false;
-    }
+template <class T>
+static bool fd_w_fused(const WQFdPlan &F) {
+    for (int c = 0; c < 3; c++)
+        if (F.tile[sizeof(T) == 4][3][c].ctas <= 0) return false;
     return true;
 }
 
@@ -1193,7 +1358,7 @@ int wq_fd_apply(yeti_wq_op *op, const T *in, T *out, const int *done, int red, T
         count_launches(1);
         a.in = t1;
     }
-    if (fd_planes_fit(F, sizeof(T)) && fd_w_fused(F, sizeof(T))) {
+    if (fd_planes_fit<T>(F) && fd_w_fused<T>(F)) {
         // three launches: u and v forward per plane, w, u and v backward
         a.out = t0;
         YETI_TRY((fd_plane<T, 0>(op, a, false, s)));
@@ -1213,7 +1378,7 @@ int wq_fd_apply(yeti_wq_op *op, const T *in, T *out, const int *done, int red, T
     YETI_TRY((fd_pass<T, 1, 0>(op, a, false, s)));
     a.in = t1;
     a.out = t0;
-    if (fd_w_fused(F, sizeof(T))) {
+    if (fd_w_fused<T>(F)) {
         YETI_TRY((fd_pass<T, 2, 3>(op, a, false, s)));
     } else {
         YETI_TRY((fd_pass<T, 2, 1>(op, a, false, s)));
