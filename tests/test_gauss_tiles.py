@@ -78,3 +78,31 @@ def test_gpu_gradient_of_one_to_four_adjoints_matches_oracle(cuda_ok, nadj, nel,
     for got, ref in zip(grad_from_system_args(args, sol, adj),
                         oracle.grad_lin_elast_work(args, sol, adj)):
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("keep", [1.0, 0.7, 0.3])
+def test_gpu_models_with_inactive_elements(cuda_ok, keep):
+    """All, most and few of the elements active: the connectivity is used as it
+    comes, gathered on the device, or gathered on the host."""
+    from yeti_b200._lib import YetiError
+    from yeti_b200.gradient import grad_from_system_args
+    args = u1_system_args(cube_patch((4, 3, 3), 2, perturb=0.1, wrange=(0.8, 1.2), seed=4),
+                          rho=1.0, clamp_u0=True, load_u1=(2, 1.5))
+    act = (np.random.default_rng(8).random(36) < keep).astype(np.int64)
+    args[0] = act
+    for got, ref in zip(sys_linmat_lindef_static(*args), oracle.sys_linmat_lindef_static(*args)):
+        np.testing.assert_array_equal(got, ref)
+    sol = 0.01 * np.random.default_rng(3).standard_normal((3, args[2].shape[1]))
+    for got, ref in zip(grad_from_system_args(args, sol, sol[None]),
+                        oracle.grad_lin_elast_work(args, sol, sol[None])):
+        np.testing.assert_array_equal(got, ref)
+    e = int(np.flatnonzero(act)[1])
+    for wrong in (0, args[2].shape[1] + 1):
+        bad = list(args)
+        bad[3] = np.array(args[3])
+        bad[3][27 * e + 5] = wrong
+        with pytest.raises(YetiError, match=f"IEN entry {wrong} of element {e + 1} out of range"):
+            sys_linmat_lindef_static(*bad)
+    for got, ref in zip(sys_linmat_lindef_static(*args), oracle.sys_linmat_lindef_static(*args)):
+        np.testing.assert_array_equal(got, ref)

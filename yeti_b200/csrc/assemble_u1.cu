@@ -162,6 +162,29 @@ void gauss_face_host(int n, int face, std::vector<double> &g) {
 }
 
 // ------------------------------------------------------------ model preparing
+// The caller's 64-bit 1-based connectivity of a patch as 32-bit 0-based
+// control points of its active elements (gid: their global ids, nullptr: all
+// of the patch's), and the weights where elements are left out (w !=
+// nullptr).  An entry outside 1..nb_cp becomes 0 and its index in the
+// connectivity (ien_off + ...) goes to *bad if it is the first.
+__global__ void k_u1_unpack(const int64_t *raw, const double *raw_w, const int32_t *gid,
+                            int64_t elem_begin, int64_t n, int nn, int64_t nb_cp, int64_t ien_off,
+                            int32_t *ien, double *w, unsigned long long *bad) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        int64_t src = t;
+        if (gid) {
+            const int64_t k = t / nn;
+            src = (gid[k] - elem_begin) * nn + (t - k * nn);
+        }
+        const int64_t cp = raw[src];
+        const bool ok = cp >= 1 && cp <= nb_cp;
+        if (!ok) atomicMin(bad, (unsigned long long)(ien_off + src));
+        ien[t] = ok ? (int32_t)(cp - 1) : 0;
+        if (w) w[t] = raw_w[src];
+    }
+}
+
 int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
     YETI_CHECK(m && m->coords && m->ien && m->nb_elem_patch && m->nkv &&
                    m->ukv && m->nijk && m->weight && m->jpqr && m->nnode &&
@@ -173,6 +196,7 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
     out.patches.resize(m->nb_patch);
     out.nb_cp = m->nb_cp;
     UploadPack pack;
+    std::vector<int64_t> ien_offs(m->nb_patch, 0);
     int64_t jelem = 0, ukv_off = 0, ien_off = 0, count = 0;
     for (int64_t ip = 0; ip < m->nb_patch; ip++) {
         U1Patch &P = out.patches[ip];
@@ -213,8 +237,12 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
         P.rho = m->rho ? m->rho[ip] : 0.0;
         P.nb_data_elem = 9LL * P.nn * (P.nn - 1) / 2 + 6LL * P.nn;
         const int nn = P.nn;
-        std::vector<int32_t> ien(nact * nn), span(nact * 3), gid;
-        std::vector<double> w(nact * nn);
+        // a patch with most of its elements active goes up as it is and is
+        // converted on the device; of one with few, only those
+        const bool sparse = 2 * nact < P.nelem;
+        std::vector<int32_t> ien(sparse ? nact * nn : 0), span(nact * 3), gid;
+        std::vector<double> w(sparse ? nact * nn : 0);
+        ien_offs[ip] = ien_off;
         P.act.reserve(nact);
         P.slot.reserve(nact);
         gid.reserve(nact);
@@ -225,7 +253,7 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
             P.slot.push_back(count);
             count += P.nb_data_elem;
             gid.push_back((int32_t)jelem);
-            for (int a = 0; a < nn; a++) {
+            for (int a = 0; sparse && a < nn; a++) {
                 int64_t cp = m->ien[ien_off + e * nn + a];
                 YETI_CHECK(cp >= 1 && cp <= m->nb_cp, YETI_EINVAL,
                            "IEN entry %lld of element %lld out of range",
@@ -248,8 +276,10 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
             std::vector<double> g;
             gauss_volume_host(P.ng, g);
             pack.add(P.gauss, g);
-            pack.add(P.ien, ien);
-            pack.add(P.w, w);
+            if (sparse) {
+                pack.add(P.ien, ien);
+                pack.add(P.w, w);
+            }
             pack.add(P.span, span);
             pack.add(P.slotd, P.slot);
             pack.add(P.gid, gid);
@@ -262,7 +292,44 @@ int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out) {
                (long long)jelem, (long long)m->nb_elem);
     out.nb_data = count;
     pack.add(out.coords, m->coords, (size_t)3 * m->nb_cp);
-    return pack.commit(ctx, out.arena);
+    const unsigned long long none = ~0ull;
+    DevBuf bad;
+    pack.add(bad, &none, 1);
+    YETI_TRY(pack.commit(ctx, out.arena));
+    bool any = false;
+    for (int64_t ip = 0; ip < m->nb_patch; ip++) {
+        U1Patch &P = out.patches[ip];
+        if (!P.nactive || P.ien.ptr) continue;
+        any = true;
+        const bool all = P.nactive == P.nelem;
+        const int64_t nraw = P.nelem * P.nn, n = P.nactive * P.nn;
+        YETI_TRY(upload(ctx, P.raw_ien, m->ien + ien_offs[ip], nraw));
+        YETI_TRY(upload(ctx, P.raw_w, m->weight + ien_offs[ip], nraw));
+        YETI_TRY(P.conv.alloc(ctx, n * sizeof(int32_t) + 256 + (all ? 0 : n * sizeof(double))));
+        double *w = all ? nullptr : P.conv.as<double>();
+        int32_t *ien = reinterpret_cast<int32_t *>(P.conv.as<char>() + (all ? 0 : n * sizeof(double)));
+        k_u1_unpack<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, ctx->stream>>>(
+            P.raw_ien.as<int64_t>(), P.raw_w.as<double>(), all ? nullptr : P.gid.as<int32_t>(),
+            P.elem_begin, n, P.nn, m->nb_cp, ien_offs[ip], ien, w, bad.as<unsigned long long>());
+        count_launches(1);
+        YETI_CUDA(cudaGetLastError());
+        P.ien.view(ien, n * sizeof(int32_t));
+        P.w.view(all ? P.raw_w.ptr : w, n * sizeof(double));
+    }
+    if (any) {
+        unsigned long long first = none;
+        YETI_CUDA(cudaMemcpyAsync(&first, bad.ptr, sizeof(first), cudaMemcpyDeviceToHost, ctx->stream));
+        YETI_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (first != none) {
+            int64_t ip = m->nb_patch - 1;
+            while (ip > 0 && (int64_t)first < ien_offs[ip]) ip--;
+            const U1Patch &P = out.patches[ip];
+            YETI_CHECK(false, YETI_EINVAL, "IEN entry %lld of element %lld out of range",
+                       (long long)m->ien[first],
+                       (long long)(P.elem_begin + ((int64_t)first - ien_offs[ip]) / P.nn + 1));
+        }
+    }
+    return YETI_OK;
 }
 
 // ---------------------------------------------------------------- kernels

@@ -582,16 +582,19 @@ __global__ void __launch_bounds__(256, NA == 1 ? 2 : 1) k_u1_grad(GradArgs a) {
     }
 }
 
-// g[k + nadj*(c + 3*cp)] = sum over elements (in order) of their entries
-__global__ void k_grad_gather(int64_t n, const int64_t *ptr, const int64_t *idx,
+// g[k + nadj*(c + 3*cp)] = sum over elements (in order) of their entries; per =
+// 3 nadj values of a control point, idx: the first of an element's
+__global__ void k_grad_gather(int64_t n, int per, const int64_t *ptr, const int64_t *idx,
                               const double *egi, const double *ege, double *gi,
                               double *ge) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= n) return;
     double ai = 0.0, ae = 0.0;
-    for (int64_t k = ptr[t]; k < ptr[t + 1]; k++) {
-        ai = ai + egi[idx[k]];
-        ae = ae + ege[idx[k]];
+    const int64_t cp = t / per;
+    const int r = (int)(t - cp * per);
+    for (int64_t k = ptr[cp]; k < ptr[cp + 1]; k++) {
+        ai = ai + egi[idx[k] + r];
+        ae = ae + ege[idx[k] + r];
     }
     gi[t] = ai;
     ge[t] = ae;
@@ -758,46 +761,48 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         count_launches(1);
         YETI_CUDA(cudaGetLastError());
     }
-    // gather per (adjoint, component, control point) in element order
+    // gather per (adjoint, component, control point) in element order: the
+    // patches' element entries one after the other
     DevBuf &ai = newbuf();
     DevBuf &ae = newbuf();
-    YETI_TRY(ai.alloc(ctx, sizeof(double) * std::max<int64_t>(etotal, 1)));
-    YETI_TRY(ae.alloc(ctx, sizeof(double) * std::max<int64_t>(etotal, 1)));
-    {
+    const double *ai_d = nullptr, *ae_d = nullptr;
+    if (ebufs_i.size() == 1) {
+        ai_d = ebufs_i[0]->as<double>();
+        ae_d = ebufs_e[0]->as<double>();
+    } else {
+        YETI_TRY(ai.alloc(ctx, sizeof(double) * std::max<int64_t>(etotal, 1)));
+        YETI_TRY(ae.alloc(ctx, sizeof(double) * std::max<int64_t>(etotal, 1)));
         int64_t off = 0;
         for (size_t i = 0; i < ebufs_i.size(); i++) {
             YETI_CUDA(cudaMemcpyAsync(ai.as<double>() + off, ebufs_i[i]->ptr, ebufs_i[i]->bytes, cudaMemcpyDeviceToDevice, s));
             YETI_CUDA(cudaMemcpyAsync(ae.as<double>() + off, ebufs_e[i]->ptr, ebufs_e[i]->bytes, cudaMemcpyDeviceToDevice, s));
             off += (int64_t)(ebufs_i[i]->bytes / sizeof(double));
         }
+        ai_d = ai.as<double>();
+        ae_d = ae.as<double>();
     }
-    // CSR of the element entries of each output, elements in order: count,
-    // then fill in the same loop order
-    std::vector<int64_t> ptr(nout + 1, 0);
+    // CSR of the element entries of each control point (the first of its 3 nadj
+    // values), elements in order: count, then fill in the same loop order
+    std::vector<int64_t> ptr(ncp + 1, 0);
     auto walk = [&](auto &&visit) {
         for (auto &D : done) {
             const U1Patch &P = M.patches[D.patch];
             const int64_t jel = P.act[D.local];
-            const int64_t base = ien_offset[D.patch] + (jel - P.elem_begin) * P.nn;
-            for (int a = 0; a < P.nn; a++) {
-                const int64_t cp = m->ien[base + a] - 1;
-                for (int c = 0; c < 3; c++)
-                    for (int k = 0; k < nadj; k++)
-                        visit(k + nadj * (c + 3 * cp), D.off + k + nadj * (c + 3 * a));
-            }
+            const int64_t *ien = m->ien + ien_offset[D.patch] + (jel - P.elem_begin) * P.nn;
+            for (int a = 0; a < P.nn; a++) visit(ien[a] - 1, D.off + 3 * nadj * a);
         }
     };
-    walk([&](int64_t o, int64_t) { ptr[o + 1]++; });
-    for (int64_t i = 0; i < nout; i++) ptr[i + 1] += ptr[i];
-    std::vector<int64_t> idx(std::max<int64_t>(ptr[nout], 1), 0), fill(ptr.begin(), ptr.end() - 1);
-    walk([&](int64_t o, int64_t e) { idx[fill[o]++] = e; });
+    walk([&](int64_t cp, int64_t) { ptr[cp + 1]++; });
+    for (int64_t i = 0; i < ncp; i++) ptr[i + 1] += ptr[i];
+    std::vector<int64_t> idx(std::max<int64_t>(ptr[ncp], 1), 0), fill(ptr.begin(), ptr.end() - 1);
+    walk([&](int64_t cp, int64_t e) { idx[fill[cp]++] = e; });
     DevBuf &garena = newbuf(), &dptr = newbuf(), &didx = newbuf();
     UploadPack gpack;
     gpack.add(dptr, ptr);
     gpack.add(didx, idx);
     YETI_TRY(gpack.commit(ctx, garena));
     k_grad_gather<<<(unsigned)((nout + 255) / 256), 256, 0, s>>>(
-        nout, dptr.as<int64_t>(), didx.as<int64_t>(), ai.as<double>(), ae.as<double>(), gi_d, ge_d);
+        nout, 3 * (int)nadj, dptr.as<int64_t>(), didx.as<int64_t>(), ai_d, ae_d, gi_d, ge_d);
     count_launches(1);
     YETI_CUDA(cudaGetLastError());
     if (!compute_wint) YETI_CUDA(cudaMemsetAsync(gi_d, 0, nout * sizeof(double), s));

@@ -29,6 +29,8 @@ struct U1Patch {
     DevBuf span;    // nactive * 3, int32 1-based knot span
     DevBuf slotd;   // nactive, int64 slot offsets
     DevBuf gid;     // nactive, int32 global element ids
+    // the caller's connectivity and weights of the patch, as they came (owned)
+    DevBuf raw_ien, raw_w, conv;
 };
 
 struct U1Model {
