@@ -33,3 +33,38 @@ def test_gpu_apply_over_cut_plane_ranges(cuda_ok, nel, p):
     assert np.linalg.norm(k1 - k0) < 1e-12 * np.linalg.norm(k0)
     k2 = op.eval_Ku(u.astype(np.float32), precision="f32").astype(np.float64)
     assert np.linalg.norm(k2 - k0) < 2e-6 * np.linalg.norm(k0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nel,p,prec", [((6, 5, 7), 3, "f64"), ((8, 8, 8), 2, "f32"),
+                                        ((31, 19, 23), 4, "f64")])
+def test_gpu_applies_in_a_row_on_device_vectors(cuda_ok, nel, p, prec):
+    """The output of one apply as the input of the next without a
+    synchronisation, into arrays that begin off 16-byte boundaries and hold
+    other values: the zeroing of an output must neither start before the
+    apply that fills its input is done nor end after the additions begin."""
+    import torch
+    from yeti_b200 import _lib
+    from yeti_b200.wq import WQElasticity
+    ctx = _lib.Context(0)
+    ctx.set_stream(torch.cuda.current_stream())
+    op = WQElasticity(cube_patch(nel, p, perturb=0.1, seed=3), 1.0, 0.3, {"w0": (0, 1, 2)}, ctx=ctx)
+    dt = torch.float64 if prec == "f64" else torch.float32
+    n = op.ndof
+    u = torch.from_numpy(np.random.default_rng(5).standard_normal(n)).to(dt).cuda()
+    ref = [u.cpu().numpy()]
+    for _ in range(4):                   # host buffers: each call synchronises
+        ref.append(op.eval_Ku(ref[-1], precision=prec))
+    bar = 1e-13 if prec == "f64" else 1e-5
+    for off in (0, 1):
+        bufs = [torch.full((n + 4,), 7.0, dtype=dt, device="cuda") for _ in range(4)]
+        src = u
+        for b in bufs:
+            op.apply_device(src, b[off:off + n], prec)
+            src = b[off:off + n]
+        torch.cuda.synchronize()
+        for b, r in zip(bufs, ref[1:]):
+            got = b[off:off + n].cpu().numpy()
+            assert np.linalg.norm(got - r) < bar * np.linalg.norm(r)
+            assert float(b[off + n]) == 7.0
+    ctx.set_stream(None)

@@ -678,6 +678,16 @@ int wq_apply_dev(yeti_wq_op *op, const void *u, void *Ku, int prec,
     return launch_apply<float>(op, (const float *)u, (float *)Ku, done, s);
 }
 
+int wq_apply_new(yeti_wq_op *op, const void *u, void *Ku, int prec, cudaStream_t s) {
+    if (op->st.active) {
+        if (prec == YETI_PREC_F64)
+            return wq_stream_apply<double>(op, (const double *)u, (double *)Ku, nullptr, s, true);
+        return wq_stream_apply<float>(op, (const float *)u, (float *)Ku, nullptr, s, true);
+    }
+    YETI_CUDA(cudaMemsetAsync(Ku, 0, op->ndof * (prec == YETI_PREC_F64 ? 8 : 4), s));
+    return wq_apply_dev(op, u, Ku, prec, nullptr, s);
+}
+
 }  // namespace yeti
 
 using namespace yeti;
@@ -919,8 +929,7 @@ YETI_API int yeti_wq_apply(yeti_wq_op *op, const void *u, void *Ku, int prec,
         uu = du.ptr;
         kk = dk.ptr;
     }
-    YETI_CUDA(cudaMemsetAsync(kk, 0, nb, s));
-    YETI_TRY(wq_apply_dev(op, uu, kk, prec, nullptr, s));
+    YETI_TRY(wq_apply_new(op, uu, kk, prec, s));
     if (mem == YETI_MEM_HOST) {
         YETI_CUDA(cudaMemcpyAsync(Ku, kk, nb, cudaMemcpyDeviceToHost, s));
         YETI_CUDA(cudaStreamSynchronize(s));

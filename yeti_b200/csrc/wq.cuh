@@ -64,6 +64,7 @@ struct WQStreamPlan {
     bool active = false;     // coefficients are in the streaming layout
     int ntile[2] = {0, 0};   // (u, v) tiles
     int grid[2] = {0, 0};
+    bool beside[2] = {false, false};   // start beside the zeroing of Ku
     int per_sm[2] = {0, 0};
     size_t smem[2] = {0, 0};
     int64_t ncoef = 0;
@@ -133,7 +134,8 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]);
 // layout (after every kernel that reads the element-block layout).
 int wq_stream_permute(yeti_wq_op *op);
 template <class T>
-int wq_stream_apply(yeti_wq_op *op, const T *u, T *Ku, const int *done, cudaStream_t s);
+int wq_stream_apply(yeti_wq_op *op, const T *u, T *Ku, const int *done, cudaStream_t s,
+                    bool zeroed = false);
 // One FP64 preconditioned Krylov solve (CG or BiCGSTAB; Jacobi or fast
 // diagonalisation) of a WQ operator (x0 = 0) that advances in
 // chunks of iterations captured once in a CUDA graph, on its own stream and
@@ -187,6 +189,8 @@ int wq_stream_check(yeti_wq_op *op);
 // optional device flag, the kernel returns at once when it is set.
 int wq_apply_dev(yeti_wq_op *op, const void *u, void *Ku, int prec,
                  const int *done, cudaStream_t s);
+// Enqueue Ku = K u on stream s (u and Ku distinct).
+int wq_apply_new(yeti_wq_op *op, const void *u, void *Ku, int prec, cudaStream_t s);
 }  // namespace yeti
 
 // The operator object behind the opaque yeti_wq_op handle.
