@@ -68,3 +68,32 @@ def test_gpu_applies_in_a_row_on_device_vectors(cuda_ok, nel, p, prec):
             assert np.linalg.norm(got - r) < bar * np.linalg.norm(r)
             assert float(b[off + n]) == 7.0
     ctx.set_stream(None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("method", ["cg", "bicgstab"])
+def test_gpu_solves_from_zero_and_from_another_start(cuda_ok, method, mixed):
+    """The start residual is b itself from x0 = 0 and b - K x0 otherwise, also
+    when x0 holds a single tiny entry or a NaN; the residual that a mixed solve
+    ends on is the one reported."""
+    from yeti_b200._lib import YetiError
+    from yeti_b200.wq import WQElasticity
+    op = WQElasticity(cube_patch((6, 5, 7), 3, perturb=0.1, wrange=(0.8, 1.2), seed=3), 1.0, 0.3,
+                      {"w0": (0, 1, 2)})
+    b = op.eval_bodyforce_vector([0.1, -0.2, -1.0])
+    kw = dict(rtol=1e-9, method=method, mixed=mixed, precond="fd")
+    x, st = op.pcg(b, **kw)
+    r = np.linalg.norm(b - op.eval_Ku(x)) / np.linalg.norm(b)
+    assert r <= 1e-9 and abs(r - st["rel_residual"]) <= 1e-2 * r + 1e-13
+    for x0 in (0.5 * x, np.where(np.arange(op.ndof) == op.ndof - 1, 1e-200, 0.0)):
+        x2, st2 = op.pcg(b, x0=x0, **kw)
+        assert st2["rel_residual"] <= 1e-9
+        assert np.linalg.norm(x2 - x) < 1e-7 * np.linalg.norm(x)
+    bad = np.zeros(op.ndof)
+    bad[-1] = np.nan
+    try:
+        _, st3 = op.pcg(b, x0=bad, **kw)
+        assert not st3["rel_residual"] <= 1e-9
+    except YetiError as e:
+        assert "EBREAKDOWN" in str(e)

@@ -24,6 +24,9 @@ constexpr int kRedBlocks = 592;     // 4 x 148 SMs
 constexpr int kRedThreads = 256;
 constexpr int kFusedThreads = 1024; // k_cg_fused: one CTA per SM
 constexpr int kChunk = 16;          // iterations enqueued per host check
+// ... of the mixed FD solve, which stops itself about every nine iterations
+// (k_pause): the kernels of the rest of a chunk are launched to return at once
+constexpr int kPauseChunk = 12;
 
 // Sum of nparts partials (single block, fixed order).
 __device__ inline double sum_parts(const double *parts, int nparts, int stride,
@@ -55,6 +58,18 @@ k_absmax(const A *a, int64_t n, double *parts) {
          i += (int64_t)gridDim.x * blockDim.x)
         v = fmax(v, fabs((double)a[i]));
     v = block_max(v, sh);
+    if (threadIdx.x == 0) parts[blockIdx.x] = v;
+}
+
+// Entries that are not zero (NaN is not).
+__global__ void __launch_bounds__(kRedThreads)
+k_nonzero(const double *a, int64_t n, double *parts) {
+    __shared__ double sh[32];
+    double v = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        v += a[i] == 0.0 ? 0.0 : 1.0;
+    v = block_sum(v, sh);
     if (threadIdx.x == 0) parts[blockIdx.x] = v;
 }
 
@@ -749,7 +764,7 @@ static int cg_chunk(yeti_wq_op *op, int prec, T *x, T *r, T *z, T *p, T *Ap,
         YETI_CUDA(cudaGetLastError());
         return YETI_OK;
     }
-    for (int k = 0; k < kChunk; k++) {
+    for (int k = 0; k < (pause ? kPauseChunk : kChunk); k++) {
         YETI_TRY(wq_apply_dev(op, p, Ap, prec, &ds->done, s));
         k_dot_alpha<T><<<kRedBlocks, kRedThreads, 0, s>>>(p, Ap, n, parts, ds);
         k_update_beta<T><<<kRedBlocks, kRedThreads, 0, s>>>(x, r, p, Ap, dinv, z, n, parts, ds);
@@ -1136,16 +1151,30 @@ static int pcg_run(yeti_wq_op *op, const double *b, double *x, double rtol, int 
     k_mask<<<kRedBlocks, kRedThreads, 0, s>>>(db, dinv, n);
     k_mask<<<kRedBlocks, kRedThreads, 0, s>>>(dx, dinv, n);
     k_dot<double, double><<<kRedBlocks, kRedThreads, 0, s>>>(db, db, n, parts, nullptr);
-    count_launches(3);
+    k_nonzero<<<kRedBlocks, kRedThreads, 0, s>>>(dx, n, parts + kRedBlocks);
+    count_launches(4);
+    std::vector<double> hp(2 * kRedBlocks);
+    YETI_CUDA(cudaMemcpyAsync(hp.data(), parts, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+    YETI_CUDA(cudaStreamSynchronize(s));
     double bb = 0.0;
-    YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &bb));
-    // r = b - A x
-    YETI_CUDA(cudaMemsetAsync(dt, 0, n * sizeof(double), s));
-    YETI_TRY(wq_apply_dev(op, dx, dt, YETI_PREC_F64, nullptr, s));
-    k_residual<<<kRedBlocks, kRedThreads, 0, s>>>(db, dt, dinv, dr, n);
-    count_launches(1);
+    bool zero = true;   // x0 == 0
+    for (int i = 0; i < kRedBlocks; i++) {
+        bb += hp[i];
+        zero = zero && hp[kRedBlocks + i] == 0.0;
+    }
+    int iters = 0, outer = 0, f64 = 0, f32 = 0, status = YETI_OK;
+    // r = b - A x (b itself from x = 0)
+    if (zero) {
+        YETI_CUDA(cudaMemcpyAsync(dr, db, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    } else {
+        YETI_CUDA(cudaMemsetAsync(dt, 0, n * sizeof(double), s));
+        YETI_TRY(wq_apply_dev(op, dx, dt, YETI_PREC_F64, nullptr, s));
+        k_residual<<<kRedBlocks, kRedThreads, 0, s>>>(db, dt, dinv, dr, n);
+        count_launches(1);
+        f64 = 1;
+    }
     YETI_CUDA(cudaGetLastError());
-    int iters = 0, outer = 0, f64 = 1, f32 = 0, status = YETI_OK;
+    bool fresh = false;   // dr is the true FP64 residual of dx
     const double tol2 = rtol * rtol * bb;
     double bmax_h = 0.0, dsmax_h = 0.0, stop_abs = 0.0;
     if (hist) {
@@ -1310,7 +1339,7 @@ static int pcg_run(yeti_wq_op *op, const double *b, double *x, double rtol, int 
                 YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &rr64));
                 iters = it;
                 if (!(rr64 == rr64)) { status = YETI_EBREAKDOWN; break; }
-                if (rr64 <= tol2 || it >= maxit) break;
+                if (rr64 <= tol2 || it >= maxit) { fresh = true; break; }
                 const double sc_new = std::sqrt(rr64);
                 // a replacement after the FP32 recursion met the tolerance
                 // restarts the direction (its last update was skipped); after
@@ -1343,7 +1372,7 @@ static int pcg_run(yeti_wq_op *op, const double *b, double *x, double rtol, int 
             count_launches(1);
             YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &rr64));
             if (!(rr64 == rr64)) { status = YETI_EBREAKDOWN; break; }
-            if (rr64 <= tol2 || iters >= maxit) break;
+            if (rr64 <= tol2 || iters >= maxit) { fresh = true; break; }
             const double sc = 1.0 / std::sqrt(rr64);
             k_to_f32<<<kRedBlocks, kRedThreads, 0, s>>>(dr, r32, d32, n, sc);
             k_bi_start<float><<<kRedBlocks, kRedThreads, 0, s>>>(r32, rh, p32, ph, v32, dinv32, n, parts);
@@ -1364,20 +1393,27 @@ static int pcg_run(yeti_wq_op *op, const double *b, double *x, double rtol, int 
         }
     }
     YETI_CUDA(cudaEventRecord(e1, s));
-    // true FP64 residual of the returned solution
-    YETI_CUDA(cudaMemsetAsync(dt, 0, n * sizeof(double), s));
-    YETI_TRY(wq_apply_dev(op, dx, dt, YETI_PREC_F64, nullptr, s));
-    k_residual<<<kRedBlocks, kRedThreads, 0, s>>>(db, dt, dinv, dr, n);
+    // true FP64 residual of the returned solution (a mixed solve that ended on
+    // its tolerance has just formed it)
+    if (!fresh) {
+        YETI_CUDA(cudaMemsetAsync(dt, 0, n * sizeof(double), s));
+        YETI_TRY(wq_apply_dev(op, dx, dt, YETI_PREC_F64, nullptr, s));
+        k_residual<<<kRedBlocks, kRedThreads, 0, s>>>(db, dt, dinv, dr, n);
+        count_launches(1);
+    }
     k_dot<double, double><<<kRedBlocks, kRedThreads, 0, s>>>(dr, dr, n, parts, nullptr);
-    count_launches(2);
+    k_absmax<double><<<kRedBlocks, kRedThreads, 0, s>>>(dr, n, parts + kRedBlocks);
+    k_absmax<double><<<kRedBlocks, kRedThreads, 0, s>>>(db, n, parts + 2 * kRedBlocks);
+    count_launches(3);
     double rr = 0.0, rmax = 0.0, bmax = 0.0;
-    YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &rr));
-    k_absmax<double><<<kRedBlocks, kRedThreads, 0, s>>>(dr, n, parts);
-    count_launches(1);
-    YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &rmax, true));
-    k_absmax<double><<<kRedBlocks, kRedThreads, 0, s>>>(db, n, parts);
-    count_launches(1);
-    YETI_TRY(host_sum(op, parts, kRedBlocks, 1, 0, &bmax, true));
+    hp.resize(3 * kRedBlocks);
+    YETI_CUDA(cudaMemcpyAsync(hp.data(), parts, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+    YETI_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < kRedBlocks; i++) {
+        rr += hp[i];
+        rmax = std::max(rmax, hp[kRedBlocks + i]);
+        bmax = std::max(bmax, hp[2 * kRedBlocks + i]);
+    }
     float ms = 0.f;
     YETI_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
