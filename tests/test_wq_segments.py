@@ -97,3 +97,30 @@ def test_gpu_solves_from_zero_and_from_another_start(cuda_ok, method, mixed):
         assert not st3["rel_residual"] <= 1e-9
     except YetiError as e:
         assert "EBREAKDOWN" in str(e)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nel,p", [((5, 2, 9), 3), ((2, 2, 2), 2), ((19, 9, 4), 5), ((3, 4, 5), (2, 3, 2)),
+                                   ((3, 2, 4), (2, 2, 6))])
+def test_gpu_setup_of_each_precision(cuda_ok, nel, p):
+    """The coefficients kept in one precision, or in both (FP32 rounded from
+    FP64), give the operator, the diagonal and the load of the oracle; the free
+    dofs are counted over face pairs that share a layer too."""
+    from yeti_b200.wq import WQElasticity
+    P = cube_patch(nel, p, perturb=0.1, wrange=(0.8, 1.2), seed=3)
+    clamp = {"w0": (0, 1, 2), "w1": (1,), "u1": (1, 2)}
+    ref = WQOracle(P, 1.0, 0.3, clamp)
+    u = np.random.default_rng(5).standard_normal(ref.ndof)
+    k0, d0, f0 = ref.apply(u), ref.diag(), ref.body_force([0.3, 0.0, -1.0])
+    for have in ("f64", "f32", "both"):
+        op = WQElasticity(P, 1.0, 0.3, clamp, precisions=have)
+        assert op.nfree == int(op.free_mask.sum())
+        if have != "f32":
+            assert np.linalg.norm(op.eval_Ku(u) - k0) < 1e-12 * np.linalg.norm(k0)
+            f = op.eval_bodyforce_vector([0.3, 0.0, -1.0])
+            assert np.linalg.norm(f - f0) < 1e-12 * np.linalg.norm(f0)
+        if have != "f64":
+            k2 = op.eval_Ku(u.astype(np.float32), precision="f32").astype(np.float64)
+            assert np.linalg.norm(k2 - k0) < 2e-6 * np.linalg.norm(k0)
+        bar = 2e-6 if have == "f32" else 1e-12
+        assert np.linalg.norm(op.diag() - d0) < bar * np.linalg.norm(d0)

@@ -17,12 +17,12 @@
 //           three directions and the block's control-point values;
 //   forward sum factorisation w -> v -> u: 4 trial kinds (value, d/du,
 //           d/dv, d/dw) per component at the block's points;
-//   point   per component i, the channels H^{kappa,lambda}_i from the
-//           streamed 45 coefficients (the HBM stream of the operator);
-//           the value channels (kappa or lambda = 0) are zero;
+//   point   per component i, the channels H^{kappa,lambda}_i (kappa, lambda
+//           = u, v, w) from the streamed 45 coefficients (the HBM stream of
+//           the operator);
 //   backward sum factorisation u -> v -> w with the 1-D weights
 //           W^{[d==kappa][d==lambda]}, channels merged as soon as their
-//           remaining weights coincide (16 -> 9 -> 4 -> 1);
+//           remaining weights coincide (9 -> 4 -> 1; the load has one);
 //   store   atomic adds of the block's function values into K u (functions
 //           are shared with neighbouring blocks; the output vector is a few
 //           MB and stays in L2).
@@ -37,20 +37,16 @@
 namespace yeti {
 
 // ----------------------------------------------------------- channel tables
-// channel ch = 4*kappa + lambda; group g = distinct (t_v, t_w); tv, tw, tu
-// encode (test order, trial order) of a direction as 2*test + trial.
-__constant__ int c_grp_nch[9] = {4, 2, 2, 2, 1, 1, 2, 1, 1};
-__constant__ int c_grp_ch[9][4] = {{0, 1, 4, 5}, {2, 6, 0, 0}, {3, 7, 0, 0},
-                                   {8, 9, 0, 0}, {10, 0, 0, 0}, {11, 0, 0, 0},
-                                   {12, 13, 0, 0}, {14, 0, 0, 0}, {15, 0, 0, 0}};
-__constant__ int c_grp_tv[9] = {0, 1, 0, 2, 3, 2, 0, 1, 0};
-__constant__ int c_h_ng[4] = {4, 2, 2, 1};
-__constant__ int c_h_g[4][4] = {{0, 1, 3, 4}, {2, 5, 0, 0}, {6, 7, 0, 0},
-                                {8, 0, 0, 0}};
+// channel ch = 3 k + l of test derivative k and trial derivative l (0: u, 1: v,
+// 2: w); the weight of direction d is tile slot 2 [k == d] + [l == d].  After
+// the u products each channel stands alone; the v products merge the channels
+// that have the same w weight (slot 2 [k == 2] + [l == 2]).
+__constant__ int c_h_n[4] = {4, 2, 2, 1};
+__constant__ int c_h_ch[4][4] = {{0, 1, 3, 4}, {2, 5, 0, 0}, {6, 7, 0, 0}, {8, 0, 0, 0}};
 
-__device__ __forceinline__ int ch_tu(int ch) {
-    const int k = ch >> 2, l = ch & 3;
-    return 2 * (k == 1) + (l == 1);
+__device__ __forceinline__ int ch_slot(int ch, int d) {
+    const int k = ch / 3, l = ch - 3 * k;
+    return 2 * (k == d) + (l == d);
 }
 
 struct BlkCtx {
@@ -84,7 +80,13 @@ __device__ __forceinline__ bool clamped(int cm, const WQAxis *ax, int gu,
            ((cm & 16) && gw == 0) || ((cm & 32) && gw == ax[2].nfun - 1);
 }
 
-// Shared-memory carve-up (in elements of T), identical on host and device.
+// Shared-memory carve-up (in elements of T), identical on host and device:
+// the parts that the sum factorisations of a kernel need, and no more: these
+// kernels wait on short FP64 chains and barriers, so CTAs on an SM are what
+// they gain from.  32x24x28 p=3: geometry 143 -> 95 us, diagonal (9 channels
+// instead of 16, seven of them zero) 191 -> 128 us, load (one channel, once
+// for the three components) 181 -> 14 us.
+enum SmemUse { SM_FWD = 1, SM_BWD = 2, SM_VALUE = 4 };   // forward, nine channels back, one value back
 struct SmemPlan {
     int tile[3];     // offsets of the three direction tiles
     int X, F, R1;    // control-point values, point values, scratch union
@@ -92,7 +94,7 @@ struct SmemPlan {
 };
 
 __host__ __device__ inline SmemPlan smem_plan(const int NF[3], const int NQ[3],
-                                              int NC, int ntile) {
+                                              int NC, int ntile, int use) {
     SmemPlan s;
     int o = 0;
     for (int d = 0; d < 3; d++) {
@@ -103,14 +105,16 @@ __host__ __device__ inline SmemPlan smem_plan(const int NF[3], const int NQ[3],
     o += NC * NF[0] * NF[1] * NF[2];
     s.F = o;
     const int nq = NQ[0] * NQ[1] * NQ[2];
-    o += 4 * NC * nq;
+    if (use & SM_FWD) o += 4 * NC * nq;
     s.R1 = o;
     const int y = 2 * NC * NQ[2] * NF[1] * NF[0];
     const int z = 3 * NC * NQ[2] * NQ[1] * NF[0];
-    const int h = 16 * nq;
-    const int g = 9 * NQ[2] * NQ[1] * NF[0];
-    const int k = 4 * NQ[2] * NF[1] * NF[0];
-    o += (y + z > h + g + k) ? (y + z) : (h + g + k);
+    const int nch = use & SM_BWD ? 9 : 1;
+    const int h = nch * nq;
+    const int g = nch * NQ[2] * NQ[1] * NF[0];
+    const int k = (use & SM_BWD ? 4 : 1) * NQ[2] * NF[1] * NF[0];
+    const int fwd = use & SM_FWD ? y + z : 0, bwd = use & (SM_BWD | SM_VALUE) ? h + g + k : 0;
+    o += fwd > bwd ? fwd : bwd;
     s.total = o;
     return s;
 }
@@ -178,37 +182,35 @@ __device__ void forward(const T *tu, const T *tv, const T *tw, const int NF[3],
 }
 
 // Backward sum factorisation of one component:
-// H[16][nqw][nqv][nqu] -> out[nfw][nfv][nfu], weights at tile slots
-// wbase + (2*test + trial).
-template <class T>
+// H[9][nqw][nqv][nqu] -> out[nfw][nfv][nfu], weights at tile slots
+// wbase + (2*test + trial).  VALUE: the single channel of values against
+// values (a load), H[nqw][nqv][nqu].
+template <class T, bool VALUE>
 __device__ void backward(const T *tu, const T *tv, const T *tw, int wbase,
                          const int NF[3], const int NQ[3], const BlkCtx &c,
                          const T *H, T *G, T *K, T *out) {
     const int nfu = c.nf[0], nfv = c.nf[1], nfw = c.nf[2];
     const int nqu = c.nq[0], nqv = c.nq[1], nqw = c.nq[2];
     const int nqb = c.nqb;
-    // G[g][qw][qv][fu] = sum_{ch in g} sum_qu Wu_tu(ch)[fu][qu] H[ch][qw][qv][qu]
-    const int n1 = 9 * nqw * nqv * nfu;
+    constexpr int NCH = VALUE ? 1 : 9, NH = VALUE ? 1 : 4;
+    // G[ch][qw][qv][fu] = sum_qu Wu[fu][qu] H[ch][qw][qv][qu]
+    const int n1 = NCH * nqw * nqv * nfu;
     for (int o = threadIdx.x; o < n1; o += blockDim.x) {
         const int fu = o % nfu;
         int r = o / nfu;
         const int qv = r % nqv;
         r /= nqv;
         const int qw = r % nqw;
-        const int g = r / nqw;
+        const int ch = r / nqw;
+        const T *W = tu + (wbase + (VALUE ? 0 : ch_slot(ch, 0))) * NF[0] * NQ[0] + fu * NQ[0];
+        const T *h = H + ch * nqb + (qw * nqv + qv) * nqu;
         T acc = 0;
-        const int nch = c_grp_nch[g];
-        for (int k = 0; k < nch; k++) {
-            const int ch = c_grp_ch[g][k];
-            const T *W = tu + (wbase + ch_tu(ch)) * NF[0] * NQ[0] + fu * NQ[0];
-            const T *h = H + ch * nqb + (qw * nqv + qv) * nqu;
-            for (int qu = 0; qu < nqu; qu++) acc += W[qu] * h[qu];
-        }
+        for (int qu = 0; qu < nqu; qu++) acc += W[qu] * h[qu];
         G[o] = acc;
     }
     __syncthreads();
-    // K[h][qw][fv][fu] = sum_{g in h} sum_qv Wv_tv(g)[fv][qv] G[g][qw][qv][fu]
-    const int n2 = 4 * nqw * nfv * nfu;
+    // K[h][qw][fv][fu] = sum_{ch in h} sum_qv Wv[fv][qv] G[ch][qw][qv][fu]
+    const int n2 = NH * nqw * nfv * nfu;
     for (int o = threadIdx.x; o < n2; o += blockDim.x) {
         const int fu = o % nfu;
         int r = o / nfu;
@@ -217,11 +219,11 @@ __device__ void backward(const T *tu, const T *tv, const T *tw, int wbase,
         const int qw = r % nqw;
         const int h = r / nqw;
         T acc = 0;
-        const int ng = c_h_ng[h];
-        for (int k = 0; k < ng; k++) {
-            const int g = c_h_g[h][k];
-            const T *W = tv + (wbase + c_grp_tv[g]) * NF[1] * NQ[1] + fv * NQ[1];
-            const T *gg = G + ((g * nqw + qw) * nqv) * nfu + fu;
+        const int nch = VALUE ? 1 : c_h_n[h];
+        for (int k = 0; k < nch; k++) {
+            const int ch = VALUE ? 0 : c_h_ch[h][k];
+            const T *W = tv + (wbase + (VALUE ? 0 : ch_slot(ch, 1))) * NF[1] * NQ[1] + fv * NQ[1];
+            const T *gg = G + ((ch * nqw + qw) * nqv) * nfu + fu;
             for (int qv = 0; qv < nqv; qv++) acc += W[qv] * gg[qv * nfu];
         }
         K[o] = acc;
@@ -235,7 +237,7 @@ __device__ void backward(const T *tu, const T *tv, const T *tw, int wbase,
         const int fv = r % nfv;
         const int fw = r / nfv;
         T acc = 0;
-        for (int h = 0; h < 4; h++) {
+        for (int h = 0; h < NH; h++) {
             const T *W = tw + (wbase + h) * NF[2] * NQ[2] + fw * NQ[2];
             const T *kk = K + ((h * nqw) * nfv + fv) * nfu + fu;
             for (int qw = 0; qw < nqw; qw++) acc += W[qw] * kk[qw * nfv * nfu];
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_setup(SetupArgs a) {
     const WQAxis *ax = a.v.ax;
     const int NF[3] = {ax[0].NF, ax[1].NF, ax[2].NF};
     const int NQ[3] = {ax[0].NQ, ax[1].NQ, ax[2].NQ};
-    const SmemPlan P = smem_plan(NF, NQ, 4, 2);
+    const SmemPlan P = smem_plan(NF, NQ, 4, 2, SM_FWD);
     BlkCtx c;
     block_ctx(ax, a.v.qoff, blockIdx.x, c);
     int pos[3];
@@ -389,8 +391,8 @@ struct ApplyArgs {
     const int *done;   // optional early-exit flag (PCG)
 };
 
-// Pointwise map of component i: the 16 channels from the 9 derivative
-// trial values (value channels are zero).
+// Pointwise map of component i: the 9 channels from the 9 derivative
+// trial values.
 template <class T>
 __device__ __forceinline__ void point_channels(const T *coef, int64_t base,
                                                int nqb, int q, int i,
@@ -398,19 +400,15 @@ __device__ __forceinline__ void point_channels(const T *coef, int64_t base,
     T f[3][3];
     for (int l = 0; l < 3; l++)
         for (int j = 0; j < 3; j++) f[l][j] = F[((l + 1) * 3 + j) * nqb + q];
-    T h[16];
-    for (int ch = 0; ch < 4; ch++) h[ch] = 0;
     for (int k = 0; k < 3; k++) {
         T S[9];
         for (int Jn = 0; Jn < 9; Jn++) S[Jn] = coef[base + (int64_t)sym9(3 * i + k, Jn) * nqb + q];
-        h[(k + 1) * 4] = 0;
         for (int l = 0; l < 3; l++) {
             T acc = 0;
             for (int j = 0; j < 3; j++) acc += S[3 * j + l] * f[l][j];
-            h[(k + 1) * 4 + (l + 1)] = acc;
+            H[(3 * k + l) * nqb + q] = acc;
         }
     }
-    for (int ch = 0; ch < 16; ch++) H[ch * nqb + q] = h[ch];
 }
 
 template <class T>
@@ -421,7 +419,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_apply(ApplyArgs<T> a) {
     const WQAxis *ax = a.v.ax;
     const int NF[3] = {ax[0].NF, ax[1].NF, ax[2].NF};
     const int NQ[3] = {ax[0].NQ, ax[1].NQ, ax[2].NQ};
-    const SmemPlan P = smem_plan(NF, NQ, 3, 6);
+    const SmemPlan P = smem_plan(NF, NQ, 3, 6, SM_FWD | SM_BWD);
     BlkCtx c;
     block_ctx(ax, a.v.qoff, blockIdx.x, c);
     int pos[3];
@@ -445,7 +443,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_apply(ApplyArgs<T> a) {
                   Y, Z, F);
     const int nqb = c.nqb;
     T *H = sm + P.R1;
-    T *G = H + 16 * NQ[0] * NQ[1] * NQ[2];
+    T *G = H + 9 * NQ[0] * NQ[1] * NQ[2];
     T *K = G + 9 * NQ[2] * NQ[1] * NF[0];
     T *out = X;   // X is dead after the forward pass
     const int64_t base = c.qoff * kWQCoef;
@@ -453,7 +451,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_apply(ApplyArgs<T> a) {
         for (int q = threadIdx.x; q < nqb; q += blockDim.x)
             point_channels<T>(a.v.coef, base, nqb, q, i, F, H);
         __syncthreads();
-        backward<T>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF, NQ, c,
+        backward<T, false>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF, NQ, c,
                     H, G, K, out);
         for (int o = threadIdx.x; o < nx; o += blockDim.x) {
             const int fu = o % nfu, fv = (o / nfu) % nfv, fw = o / (nfu * nfv);
@@ -483,7 +481,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_diag(DiagArgs<T> a) {
     const WQAxis *ax = a.v.ax;
     const int NF[3] = {ax[0].NF, ax[1].NF, ax[2].NF};
     const int NQ[3] = {ax[0].NQ, ax[1].NQ, ax[2].NQ};
-    const SmemPlan P = smem_plan(NF, NQ, 3, 6);
+    const SmemPlan P = smem_plan(NF, NQ, 1, 6, SM_BWD);
     BlkCtx c;
     block_ctx(ax, a.v.qoff, blockIdx.x, c);
     int pos[3];
@@ -494,21 +492,19 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_diag(DiagArgs<T> a) {
     const int nx = nfu * nfv * nfw;
     const int nqb = c.nqb;
     T *H = sm + P.R1;
-    T *G = H + 16 * NQ[0] * NQ[1] * NQ[2];
+    T *G = H + 9 * NQ[0] * NQ[1] * NQ[2];
     T *K = G + 9 * NQ[2] * NQ[1] * NF[0];
     T *out = sm + P.X;
     const int64_t base = c.qoff * kWQCoef;
     const T *coef = a.v.coef;
     for (int i = 0; i < 3; i++) {
         for (int q = threadIdx.x; q < nqb; q += blockDim.x) {
-            for (int kap = 0; kap < 4; kap++)
-                for (int lam = 0; lam < 4; lam++)
-                    H[(kap * 4 + lam) * nqb + q] =
-                        (kap && lam) ? coef[base + (int64_t)sym9(3 * i + kap - 1, 3 * i + lam - 1) * nqb + q]
-                                     : T(0);
+            for (int k = 0; k < 3; k++)
+                for (int l = 0; l < 3; l++)
+                    H[(3 * k + l) * nqb + q] = coef[base + (int64_t)sym9(3 * i + k, 3 * i + l) * nqb + q];
         }
         __syncthreads();
-        backward<T>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF, NQ, c,
+        backward<T, false>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF, NQ, c,
                     H, G, K, out);
         for (int o = threadIdx.x; o < nx; o += blockDim.x) {
             const int fu = o % nfu, fv = (o / nfu) % nfv, fw = o / (nfu * nfv);
@@ -534,7 +530,7 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_force(ForceArgs a) {
     const WQAxis *ax = a.v.ax;
     const int NF[3] = {ax[0].NF, ax[1].NF, ax[2].NF};
     const int NQ[3] = {ax[0].NQ, ax[1].NQ, ax[2].NQ};
-    const SmemPlan P = smem_plan(NF, NQ, 3, 6);
+    const SmemPlan P = smem_plan(NF, NQ, 1, 6, SM_VALUE);
     BlkCtx c;
     block_ctx(ax, a.v.qoff, blockIdx.x, c);
     int pos[3];
@@ -545,25 +541,19 @@ __global__ void __launch_bounds__(kWQThreads) k_wq_force(ForceArgs a) {
     const int nx = nfu * nfv * nfw;
     const int nqb = c.nqb;
     double *H = sm + P.R1;
-    double *G = H + 16 * NQ[0] * NQ[1] * NQ[2];
-    double *K = G + 9 * NQ[2] * NQ[1] * NF[0];
+    double *G = H + NQ[0] * NQ[1] * NQ[2];
+    double *K = G + NQ[2] * NQ[1] * NF[0];
     double *out = sm + P.X;
-    for (int i = 0; i < 3; i++) {
-        for (int q = threadIdx.x; q < nqb; q += blockDim.x) {
-            for (int ch = 1; ch < 16; ch++) H[ch * nqb + q] = 0.0;
-            H[q] = a.f[i] * a.jw[c.qoff + q];
-        }
-        __syncthreads();
-        backward<double>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF,
-                         NQ, c, H, G, K, out);
-        for (int o = threadIdx.x; o < nx; o += blockDim.x) {
-            const int fu = o % nfu, fv = (o / nfu) % nfv, fw = o / (nfu * nfv);
-            const int gu = c.b[0].e0 + fu, gv = c.b[1].e0 + fv, gw = c.b[2].e0 + fw;
-            if (clamped(a.v.cmask[i], ax, gu, gv, gw)) continue;
-            const int64_t cp = gu + (int64_t)ax[0].nfun * (gv + (int64_t)ax[1].nfun * gw);
-            atomicAdd(&a.F[i * a.v.ncp + cp], out[o]);
-        }
-        __syncthreads();
+    // the load of a unit force density, the same for the three components
+    for (int q = threadIdx.x; q < nqb; q += blockDim.x) H[q] = a.jw[c.qoff + q];
+    __syncthreads();
+    backward<double, true>(sm + P.tile[0], sm + P.tile[1], sm + P.tile[2], 2, NF, NQ, c, H, G, K, out);
+    for (int o = threadIdx.x; o < nx; o += blockDim.x) {
+        const int fu = o % nfu, fv = (o / nfu) % nfv, fw = o / (nfu * nfv);
+        const int gu = c.b[0].e0 + fu, gv = c.b[1].e0 + fv, gw = c.b[2].e0 + fw;
+        const int64_t cp = gu + (int64_t)ax[0].nfun * (gv + (int64_t)ax[1].nfun * gw);
+        for (int i = 0; i < 3; i++)
+            if (!clamped(a.v.cmask[i], ax, gu, gv, gw)) atomicAdd(&a.F[i * a.v.ncp + cp], a.f[i] * out[o]);
     }
 }
 
@@ -636,8 +626,8 @@ static WQView<T> make_view(const yeti_wq_op *op, const DevBuf *tiles,
     return v;
 }
 
-static size_t smem_bytes(const yeti_wq_op *op, int NC, int ntile, size_t elem) {
-    SmemPlan P = smem_plan(op->NF, op->NQ, NC, ntile);
+static size_t smem_bytes(const yeti_wq_op *op, int NC, int ntile, int use, size_t elem) {
+    SmemPlan P = smem_plan(op->NF, op->NQ, NC, ntile, use);
     return (size_t)P.total * elem;
 }
 
@@ -658,7 +648,7 @@ static int launch_apply(yeti_wq_op *op, const T *u, T *Ku, const int *done,
     a.u = u;
     a.Ku = Ku;
     a.done = done;
-    const size_t smem = smem_bytes(op, 3, 6, sizeof(T));
+    const size_t smem = smem_bytes(op, 3, 6, SM_FWD | SM_BWD, sizeof(T));
     YETI_TRY(set_smem_optin((const void *)k_wq_apply<T>, op->ctx->device, smem, "WQ apply block"));
     k_wq_apply<T><<<(unsigned)op->nblocks, kWQThreads, smem, s>>>(a);
     count_launches(1);
@@ -735,16 +725,12 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
     // free dofs
     {
         int64_t nfree = 0;
-        for (int c = 0; c < 3; c++)
-            for (int w = 0; w < op->n[2]; w++)
-                for (int v = 0; v < op->n[1]; v++)
-                    for (int u = 0; u < op->n[0]; u++) {
-                        const int cm = op->cmask[c];
-                        bool cl = ((cm & 1) && u == 0) || ((cm & 2) && u == op->n[0] - 1) ||
-                                  ((cm & 4) && v == 0) || ((cm & 8) && v == op->n[1] - 1) ||
-                                  ((cm & 16) && w == 0) || ((cm & 32) && w == op->n[2] - 1);
-                        nfree += !cl;
-                    }
+        for (int c = 0; c < 3; c++) {
+            int64_t box = 1;   // the dofs off the clamped faces (a face pair may be one layer)
+            for (int d = 0; d < 3; d++)
+                box *= std::max(0, op->n[d] - (op->cmask[c] >> (2 * d) & 1) - (op->cmask[c] >> (2 * d + 1) & 1));
+            nfree += box;
+        }
         op->nfree = nfree;
     }
     for (int i = 0; i < ncp; i++)
@@ -791,7 +777,8 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
     YETI_TRY(upload(ctx, dw, weights, (size_t)ncp));
     const int64_t ncoef = op->nqp_total * kWQCoef;
     if (prec_mask & YETI_WQ_F64) YETI_TRY(op->coef64.alloc(ctx, ncoef * sizeof(double)));
-    if (prec_mask & YETI_WQ_F32) YETI_TRY(op->coef32.alloc(ctx, ncoef * sizeof(float)));
+    if ((prec_mask & YETI_WQ_F32) && !(wq_stream_supported(op.get()) && (prec_mask & YETI_WQ_F64)))
+        YETI_TRY(op->coef32.alloc(ctx, ncoef * sizeof(float)));
     YETI_TRY(op->jw.alloc(ctx, op->nqp_total * sizeof(double)));
     YETI_TRY(flags.alloc(ctx, sizeof(int)));
     YETI_CUDA(cudaMemsetAsync(flags.ptr, 0, sizeof(int), ctx->stream));
@@ -820,13 +807,14 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
             }
     }
     sa.coef64 = op->coef64.ptr ? op->coef64.as<double>() : nullptr;
+    // the streaming layout's FP32 coefficients are rounded from the FP64 ones
     sa.coef32 = op->coef32.ptr ? op->coef32.as<float>() : nullptr;
     sa.jw = op->jw.as<double>();
     YETI_TRY(op->sdiag.alloc(ctx, (size_t)op->nblocks * 9 * sizeof(double)));
     sa.sdiag = op->sdiag.as<double>();
     sa.flags = flags.as<int>();
     {
-        const size_t smem = smem_bytes(op.get(), 4, 2, sizeof(double));
+        const size_t smem = smem_bytes(op.get(), 4, 2, SM_FWD, sizeof(double));
         YETI_TRY(wq_smem_limit(ctx, smem));
         YETI_TRY(set_smem_optin((const void *)k_wq_setup, ctx->device, smem, "WQ setup block"));
         k_wq_setup<<<(unsigned)op->nblocks, kWQThreads, smem, ctx->stream>>>(sa);
@@ -842,8 +830,8 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
     YETI_TRY(op->diag.alloc(ctx, op->ndof * sizeof(double)));
     YETI_CUDA(cudaMemsetAsync(op->diag.ptr, 0, op->ndof * sizeof(double), ctx->stream));
     {
-        const size_t smem = (prec_mask & YETI_WQ_F64) ? smem_bytes(op.get(), 3, 6, sizeof(double))
-                                                      : smem_bytes(op.get(), 3, 6, sizeof(float));
+        const size_t smem = (prec_mask & YETI_WQ_F64) ? smem_bytes(op.get(), 1, 6, SM_BWD, sizeof(double))
+                                                      : smem_bytes(op.get(), 1, 6, SM_BWD, sizeof(float));
         YETI_TRY(wq_smem_limit(ctx, smem));
         if (prec_mask & YETI_WQ_F64) {
             DiagArgs<double> da;
@@ -990,7 +978,7 @@ YETI_API int yeti_wq_body_force(yeti_wq_op *op, const double f[3], double *F,
     a.jw = op->jw.as<double>();
     for (int d = 0; d < 3; d++) a.f[d] = f[d];
     a.F = FF;
-    const size_t smem = smem_bytes(op, 3, 6, sizeof(double));
+    const size_t smem = smem_bytes(op, 1, 6, SM_VALUE, sizeof(double));
     YETI_TRY(wq_smem_limit(op->ctx, smem));
     YETI_TRY(set_smem_optin((const void *)k_wq_force, op->ctx->device, smem, "WQ force block"));
     k_wq_force<<<(unsigned)op->nblocks, kWQThreads, smem, s>>>(a);
