@@ -41,6 +41,26 @@ def test_gpu_stiffness_and_mass_tiles_match_oracle(cuda_ok, nel, p):
         np.testing.assert_array_equal(got, ref)
 
 
+# (nel, p, Gauss points per direction): column nodes in one and in several
+# groups, fewer and more functions than points, one to eight points, a layout
+# whose blocks leave no room for the spacing between them
+SF_CASES = [((2, 2, 2), (1, 1, 1), 2), ((2, 1, 2), (3, 1, 2), 2), ((1, 2, 2), (4, 2, 1), 3),
+            ((1, 1, 2), (1, 2, 3), 4), ((1, 1, 1), (6, 5, 4), 5), ((1, 1, 1), (2, 6, 3), 6),
+            ((1, 1, 1), (3, 3, 3), 7), ((1, 1, 1), (7, 2, 3), 8), ((1, 1, 1), (1, 7, 3), 7)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nel,p,ng", SF_CASES)
+def test_gpu_sumfact_shapes_match_oracle(cuda_ok, nel, p, ng):
+    args = u1_system_args(cube_patch(nel, p, perturb=0.1, wrange=(0.8, 1.2), seed=4), E=2.1, nu=0.3,
+                          nbint=ng ** 3)
+    k0, r0, c0, _ = oracle.sys_linmat_lindef_static(*args)
+    k1, r1, c1, _ = sys_linmat_lindef_static(*args, element_kernel="sumfact")
+    np.testing.assert_array_equal(r1, r0)
+    np.testing.assert_array_equal(c1, c0)
+    assert np.linalg.norm(k1 - k0) <= 1e-12 * np.linalg.norm(k0)   # as in test_assembly.py
+
+
 @pytest.mark.gpu
 def test_gpu_assembly_into_arrays_on_8_byte_boundaries(cuda_ok):
     import torch

@@ -455,34 +455,6 @@ __host__ __device__ inline size_t mass_perq(int nn) { return (size_t)stiff_ds(nn
 // Scalar of a point that takes entry c of the inverse Jacobian.
 __host__ __device__ constexpr int inv_slot(int c) { return c < 4 ? c : c + 10; }
 
-// First slot of column node j's blocks, relative to the element's.
-__host__ __device__ inline int64_t slot_col(int j) { return 9LL * j * (j - 1) / 2 + 6LL * j; }
-
-// The slots of an element, a warp per column node j and consecutive lanes on
-// consecutive slots: visit(slot, i, j, row component, column component) for
-// the 9 j + 6 slots of the column (9 per node i < j with the row component
-// fastest, then the upper triangle of the diagonal block).
-template <class V>
-__device__ __forceinline__ void for_slots(int nn, int64_t base, V visit) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    for (int j = warp; j < nn; j += nwarp) {
-        const int64_t jb = base + slot_col(j);
-        for (int sl = lane; sl < 9 * j + 6; sl += 32) {
-            int i = sl / 9, r = sl - 9 * i, ll, kk;
-            if (sl < 9 * j) {
-                ll = r / 3;
-                kk = r - 3 * ll;
-            } else {
-                i = j;
-                r = sl - 9 * j;
-                ll = r < 1 ? 0 : r < 3 ? 1 : 2;
-                kk = r - ll * (ll + 1) / 2;
-            }
-            visit(jb + sl, i, j, kk, ll);
-        }
-    }
-}
-
 // Tile t of the upper triangle of 2 x 2 tiles, column by column.
 __device__ __forceinline__ void tile_of(int t, int &ti, int &tj) {
     tj = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
@@ -553,7 +525,7 @@ k_u1_stiffness(StiffArgs a) {
     const double *Ud[3] = {a.U0, a.U1, a.U2};
     __syncthreads();
     basis_rows(pd, Ud, sni, su1, su2, a.gauss, a.ng, nn, rows, nodes);
-    for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+    for_slots(nn, base, threadIdx.x >> 5, blockDim.x >> 5, [&](int64_t o, int i, int j, int kk, int ll) {
         a.krow[o] = dof[i] + kk;
         a.kcol[o] = dof[j] + ll;
     });
@@ -750,7 +722,7 @@ __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
     __syncthreads();
     basis_rows(pd, Ud, sni, su1, su2, a.gauss, a.ng, nn, rows, nodes);
     if (!a.staged)
-        for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+        for_slots(nn, base, threadIdx.x >> 5, blockDim.x >> 5, [&](int64_t o, int i, int j, int kk, int ll) {
             a.mrow[o] = dof[i] + kk;
             a.mcol[o] = dof[j] + ll;
             if (kk != ll) a.mdata[o] = 0.0;
@@ -822,7 +794,7 @@ __global__ void __launch_bounds__(256) k_u1_mass(MassArgs a) {
     }
     if (!a.staged) return;
     __syncthreads();
-    for_slots(nn, base, [&](int64_t o, int i, int j, int kk, int ll) {
+    for_slots(nn, base, threadIdx.x >> 5, blockDim.x >> 5, [&](int64_t o, int i, int j, int kk, int ll) {
         const double v = ms[j * (j + 1) / 2 + i];
         a.mdata[o] = kk != ll ? 0.0 : i < j ? v : v * 0.5;
         a.mrow[o] = dof[i] + kk;

@@ -45,6 +45,38 @@ struct U1Model {
 // elements, build_system_elemStorage.f90:156-293) and upload the geometry.
 int u1_prepare(yeti_ctx *ctx, const yeti_u1_model *m, U1Model &out);
 
+#ifdef __CUDACC__
+// First slot of column node j's blocks, relative to the element's.
+__host__ __device__ inline int64_t slot_col(int j) { return 9LL * j * (j - 1) / 2 + 6LL * j; }
+
+// The slots of an element, a warp per column node j (of the nwarp that take
+// part) and consecutive lanes on consecutive slots: visit(slot, i, j, row
+// component, column component) for the 9 j + 6 slots of the column (9 per node
+// i < j with the row component fastest, then the upper triangle of the
+// diagonal block).
+template <class V>
+__device__ __forceinline__ void for_slots(int nn, int64_t base, int warp, int nwarp, V visit) {
+    const int lane = threadIdx.x & 31;
+    for (int j = warp; j < nn; j += nwarp) {
+        const int64_t jb = base + slot_col(j);
+        int i = lane / 9, r = lane - 9 * i;
+        for (int sl = lane; sl < 9 * j; sl += 32) {
+            const int ll = r * 11 >> 5;   // r / 3
+            visit(jb + sl, i, j, r - 3 * ll, ll);
+            i += 3;                       // 32 = 3 * 9 + 5
+            if ((r += 5) >= 9) {
+                r -= 9;
+                i++;
+            }
+        }
+        if (lane < 6) {
+            const int ll = lane < 1 ? 0 : lane < 3 ? 1 : 2;
+            visit(jb + 9 * j + lane, j, j, lane - ll * (ll + 1) / 2, ll);
+        }
+    }
+}
+#endif
+
 // Element stiffness of one patch's active elements by the sum-factorised
 // kernel (stiff_sf.cu), written into the COO slots of the pair kernel.
 int launch_u1_stiffness_sf(yeti_ctx *ctx, const U1Patch &P, const double *coords,
