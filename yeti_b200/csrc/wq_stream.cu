@@ -514,8 +514,8 @@ struct StreamArgs {
     const int *elem[2];        // element owning each point along u, v
     const T *band[3];          // [nqp][6][round4(p+1)]: B0 B1 W00 W01 W10 W11
     const int *wq0;            // first w point of each element (nel_w + 1)
-    const WQSeg *seg;
-    const int *cta_seg;        // segments of a CTA
+    const WQSeg *seg;          // the first segment of every CTA, then the others
+    const int *cta_seg;        // where a CTA's others begin (grid + 1)
     int nfun[3];
     int64_t ncp;
     int cmask[3];
@@ -530,11 +530,11 @@ constexpr int kBesidePlanes = 4;
 // CTAs per SM the registers are cut for.  FP32: 128 registers hold a thread's
 // work, and 51.5 KB of shared memory admit four.  FP64: the walks'
 // accumulators, the register rings and the 27 channels of a point, two
-// registers each, outgrow 128 from degree 3 on; fewer CTAs without spills are
-// faster.  Measured (us) with 4 / 3 / 2 CTAs: 64^3 p=2 249 / 247 / 294, p=3
-// 315 / 278 / 320, 128x128x32 p=4 1099 / 919 / 772, 40^3 p=5 250 / 220 / 185.
+// registers each, outgrow 128; fewer CTAs without spills are faster.  Measured
+// (us) with 4 / 3 / 2 CTAs: 64^3 p=2 263 / 233 / 294, p=3 315 / 278 / 320,
+// 128x128x32 p=4 1099 / 919 / 772, 40^3 p=5 250 / 220 / 185.
 template <class T, int P>
-constexpr int kMinCtas = sizeof(T) == 4 || P == 2 ? 4 : P == 3 ? 3 : 2;
+constexpr int kMinCtas = sizeof(T) == 4 ? 4 : P <= 3 ? 3 : 2;
 
 template <class T, int P>
 __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(StreamArgs<T> a) {
@@ -544,7 +544,18 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     // FP32: each plane's coefficient block is brought into shared memory by a
     // bulk copy issued one plane ahead; FP64 reads it from HBM directly
     constexpr bool kStaged = sizeof(T) == 4;
-    if (a.done && *a.done) return;
+    // A small patch's CTA has a plane or two: what it waits for before the
+    // first is a good part of its time, so the loads that do not depend on one
+    // another are issued together: the done flag and the segment; then the
+    // plane's coefficients, the tables and the columns of u.  One after the
+    // other they took 21.0 us for 21x17x25 p=3 FP64 against 19.0, 17.3 against
+    // 15.0 us in FP32, 153 against 150 us for 61x47x29 p=4 FP64 and 138 against
+    // 137 us for 64^3 p=3 FP32.
+    const int done = a.done ? *a.done : 0;
+    int more = a.cta_seg[blockIdx.x];
+    const int more_end = a.cta_seg[blockIdx.x + 1];
+    WQSeg sg = a.seg[blockIdx.x];
+    if (done) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T *const sm = reinterpret_cast<T *>(smraw);
     T *const RY = sm;
@@ -564,8 +575,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     }
     const int64_t plane = (int64_t)a.nfun[0] * a.nfun[1];
 
-    for (int si = a.cta_seg[blockIdx.x]; si < a.cta_seg[blockIdx.x + 1]; si++) {
-        const WQSeg sg = a.seg[si];
+    for (;; sg = a.seg[more++]) {
         const int qu0 = sg.qu0, nqu = sg.nqu, qv0 = sg.qv0, nqv = sg.nqv;
         const int patu = sg.regu & 7, patv = sg.regv & 7;
         const bool peru = (sg.regu & 8) != 0, perv = (sg.regv & 8) != 0;
@@ -579,18 +589,25 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
         const int pbytes = npts * kWQCoef * (int)sizeof(T);
         const int nrow = min(2, nqv - 2 * warp);   // rows of this warp (may be <= 0)
 
-        __syncthreads();   // the previous segment is done with the tables
-        for (int i = tid; i < kTQ * 6 * PBP; i += kThreads) {
-            const int q = i / (6 * PBP), r = i - q * (6 * PBP);
-            tabu[q * TS + r] = q < nqu ? a.band[0][(size_t)(qu0 + q) * 6 * PBP + r] : T(0);
-            if (q < kTV) tabv[q * TS + r] = q < nqv ? a.band[1][(size_t)(qv0 + q) * 6 * PBP + r] : T(0);
-        }
-        if (tid < kTQ) relu[tid] = tid < nqu ? a.elem[0][qu0 + tid] - fu0 : 0;
-        if (tid < kTV) relv[tid] = tid < nqv ? a.elem[1][qv0 + tid] - fv0 : 0;
         const uint32_t cbytes = (uint32_t)((npts * kWQCoef * (int)sizeof(T) + 15) & ~15);
+        // the first plane's coefficients (the previous segment's last block was
+        // read before that plane's last barriers)
         if constexpr (kStaged) {
             if (tid == 0) bulk_load(cbuf, coef_t + (int64_t)sg.qb * pstride, cbytes, bar);
+        } else {
+            const char *p0 = reinterpret_cast<const char *>(coef_t + (int64_t)sg.qb * pstride);
+            for (int off = tid * 128; off < pbytes; off += kThreads * 128) prefetch_l2(p0 + off);
         }
+        constexpr int NTB = (kTQ * 6 * PBP + kThreads - 1) / kThreads;
+        T tu[NTB], tv[NTB];
+#pragma unroll
+        for (int n = 0; n < NTB; n++) {
+            const int i = tid + n * kThreads, q = i / (6 * PBP), r = i - q * (6 * PBP);
+            tu[n] = q < nqu ? a.band[0][(size_t)(qu0 + q) * 6 * PBP + r] : T(0);
+            tv[n] = q < nqv ? a.band[1][(size_t)(qv0 + q) * 6 * PBP + r] : T(0);
+        }
+        const int ru = tid < nqu ? a.elem[0][qu0 + tid] - fu0 : 0;
+        const int rv = tid < nqv ? a.elem[1][qv0 + tid] - fv0 : 0;
         // stage D thread: (ik, fu) and (ik, fu + nfp), the nine ik fastest
         // (FP64: one fu, nfp = nfu)
         constexpr int kDC = sizeof(T) == 4 ? 2 : 1;
@@ -663,11 +680,16 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
         for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
             for (int m = 0; m <= P; m++) x[cc][m] = load_x(cc, sg.eb + m);
-        stage_a(sg.qb);
-        if (!kStaged) {
-            const char *p0 = reinterpret_cast<const char *>(coef_t + (int64_t)sg.qb * pstride);
-            for (int off = tid * 128; off < pbytes; off += kThreads * 128) prefetch_l2(p0 + off);
+        // (the previous segment read its tables before its last barrier)
+#pragma unroll
+        for (int n = 0; n < NTB; n++) {
+            const int i = tid + n * kThreads, q = i / (6 * PBP), r = i - q * (6 * PBP);
+            if (q < kTQ) tabu[q * TS + r] = tu[n];
+            if (q < kTV) tabv[q * TS + r] = tv[n];
         }
+        if (tid < kTQ) relu[tid] = ru;
+        if (tid < kTV) relv[tid] = rv;
+        stage_a(sg.qb);
 
         int e = sg.eb;
         for (int qw = sg.qb; qw < sg.qe; e++) {
@@ -881,6 +903,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
         for (int cc = 0; cc < CPT; cc++)
 #pragma unroll
             for (int m = 0; m < P; m++) retire(cc, e + m, acc[cc][m]);
+        if (more == more_end) break;
     }
 }
 
@@ -1119,8 +1142,8 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
     for (int which = 0; which < 2; which++) {
         const int64_t total = (int64_t)ntiles * nqw;
         const int64_t ncta = std::min<int64_t>((int64_t)nsm * st.per_sm[which], total);
-        std::vector<WQSeg> seg;
-        std::vector<int> cta_seg(ncta + 1, 0);
+        std::vector<WQSeg> seg(ncta);   // every CTA has a segment: ncta <= total
+        std::vector<int> cta_seg(ncta + 1);
         // planes before CTA c: sum over the CTAs before it of 1 + less * ((per_sm - 1) / 2 - round)
         const double less = total >= kRoundPlanes * ncta ? kRoundLess : 0.0;
         std::vector<int64_t> cut(ncta + 1, total);
@@ -1133,6 +1156,7 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
         }
         for (int64_t c = 0; c < ncta; c++) {
             const int64_t end = cut[c + 1];
+            cta_seg[c] = (int)seg.size();
             for (int64_t i = cut[c]; i < end;) {
                 const int t = (int)(i / nqw), tu = t % st.ntile[0], tv = t / st.ntile[0];
                 WQSeg sg;
@@ -1153,11 +1177,12 @@ int wq_stream_setup(yeti_wq_op *op, const WQRule1D R[3]) {
                 sg.nev = (unsigned char)(elem_uv[1][tq0[1][tv] + tnq[1][tv] - 1] - sg.fv0 + 1);
                 sg.nfu = (unsigned char)(sg.neu + P);
                 sg.nfv = (unsigned char)(sg.nev + P);
+                if (i == cut[c]) seg[c] = sg;
+                else seg.push_back(sg);
                 i += sg.qe - sg.qb;
-                seg.push_back(sg);
             }
-            cta_seg[c + 1] = (int)seg.size();
         }
+        cta_seg[ncta] = (int)seg.size();
         st.grid[which] = (int)ncta;
         st.beside[which] = total <= kBesidePlanes * ncta;
         pack.add(st.seg[which], seg);
