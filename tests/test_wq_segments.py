@@ -124,3 +124,19 @@ def test_gpu_setup_of_each_precision(cuda_ok, nel, p):
             assert np.linalg.norm(k2 - k0) < 2e-6 * np.linalg.norm(k0)
         bar = 2e-6 if have == "f32" else 1e-12
         assert np.linalg.norm(op.diag() - d0) < bar * np.linalg.norm(d0)
+
+
+@pytest.mark.gpu
+def test_gpu_fp64_wait_that_runs_out_is_reported(cuda_ok):
+    """FP64 from degree 4 on waits for its coefficients too: with a limit of no
+    polls the apply says so, with the default limit it succeeds again."""
+    from yeti_b200._lib import MEM_HOST, PREC_F64, check, lib, ptr
+    from yeti_b200.wq import WQElasticity
+    op = WQElasticity(cube_patch((5, 4, 6), 4, perturb=0.1, seed=3), 1.0, 0.3, {"w0": (0, 1, 2)})
+    u = np.random.default_rng(5).standard_normal(op.ndof)
+    ref, out = op.eval_Ku(u), np.empty_like(u)
+    check(lib().yeti_wq_set_wait_limit(op.handle, 0), "yeti_wq_set_wait_limit")
+    assert lib().yeti_wq_apply(op.handle, ptr(u), ptr(out), PREC_F64, MEM_HOST) == -5
+    check(lib().yeti_wq_set_wait_limit(op.handle, -1), "yeti_wq_set_wait_limit")
+    check(lib().yeti_wq_apply(op.handle, ptr(u), ptr(out), PREC_F64, MEM_HOST), "yeti_wq_apply")
+    assert np.linalg.norm(out - ref) < 1e-13 * np.linalg.norm(ref)

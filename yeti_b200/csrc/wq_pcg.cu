@@ -1047,7 +1047,11 @@ int cgsolve_finish(CgSolve &cs, double *x_host, cudaStream_t on) {
     std::vector<double> hp(2 * (size_t)nb);
     YETI_CUDA(cudaMemcpyAsync(hp.data(), v.parts, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     YETI_CUDA(cudaMemcpyAsync(x_host, v.x, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    int gave_up = 0;   // as wq_stream_check, beside the other results
+    if (op->st.active)
+        YETI_CUDA(cudaMemcpyAsync(&gave_up, op->st.err.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
     YETI_CUDA(cudaStreamSynchronize(st));
+    YETI_CHECK(!gave_up, YETI_ETIMEDOUT, "WQ apply: a bounded wait for a coefficient copy gave up; results are invalid");
     double rr = 0.0, bb = 0.0;
     for (int i = 0; i < nb; i++) {
         rr += hp[i];

@@ -40,7 +40,8 @@
 // element of a direction) the walk is unrolled at compile time and the ring
 // is register renaming; the first and last tiles take a run-time walk.
 // While a plane is processed, the next plane's coefficient block
-// (contiguous, 256-byte aligned) is prefetched into L2.
+// (contiguous, 256-byte aligned) is copied into shared memory or prefetched
+// into L2 (kStaged).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -69,6 +70,16 @@ constexpr int kHS = 2 * kTQ + 1; // channel stride of a warp's h block
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
 constexpr int round4(int a) { return (a + 3) / 4 * 4; }
 
+// Each plane's coefficient block is brought into shared memory by a bulk copy
+// issued one plane ahead (FP32, and FP64 from degree 4 on, whose two CTAs per SM
+// leave the 46 KB), or read from L2, into which it is prefetched one plane
+// ahead.  FP64, read / staged: 61x47x29 p=4 150 / 140 us, 128x128x32 p=4 713 /
+// 646 us, 40^3 p=5 154 / 143 us.  For p <= 3 three CTAs leave 20 KB: the first 19
+// or 21 of the 45 entries staged there measured the same (64^3 p=3 263 / 264,
+// p=2 233 / 231 us), copied by their own threads slower (287 and 261 us).
+template <class T, int P>
+constexpr bool kStaged = sizeof(T) == 4 || P >= 4;
+
 template <int P>
 struct Dims {
     static constexpr int PB = P + 1;
@@ -96,11 +107,11 @@ struct Dims {
     static constexpr int CPT = (NCOL + kThreads - 1) / kThreads;
     static constexpr int CB = kTQ * kTV * 45;   // one plane's coefficients (staged kernels)
     static_assert(K <= kWarps * ZHP, "K must fit in the Z/h parts");
-    // values, then the staged coefficient block (FP32), the two rel tables
+    // values, then the staged coefficient block, the two rel tables
     // and the mbarrier
     template <class T>
     static constexpr size_t smem_bytes() {
-        return (size_t)(TOTAL + (sizeof(T) == 4 ? CB : 0)) * sizeof(T) + (kTQ + kTV) * sizeof(int) +
+        return (size_t)(TOTAL + (kStaged<T, P> ? CB : 0)) * sizeof(T) + (kTQ + kTV) * sizeof(int) +
                sizeof(uint64_t);
     }
 };
@@ -541,9 +552,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     using D = Dims<P>;
     constexpr int PB = D::PB, PBP = D::PBP, NFM = D::NFM, CPT = D::CPT;
     constexpr int TS = D::TS, GP = D::GP, ZHP = D::ZHP;
-    // FP32: each plane's coefficient block is brought into shared memory by a
-    // bulk copy issued one plane ahead; FP64 reads it from HBM directly
-    constexpr bool kStaged = sizeof(T) == 4;
+    constexpr bool kF32 = sizeof(T) == 4;
     // A small patch's CTA has a plane or two: what it waits for before the
     // first is a good part of its time, so the loads that do not depend on one
     // another are issued together: the done flag and the segment; then the
@@ -564,12 +573,12 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     T *const tabu = sm + D::OFF_TAB;
     T *const tabv = tabu + D::TAB;
     T *const cbuf = sm + D::TOTAL;
-    int *const relu = reinterpret_cast<int *>(sm + D::TOTAL + (kStaged ? D::CB : 0));
+    int *const relu = reinterpret_cast<int *>(sm + D::TOTAL + (kStaged<T, P> ? D::CB : 0));
     int *const relv = relu + kTQ;
     uint64_t *const bar = reinterpret_cast<uint64_t *>(relv + kTV);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t phase = 0;
-    if constexpr (kStaged) {
+    if constexpr (kStaged<T, P>) {
         if (tid == 0) mbar_init(bar);
         __syncthreads();
     }
@@ -592,7 +601,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
         const uint32_t cbytes = (uint32_t)((npts * kWQCoef * (int)sizeof(T) + 15) & ~15);
         // the first plane's coefficients (the previous segment's last block was
         // read before that plane's last barriers)
-        if constexpr (kStaged) {
+        if constexpr (kStaged<T, P>) {
             if (tid == 0) bulk_load(cbuf, coef_t + (int64_t)sg.qb * pstride, cbytes, bar);
         } else {
             const char *p0 = reinterpret_cast<const char *>(coef_t + (int64_t)sg.qb * pstride);
@@ -698,13 +707,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
             const int qw_end = min(a.wq0[e + 1], sg.qe);
             for (; qw < qw_end; qw++) {
                 const T *bw = a.band[2] + (size_t)qw * 6 * PBP;
-                if (!kStaged && qw + 1 < sg.qe) {
-                    // FP64 reads the coefficients straight from HBM: prefetch
-                    // the next plane into L2 (FP32 stages it with a bulk copy)
+                if (!kStaged<T, P> && qw + 1 < sg.qe) {
                     const char *pn = reinterpret_cast<const char *>(coef_t + (int64_t)(qw + 1) * pstride);
                     for (int off = tid * 128; off < pbytes; off += kThreads * 128) prefetch_l2(pn + off);
                 }
-                if constexpr (kStaged) {
+                if constexpr (kStaged<T, P>) {
                     // this plane's coefficient block has landed in shared memory
                     const bool ok = mbar_wait(bar, phase, a.wait_tries);
                     if (__syncthreads_or(!ok)) {
@@ -772,11 +779,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                         __syncwarp();   // the warp's Z is read; h takes its place
                         if (act) {
                             const int pt = (2 * warp + row) * nqu + qu;
-                            // FP32: point-major block in shared memory, 45 values
-                            // per point; FP64: entry-major block in HBM.  Every
-                            // coefficient is read once
-                            const T *cp = kStaged ? cbuf + pt * kWQCoef
-                                                  : coef_t + (int64_t)qw * pstride + pt;
+                            // FP32: point-major block, 45 values per point; FP64:
+                            // entry-major.  Every coefficient is read once
+                            const T *cs = kF32 ? cbuf + pt * kWQCoef : cbuf + pt;
+                            const T *cp = coef_t + (int64_t)qw * pstride + pt;
                             T h[27];
 #pragma unroll
                             for (int ch = 0; ch < 27; ch++) h[ch] = T(0);
@@ -784,7 +790,8 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                             for (int I = 0; I < 9; I++) {
 #pragma unroll
                                 for (int J = I; J < 9; J++) {
-                                    const T sv = kStaged ? cp[sym9(I, J)] : __ldg(cp + sym9(I, J) * npts);
+                                    const int en = sym9(I, J);
+                                    const T sv = kF32 ? cs[en] : kStaged<T, P> ? cs[en * npts] : __ldg(cp + en * npts);
                                     const int i = I / 3, k = I % 3, j = J / 3, l = J % 3;
                                     h[(i * 3 + k) * 3 + l] += sv * f[l][j];
                                     if (I != J) h[(j * 3 + l) * 3 + k] += sv * f[k][i];
@@ -819,7 +826,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                     }
                 }
                 __syncthreads();
-                if constexpr (kStaged) {
+                if constexpr (kStaged<T, P>) {
                     // every warp is done with the block: bring in the next plane's
                     if (tid == 0 && qw + 1 < sg.qe)
                         bulk_load(cbuf, coef_t + (int64_t)(qw + 1) * pstride, cbytes, bar);
@@ -877,7 +884,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                         const T s00 = k00 + k10, s01 = k01 + k11;
 #pragma unroll
                         for (int m = 0; m < PB; m++) {
-                            if constexpr (kStaged) {
+                            if constexpr (kF32) {
                                 acc[cc][m] += w00[m] * s00 + w01[m] * s01 + w10[m] * k20 + w11[m] * k21;
                             } else {
                                 mac2(acc[cc][m], w00[m], s00, w01[m], s01);
