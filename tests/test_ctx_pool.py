@@ -69,3 +69,35 @@ def test_operators_rebuilt_over_freed_ones(cuda_ok):
     for a, b in ((0, 2), (1, 3)):
         assert np.linalg.norm(out[a] - out[b]) < 1e-13 * np.linalg.norm(out[a])
     ctx.close()
+
+
+@pytest.mark.gpu
+def test_a_full_pool_keeps_the_blocks_freed_last(cuda_ok):
+    """Operators of many sizes fill the pool; the calls after them find their
+    blocks in it all the same, and it stays within its 512 MiB."""
+    import torch
+    from yeti_b200._lib import Context
+    from yeti_b200.wq import WQElasticity
+    ctx = Context(0)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def build(nel):
+        op = WQElasticity(cube_patch(nel, 3, perturb=0.1, seed=1), 1.0, 0.3, {"w0": (0, 1, 2)}, ctx=ctx)
+        out = op.eval_Ku(np.ones(op.ndof))
+        op.close()
+        return out
+    build((2, 2, 2))
+    start = free()
+    for n in (16, 20, 24, 26, 28, 30):
+        build((n, n, n))
+    assert start - free() <= (512 + 64) << 20      # and cudaMalloc's own rounding
+    ref, kept = build((32, 24, 28)), free()
+    for _ in range(3):
+        again = build((32, 24, 28))
+        assert np.linalg.norm(again - ref) < 1e-13 * np.linalg.norm(ref)
+        assert abs(free() - kept) <= 8 << 20
+    ctx.close()
+    assert start - free() <= 64 << 20

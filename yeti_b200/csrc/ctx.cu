@@ -101,12 +101,21 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     return YETI_OK;
 }
 
-// Keep the block for the next dev_alloc of its class if there is room.
+// Keep the block for the next dev_alloc of its class; the blocks kept longest
+// make room for it.
 static bool pool_put(yeti_ctx *ctx, void *ptr, size_t cls) {
     if (cls > kPoolBlock) return false;
     std::lock_guard<std::mutex> lock(ctx->pool_mu);
-    if (ctx->pool_bytes + cls > kPoolBytes) return false;
-    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->stream};
+    while (ctx->pool_bytes + cls > kPoolBytes) {
+        auto old = ctx->pool.begin();
+        for (auto it = ctx->pool.begin(); it != ctx->pool.end(); ++it)
+            if (it->second.age < old->second.age) old = it;
+        cudaEventDestroy(old->second.freed);
+        cudaFree(old->second.ptr);
+        ctx->pool_bytes -= old->first;
+        ctx->pool.erase(old);
+    }
+    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->stream, ctx->pool_age++};
     if (cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventRecord(b.freed, ctx->stream) != cudaSuccess) {
         (void)cudaGetLastError();
