@@ -34,6 +34,7 @@
 #include <tuple>
 #include <vector>
 
+#include "fd_stage.cuh"
 #include "reduce.cuh"
 #include "wq.cuh"
 
@@ -376,8 +377,6 @@ constexpr int kFdUnits = sizeof(T) == 4 ? kFdThreads : 8 * FdGemm<double>::kBloc
 template <class T>
 constexpr int kFdLeast = sizeof(T) == 4 ? 32 : kFdThreads;
 
-// m rounded up to whole steps of the contractions.
-__host__ __device__ inline int fd_m4(int m) { return (m + 3) / 4 * 4; }
 // Leading dimension of the 1-D matrices in global memory: that of a staged
 // matrix with all its rows in one tile, so that it is copied as one run.
 template <class T>
@@ -448,7 +447,7 @@ __device__ __forceinline__ void cp_elem(T *sdst, const T *gsrc, bool valid) {
                  : "memory");
 }
 // 16 bytes (both addresses 16-byte aligned), of which the first n elements
-// are read and the rest written as zero.
+// (0 <= n <= 16 / sizeof(T): fd_piece) are read and the rest written as zero.
 template <class T>
 __device__ __forceinline__ void cp_vec(T *sdst, const T *gsrc, int n) {
     const unsigned saddr = (unsigned)__cvta_generic_to_shared(sdst);
@@ -609,8 +608,10 @@ __global__ void __launch_bounds__(kFdThreads, sizeof(T) == 4 ? 3 : 2) k_fd_pass(
             const int64_t base = lb[ll];
             const T *src = base >= 0 ? a.in + base : a.in;
             if (a.vec)
-                for (int k = (tid & 31) * VEC; k < m4; k += 32 * VEC)
-                    cp_vec(Xs + ll * ldx + k, src + k, base >= 0 ? min(VEC, m - k) : 0);
+                for (int k = (tid & 31) * VEC; k < m4; k += 32 * VEC) {
+                    const int n = base >= 0 ? fd_piece(m, k, VEC) : 0;
+                    cp_vec(Xs + ll * ldx + k, n ? src + k : a.in, n);
+                }
             else
                 for (int k = tid & 31; k < m4; k += 32)
                     cp_elem(Xs + ll * ldx + k, k < m ? src + k : src, base >= 0 && k < m);
@@ -707,8 +708,10 @@ __global__ void __launch_bounds__(kFdThreads, sizeof(T) == 4 ? 3 : 2) k_fd_plane
     for (int v = tid >> 5; v < TB; v += nthr >> 5) {
         const T *src = v < mv ? a.in + plane + v * nu : a.in;
         if (a.vec)
-            for (int i = (tid & 31) * VEC; i < mu4; i += 32 * VEC)
-                cp_vec(Xs + v * ldx + i, src + i, v < mv ? min(VEC, mu - i) : 0);
+            for (int i = (tid & 31) * VEC; i < mu4; i += 32 * VEC) {
+                const int n = v < mv ? fd_piece(mu, i, VEC) : 0;
+                cp_vec(Xs + v * ldx + i, n ? src + i : a.in, n);
+            }
         else
             for (int i = tid & 31; i < mu4; i += 32)
                 cp_elem(Xs + v * ldx + i, i < mu ? src + i : src, v < mv && i < mu);
