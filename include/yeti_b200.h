@@ -63,6 +63,8 @@ uint64_t yeti_kernel_launches(void);
  * (non-blocking) unless yeti_ctx_set_stream() supplies one.  hbm_budget_bytes
  * bounds the device memory the context's operators may hold (0 = no bound). */
 int yeti_ctx_create(int device, size_t hbm_budget_bytes, yeti_ctx **out);
+/* Operators of the context may outlive the handle: the context itself goes
+ * with the last of them. */
 int yeti_ctx_destroy(yeti_ctx *ctx);
 /* Use an existing cudaStream_t (passed as void*) for all work of the
  * context; NULL restores the context's own stream (pass cudaStreamLegacy,

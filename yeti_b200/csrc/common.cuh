@@ -48,6 +48,11 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 
 // Context: device, stream and device-memory accounting.
 struct yeti_ctx {
+    // the caller (until yeti_ctx_destroy) and every operator: whoever lets go
+    // last deletes the context, in whatever order they are destroyed (a
+    // garbage collector does not keep one)
+    std::atomic<int> holders{1};
+    std::atomic<bool> closed{false};    // yeti_ctx_destroy was called
     int device = 0;
     cudaStream_t stream = nullptr;      // stream all work goes to
     cudaStream_t own_stream = nullptr;  // stream created by the context
@@ -96,6 +101,23 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes);
 void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes);
 // Give the pool's blocks back to the device.
 void pool_release(yeti_ctx *ctx);
+// One holder less; the last one deletes the context.
+void ctx_let_go(yeti_ctx *ctx);
+
+// A holder of a context.
+struct CtxHold {
+    yeti_ctx *ctx = nullptr;
+    CtxHold() = default;
+    CtxHold(const CtxHold &) = delete;
+    CtxHold &operator=(const CtxHold &) = delete;
+    ~CtxHold() {
+        if (ctx) ctx_let_go(ctx);
+    }
+    void take(yeti_ctx *c) {
+        c->holders.fetch_add(1);
+        ctx = c;
+    }
+};
 
 // RAII device buffer owned by a context, or a view of a part of another one
 // (owned == false).

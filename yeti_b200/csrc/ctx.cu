@@ -104,7 +104,7 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
 // Keep the block for the next dev_alloc of its class; the blocks kept longest
 // make room for it.
 static bool pool_put(yeti_ctx *ctx, void *ptr, size_t cls) {
-    if (cls > kPoolBlock) return false;
+    if (cls > kPoolBlock || ctx->closed) return false;
     std::lock_guard<std::mutex> lock(ctx->pool_mu);
     while (ctx->pool_bytes + cls > kPoolBytes) {
         auto old = ctx->pool.begin();
@@ -133,6 +133,17 @@ void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes) {
     if (ctx && ctx->stream_ordered) cudaFreeAsync(ptr, ctx->stream);
     else if (!ctx || !pool_put(ctx, ptr, pool_class(bytes))) cudaFree(ptr);
     if (ctx) ctx->bytes_in_use -= bytes;
+}
+
+void ctx_let_go(yeti_ctx *ctx) {
+    if (ctx->holders.fetch_sub(1) > 1) return;
+    DeviceGuard g(ctx->device);
+    pool_release(ctx);
+    if (ctx->own_stream) {
+        cudaStreamSynchronize(ctx->own_stream);
+        cudaStreamDestroy(ctx->own_stream);
+    }
+    delete ctx;
 }
 
 static std::atomic<uint64_t> g_launches{0};
@@ -198,13 +209,12 @@ YETI_API int yeti_ctx_create(int device, size_t hbm_budget_bytes,
 
 YETI_API int yeti_ctx_destroy(yeti_ctx *ctx) {
     if (!ctx) return YETI_OK;
-    DeviceGuard g(ctx->device);
-    pool_release(ctx);
-    if (ctx->own_stream) {
-        cudaStreamSynchronize(ctx->own_stream);
-        cudaStreamDestroy(ctx->own_stream);
+    ctx->closed = true;
+    {
+        DeviceGuard g(ctx->device);
+        pool_release(ctx);
     }
-    delete ctx;
+    ctx_let_go(ctx);
     return YETI_OK;
 }
 

@@ -698,6 +698,7 @@ YETI_API int yeti_wq_setup(yeti_ctx *ctx, const int32_t p[3],
     DeviceGuard guard(ctx->device);
     auto t0 = std::chrono::steady_clock::now();
     std::unique_ptr<yeti_wq_op> op(new yeti_wq_op());
+    op->hold.take(ctx);
     op->ctx = ctx;
     op->prec_mask = prec_mask;
     op->E = E;

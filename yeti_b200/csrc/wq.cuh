@@ -195,6 +195,7 @@ int wq_apply_new(yeti_wq_op *op, const void *u, void *Ku, int prec, cudaStream_t
 
 // The operator object behind the opaque yeti_wq_op handle.
 struct yeti_wq_op {
+    yeti::CtxHold hold;     // first: let go after the buffers below are freed
     yeti_ctx *ctx = nullptr;
     int p[3] = {0, 0, 0}, nel[3] = {0, 0, 0}, n[3] = {0, 0, 0};
     int nqp[3] = {0, 0, 0};
