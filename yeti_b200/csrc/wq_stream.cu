@@ -200,8 +200,10 @@ template <class T> struct Pair;
 template <> struct Pair<float> { using type = float2; };
 template <> struct Pair<double> { using type = double2; };
 
-// Wait until the grid this one was launched beside (wq_stream_apply_zeroed)
-// has completed; returns at once in an ordinary launch.
+// Wait until the grid this one was launched beside (launch_stream's k_zero)
+// has completed; returns at once in an ordinary launch.  Every path out of the
+// kernel passes here: what follows it in the stream waits for this grid and
+// may write Ku itself.
 __device__ __forceinline__ void wait_for_primary() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ------------------------------------------------ bulk copies (TMA engine)
@@ -564,7 +566,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
     int more = a.cta_seg[blockIdx.x];
     const int more_end = a.cta_seg[blockIdx.x + 1];
     WQSeg sg = a.seg[blockIdx.x];
-    if (done) return;
+    if (done) {
+        wait_for_primary();
+        return;
+    }
     extern __shared__ __align__(16) unsigned char smraw[];
     T *const sm = reinterpret_cast<T *>(smraw);
     T *const RY = sm;
@@ -718,6 +723,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas<T, P>) k_wq_apply_stream(St
                         if (tid == 0) atomicOr(a.err, 1);
                         // let the copy still in flight land (default bound)
                         mbar_wait(bar, phase, kWaitTries);
+                        wait_for_primary();
                         return;
                     }
                     phase ^= 1;
