@@ -8,6 +8,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/yeti_b200.h"
@@ -63,15 +64,17 @@ struct yeti_ctx {
     bool stream_ordered = false;
     // Freed blocks kept for the next allocations (dev_alloc): a call's
     // scratch costs a list lookup instead of cudaMalloc and cudaFree, which
-    // took 2 to 4 ms of a Gauss call or an operator setup.  Blocks of a size
-    // class are interchangeable; each carries an event recorded on the
-    // context's stream when it was freed, which another stream waits for
-    // before it takes the block.  At most kPoolBytes are kept, the blocks
-    // freed last; they are given back with the context, and earlier when an
-    // allocation fails or the HBM budget needs the room.  (When a full pool kept
-    // the oldest instead, a 32x24x28 p=3 setup after calls of other sizes paid
-    // for cudaMalloc and cudaFree of its 80 MB blocks every time: up to 11 ms
-    // against 1.4 ms.)
+    // took 2 to 4 ms of a Gauss call or an operator setup.  An allocation
+    // takes the smallest kept block that holds it and is at most an eighth
+    // larger (no larger under an HBM budget, which therefore bounds what the
+    // device gives); a new block has the size asked for.  Each kept block
+    // carries an event recorded on the context's stream when it was freed, which
+    // another stream waits for before it takes the block.  At most kPoolBytes
+    // are kept, the blocks freed last; they are given back with the context, and
+    // earlier when an allocation fails or the HBM budget needs the room.  (When
+    // a full pool kept the oldest instead, a 32x24x28 p=3 setup after calls of
+    // other sizes paid for cudaMalloc and cudaFree of its 80 MB blocks every
+    // time: up to 11 ms against 1.4 ms.)
     struct PoolBlock {
         void *ptr;
         cudaEvent_t freed;
@@ -79,7 +82,8 @@ struct yeti_ctx {
         uint64_t age;          // count of blocks kept before it
     };
     std::mutex pool_mu;
-    std::multimap<size_t, PoolBlock> pool;
+    std::multimap<size_t, PoolBlock> pool;     // by size
+    std::unordered_map<void *, size_t> larger; // sizes of blocks in use that exceed what was asked for
     size_t pool_bytes = 0;
     uint64_t pool_age = 0;
     // device-time accounting of the element kernels (yeti_ctx_set_timing)

@@ -23,12 +23,9 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return YETI_ECUDA;
 }
 
-// Size class of a pooled block: bytes rounded up to an eighth of its power of
-// two (512 bytes at least).
-static size_t pool_class(size_t bytes) {
-    size_t step = 512;
-    while (step * 16 <= bytes) step *= 2;
-    return (bytes + step - 1) / step * step;
+// Size of a new block: bytes in units that cudaMalloc hands out anyway.
+static size_t block_size(size_t bytes) {
+    return bytes > SIZE_MAX - 511 ? bytes : (bytes + 511) / 512 * 512;
 }
 
 // The caller holds pool_mu.
@@ -46,18 +43,20 @@ void pool_release(yeti_ctx *ctx) {
     pool_release_locked(ctx);
 }
 
-// A block of the class from the pool, or nullptr.
-static void *pool_take(yeti_ctx *ctx, size_t cls) {
+// A block of at least `size` from the pool, or nullptr.
+static void *pool_take(yeti_ctx *ctx, size_t size) {
+    const size_t most = ctx->hbm_budget ? size : size + std::max<size_t>(size / 8, 4096);
     std::lock_guard<std::mutex> lock(ctx->pool_mu);
-    auto it = ctx->pool.find(cls);
-    if (it == ctx->pool.end()) return nullptr;
+    auto it = ctx->pool.lower_bound(size);
+    if (it == ctx->pool.end() || it->first > most) return nullptr;
     const yeti_ctx::PoolBlock b = it->second;
     if (b.stream != ctx->stream && cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
+    if (it->first > size) ctx->larger[b.ptr] = it->first;
+    ctx->pool_bytes -= it->first;
     ctx->pool.erase(it);
-    ctx->pool_bytes -= cls;
     cudaEventDestroy(b.freed);
     return b.ptr;
 }
@@ -74,19 +73,19 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     if (ctx->stream_ordered) {
         e = cudaMallocAsync(ptr, bytes, ctx->stream);
     } else {
-        const size_t cls = pool_class(bytes);
-        *ptr = pool_take(ctx, cls);
+        const size_t size = block_size(bytes);
+        *ptr = pool_take(ctx, size);
         if (!*ptr) {
             {
                 std::lock_guard<std::mutex> lock(ctx->pool_mu);
                 if (ctx->hbm_budget && ctx->bytes_in_use + ctx->pool_bytes + bytes > ctx->hbm_budget)
                     pool_release_locked(ctx);
             }
-            e = cudaMalloc(ptr, cls);
+            e = cudaMalloc(ptr, size);
             if (e != cudaSuccess) {
                 (void)cudaGetLastError();
                 pool_release(ctx);
-                e = cudaMalloc(ptr, cls);
+                e = cudaMalloc(ptr, size);
             }
         }
     }
@@ -101,12 +100,18 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     return YETI_OK;
 }
 
-// Keep the block for the next dev_alloc of its class; the blocks kept longest
-// make room for it.
-static bool pool_put(yeti_ctx *ctx, void *ptr, size_t cls) {
-    if (cls > kPoolBlock || ctx->closed) return false;
+// Keep the block, asked for as `bytes`, for a later dev_alloc; the blocks kept
+// longest make room for it.
+static bool pool_put(yeti_ctx *ctx, void *ptr, size_t bytes) {
     std::lock_guard<std::mutex> lock(ctx->pool_mu);
-    while (ctx->pool_bytes + cls > kPoolBytes) {
+    size_t size = block_size(bytes);
+    const auto big = ctx->larger.find(ptr);
+    if (big != ctx->larger.end()) {
+        size = big->second;
+        ctx->larger.erase(big);
+    }
+    if (size > kPoolBlock || ctx->closed) return false;
+    while (ctx->pool_bytes + size > kPoolBytes) {
         auto old = ctx->pool.begin();
         for (auto it = ctx->pool.begin(); it != ctx->pool.end(); ++it)
             if (it->second.age < old->second.age) old = it;
@@ -122,8 +127,8 @@ static bool pool_put(yeti_ctx *ctx, void *ptr, size_t cls) {
         if (b.freed) cudaEventDestroy(b.freed);
         return false;
     }
-    ctx->pool.emplace(cls, b);
-    ctx->pool_bytes += cls;
+    ctx->pool.emplace(size, b);
+    ctx->pool_bytes += size;
     return true;
 }
 
@@ -131,7 +136,7 @@ void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes) {
     if (!ptr) return;
     if (!bytes) bytes = 16;
     if (ctx && ctx->stream_ordered) cudaFreeAsync(ptr, ctx->stream);
-    else if (!ctx || !pool_put(ctx, ptr, pool_class(bytes))) cudaFree(ptr);
+    else if (!ctx || !pool_put(ctx, ptr, bytes)) cudaFree(ptr);
     if (ctx) ctx->bytes_in_use -= bytes;
 }
 
