@@ -61,7 +61,10 @@ uint64_t yeti_kernel_launches(void);
 
 /* Create a context on CUDA device `device`.  The context owns a stream
  * (non-blocking) unless yeti_ctx_set_stream() supplies one.  hbm_budget_bytes
- * bounds the device memory the context's operators may hold (0 = no bound). */
+ * bounds the device memory the context's operators may hold (0 = no bound).
+ * The context keeps up to 512 MiB of the device memory that its calls and
+ * operators have freed (blocks of 128 MiB at most; within the budget) for the
+ * next ones: see yeti_ctx_trim. */
 int yeti_ctx_create(int device, size_t hbm_budget_bytes, yeti_ctx **out);
 /* Operators of the context may outlive the handle: the context itself goes
  * with the last of them. */
@@ -71,8 +74,13 @@ int yeti_ctx_destroy(yeti_ctx *ctx);
  * (void*)0x1, for the legacy default stream). */
 int yeti_ctx_set_stream(yeti_ctx *ctx, void *stream);
 int yeti_ctx_synchronize(yeti_ctx *ctx);
-/* Bytes of device memory currently held by the context's objects. */
+/* Bytes of device memory currently held by the context's objects (without
+ * what is kept for the next ones). */
 size_t yeti_ctx_bytes_in_use(const yeti_ctx *ctx);
+/* Give the freed device memory that the context keeps back to the device, for
+ * other allocators of the process.  (A context of this library that runs out
+ * of memory takes back what all of them keep by itself.) */
+int yeti_ctx_trim(yeti_ctx *ctx);
 /* Device-time accounting (no counterpart in the reference).  With timing
  * on, the element kernels of the Gauss-quadrature calls ("k_u1_stiffness",
  * "k_u1_stiffness_sf", "k_u1_mass", "k_u1_grad") are bracketed by CUDA

@@ -178,10 +178,40 @@ static void reuse() {
     HOLDS(used == 0 && events.empty());
 }
 
+// What a context keeps goes back on request, and when another one, serving or
+// not, finds the device full.
+static void given_back() {
+    capacity = 400 * MiB;
+    yeti_ctx *a = context(), *b = context();
+    auto keep = [&] {
+        void *p = take(a, 120 * MiB), *q = take(a, 110 * MiB);
+        HOLDS(p && q);
+        yeti::dev_free(a, p, 120 * MiB);
+        yeti::dev_free(a, q, 110 * MiB);
+        HOLDS(used == 230 * MiB && yeti_ctx_bytes_in_use(a) == 0);
+    };
+    keep();
+    HOLDS(yeti_ctx_trim(a) == YETI_OK && used == 0 && events.empty());
+    for (bool serving : {false, true}) {
+        b->stream_ordered = serving;
+        keep();
+        void *p = take(b, 300 * MiB);
+        HOLDS(p && used == 300 * MiB);
+        yeti::dev_free(b, p, 300 * MiB);
+        HOLDS(used == 0);
+    }
+    HOLDS(yeti_ctx_trim(nullptr) == YETI_EINVAL);
+    yeti_ctx_destroy(a);
+    void *p = take(b, 401 * MiB);                    // past the context that is gone
+    HOLDS(!p);
+    yeti_ctx_destroy(b);
+}
+
 int main(int, char **argv) {
     const std::map<std::string, void (*)()> all = {{"sizes", sizes},
                                                    {"device_just_large_enough", device_just_large_enough},
                                                    {"budget", budget},
-                                                   {"reuse", reuse}};
+                                                   {"reuse", reuse},
+                                                   {"given_back", given_back}};
     all.at(argv[1])();
 }

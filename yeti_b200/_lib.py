@@ -96,6 +96,7 @@ def _declare(lib):
         "yeti_ctx_set_stream": (i32, [vp, vp]),
         "yeti_ctx_synchronize": (i32, [vp]),
         "yeti_ctx_bytes_in_use": (ctypes.c_size_t, [vp]),
+        "yeti_ctx_trim": (i32, [vp]),
         "yeti_ctx_set_timing": (i32, [vp, i32]),
         "yeti_ctx_kernel_ms": (ctypes.c_double, [vp, ctypes.c_char_p]),
         "yeti_serve_open": (i32, [i32, ctypes.c_size_t, i32, ctypes.POINTER(vp)]),
@@ -204,6 +205,11 @@ class Context:
 
     def bytes_in_use(self):
         return int(lib().yeti_ctx_bytes_in_use(self.handle))
+
+    def trim(self):
+        """Give the freed device memory that the context keeps for its next
+        calls (512 MiB at most) back to the device."""
+        check(lib().yeti_ctx_trim(self.handle), "yeti_ctx_trim")
 
     def set_timing(self, on=True):
         """Sum the device time of the element kernels per name (CUDA events

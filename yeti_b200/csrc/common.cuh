@@ -71,7 +71,8 @@ struct yeti_ctx {
     // carries an event recorded on the context's stream when it was freed, which
     // another stream waits for before it takes the block.  At most kPoolBytes
     // are kept, the blocks freed last; they are given back with the context, and
-    // earlier when an allocation fails or the HBM budget needs the room.  (When
+    // earlier by yeti_ctx_trim, when an allocation of any context on the device
+    // fails, or when the HBM budget needs the room.  (When
     // a full pool kept the oldest instead, a 32x24x28 p=3 setup after calls of
     // other sizes paid for cudaMalloc and cudaFree of its 80 MB blocks every
     // time: up to 11 ms against 1.4 ms.)

@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstring>
+#include <set>
 
 #include "common.cuh"
 
@@ -43,6 +44,23 @@ void pool_release(yeti_ctx *ctx) {
     pool_release_locked(ctx);
 }
 
+// All contexts (never destroyed: they may outlive this file's objects).
+static std::mutex &all_mu() {
+    static std::mutex &m = *new std::mutex;
+    return m;
+}
+static std::set<yeti_ctx *> &all_contexts() {
+    static std::set<yeti_ctx *> &s = *new std::set<yeti_ctx *>;
+    return s;
+}
+
+// Room on the device: what any context of the process keeps there.
+static void pools_release(int device) {
+    std::lock_guard<std::mutex> lock(all_mu());
+    for (yeti_ctx *c : all_contexts())
+        if (c->device == device) pool_release(c);
+}
+
 // A block of at least `size` from the pool, or nullptr.
 static void *pool_take(yeti_ctx *ctx, size_t size) {
     const size_t most = ctx->hbm_budget ? size : size + std::max<size_t>(size / 8, 4096);
@@ -72,6 +90,11 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
     cudaError_t e = cudaSuccess;
     if (ctx->stream_ordered) {
         e = cudaMallocAsync(ptr, bytes, ctx->stream);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            pools_release(ctx->device);
+            e = cudaMallocAsync(ptr, bytes, ctx->stream);
+        }
     } else {
         const size_t size = block_size(bytes);
         *ptr = pool_take(ctx, size);
@@ -84,7 +107,7 @@ int dev_alloc(yeti_ctx *ctx, void **ptr, size_t bytes) {
             e = cudaMalloc(ptr, size);
             if (e != cudaSuccess) {
                 (void)cudaGetLastError();
-                pool_release(ctx);
+                pools_release(ctx->device);
                 e = cudaMalloc(ptr, size);
             }
         }
@@ -142,6 +165,10 @@ void dev_free(yeti_ctx *ctx, void *ptr, size_t bytes) {
 
 void ctx_let_go(yeti_ctx *ctx) {
     if (ctx->holders.fetch_sub(1) > 1) return;
+    {
+        std::lock_guard<std::mutex> lock(all_mu());
+        all_contexts().erase(ctx);
+    }
     DeviceGuard g(ctx->device);
     pool_release(ctx);
     if (ctx->own_stream) {
@@ -208,6 +235,10 @@ YETI_API int yeti_ctx_create(int device, size_t hbm_budget_bytes,
         return cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
     c->stream = c->own_stream;
+    {
+        std::lock_guard<std::mutex> lock(all_mu());
+        all_contexts().insert(c);
+    }
     *out = c;
     return YETI_OK;
 }
@@ -233,6 +264,13 @@ YETI_API int yeti_ctx_synchronize(yeti_ctx *ctx) {
     YETI_CHECK(ctx, YETI_EINVAL, "yeti_ctx_synchronize: ctx is NULL");
     DeviceGuard g(ctx->device);
     YETI_CUDA(cudaStreamSynchronize(ctx->stream));
+    return YETI_OK;
+}
+
+YETI_API int yeti_ctx_trim(yeti_ctx *ctx) {
+    YETI_CHECK(ctx, YETI_EINVAL, "yeti_ctx_trim: ctx is NULL");
+    DeviceGuard g(ctx->device);
+    pool_release(ctx);
     return YETI_OK;
 }
 
