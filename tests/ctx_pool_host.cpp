@@ -207,11 +207,33 @@ static void given_back() {
     yeti_ctx_destroy(b);
 }
 
+// The stream that takes a block waits for the one that freed it, also where
+// the same handle names a stream created since.
+static void order() {
+    yeti_ctx *c = context();
+    cudaStream_t s[] = {reinterpret_cast<cudaStream_t>(0x11), reinterpret_cast<cudaStream_t>(0x22)};
+    size_t n = 0;
+    for (int from : {0, 1})
+        for (int to : {0, 1}) {
+            HOLDS(yeti_ctx_set_stream(c, s[from]) == YETI_OK);
+            void *p = take(c, 3 * MiB);
+            HOLDS(p && waits.size() == n);
+            yeti::dev_free(c, p, 3 * MiB);
+            HOLDS(yeti_ctx_set_stream(c, s[to]) == YETI_OK);
+            HOLDS(take(c, 3 * MiB) == p && waits.size() == ++n && waits.back() == std::make_pair(s[to], s[from]));
+            yeti::dev_free(c, p, 3 * MiB);
+            HOLDS(yeti_ctx_trim(c) == YETI_OK);
+        }
+    yeti_ctx_destroy(c);
+    HOLDS(used == 0 && events.empty());
+}
+
 int main(int, char **argv) {
     const std::map<std::string, void (*)()> all = {{"sizes", sizes},
                                                    {"device_just_large_enough", device_just_large_enough},
                                                    {"budget", budget},
                                                    {"reuse", reuse},
-                                                   {"given_back", given_back}};
+                                                   {"given_back", given_back},
+                                                   {"order", order}};
     all.at(argv[1])();
 }

@@ -20,7 +20,8 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["sizes", "device_just_large_enough", "budget", "reuse", "given_back"])
+@pytest.mark.parametrize("scenario", ["sizes", "device_just_large_enough", "budget", "reuse", "given_back",
+                                      "order"])
 def test_pool(harness, scenario):
     r = subprocess.run([harness, scenario], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -68,7 +68,8 @@ static void *pool_take(yeti_ctx *ctx, size_t size) {
     auto it = ctx->pool.lower_bound(size);
     if (it == ctx->pool.end() || it->first > most) return nullptr;
     const yeti_ctx::PoolBlock b = it->second;
-    if (b.stream != ctx->stream && cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
+    // on the same stream too: a handle may be that of a stream created since
+    if (cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
@@ -143,7 +144,7 @@ static bool pool_put(yeti_ctx *ctx, void *ptr, size_t bytes) {
         ctx->pool_bytes -= old->first;
         ctx->pool.erase(old);
     }
-    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->stream, ctx->pool_age++};
+    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->pool_age++};
     if (cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventRecord(b.freed, ctx->stream) != cudaSuccess) {
         (void)cudaGetLastError();
