@@ -1092,7 +1092,10 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
     std::vector<Loaded> loaded;
     std::vector<PatchRhs> patch_erhs;
     int64_t erhs_total = 0;
-    const LoadMarks marks(m, [](int64_t ty) { return ty == 101 || ty == 102 || (ty > 9 && ty < 100); });
+    const ElementLoads eloads(m, [](int64_t ty) { return ty == 101 || ty == 102 || (ty > 9 && ty < 100); });
+    std::vector<int64_t> infos(m->nb_load > 0 ? m->nb_load : 0, 0);   // where a load's additional infos begin
+    for (size_t il = 1; il < infos.size(); il++)
+        infos[il] = infos[il - 1] + (m->nb_load_addinfos ? m->nb_load_addinfos[il - 1] : 0);
     std::vector<int64_t> ien_offset(M.patches.size(), 0);
     for (size_t ip = 1; ip < M.patches.size(); ip++)
         ien_offset[ip] = ien_offset[ip - 1] + M.patches[ip - 1].nelem * M.patches[ip - 1].nn;
@@ -1147,37 +1150,33 @@ YETI_API int yeti_assemble_u1_coo_ex(yeti_ctx *ctx, const yeti_u1_model *m,
         int max_body = 0;
         for (int64_t le = 0; le < P.nactive; le++) {
             const int64_t jel = P.act[le] + 1;   // 1-based element number
-            int64_t cinfo = 0;
             size_t before = terms.size();
             int nbody = 0;
-            for (int64_t il = 0; il < m->nb_load; il++) {
-                const int64_t ty = m->jdltype[il];
-                if (marks.on(il, jel)) {
-                    LoadTerm T;
-                    memset(&T, 0, sizeof(T));
-                    T.mag = m->adlmag[il];
-                    if (ty == 101 || ty == 102) {
-                        T.kind = ty == 101 ? 0 : 1;
-                        int nneed = ty == 101 ? 6 : 3;
-                        YETI_CHECK(cinfo + nneed <= m->len_load_addinfos, YETI_EINVAL,
-                                   "load %lld: missing additional infos", (long long)il + 1);
-                        for (int d = 0; d < nneed; d++) T.info[d] = m->load_addinfos[cinfo + d];
-                        nbody++;
-                    } else {
-                        T.kind = 2;
-                        T.face = (int)(ty / 10);
-                        T.type = (int)(ty % 10);
-                        if (T.type == 4) {
-                            YETI_CHECK(cinfo < m->len_load_addinfos && m->nodal_dist, YETI_EINVAL,
-                                       "load %lld: nodal distribution missing", (long long)il + 1);
-                            T.ifield = (int)m->load_addinfos[cinfo] - 1;
-                            YETI_CHECK(T.ifield >= 0 && T.ifield < m->nb_n_dist, YETI_EINVAL,
-                                       "load %lld: nodal field index", (long long)il + 1);
-                        }
+            for (const int64_t il : eloads.of(jel)) {
+                const int64_t ty = m->jdltype[il], cinfo = infos[il];
+                LoadTerm T;
+                memset(&T, 0, sizeof(T));
+                T.mag = m->adlmag[il];
+                if (ty == 101 || ty == 102) {
+                    T.kind = ty == 101 ? 0 : 1;
+                    int nneed = ty == 101 ? 6 : 3;
+                    YETI_CHECK(cinfo + nneed <= m->len_load_addinfos, YETI_EINVAL,
+                               "load %lld: missing additional infos", (long long)il + 1);
+                    for (int d = 0; d < nneed; d++) T.info[d] = m->load_addinfos[cinfo + d];
+                    nbody++;
+                } else {
+                    T.kind = 2;
+                    T.face = (int)(ty / 10);
+                    T.type = (int)(ty % 10);
+                    if (T.type == 4) {
+                        YETI_CHECK(cinfo < m->len_load_addinfos && m->nodal_dist, YETI_EINVAL,
+                                   "load %lld: nodal distribution missing", (long long)il + 1);
+                        T.ifield = (int)m->load_addinfos[cinfo] - 1;
+                        YETI_CHECK(T.ifield >= 0 && T.ifield < m->nb_n_dist, YETI_EINVAL,
+                                   "load %lld: nodal field index", (long long)il + 1);
                     }
-                    terms.push_back(T);
                 }
-                cinfo += m->nb_load_addinfos ? m->nb_load_addinfos[il] : 0;
+                terms.push_back(T);
             }
             if (terms.size() > before) {
                 elems.push_back((int32_t)le);

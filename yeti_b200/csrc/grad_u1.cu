@@ -662,7 +662,7 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         sol_d = dsol.as<double>();
         adj_d = dadj.as<double>();
     }
-    const LoadMarks marks(m, [](int64_t ty) { return ty == 101 || (ty > 9 && ty < 100); });
+    const ElementLoads eloads(m, [](int64_t ty) { return ty == 101 || (ty > 9 && ty < 100); });
     // element contributions, in global element order
     struct Done { int patch; int64_t local; int64_t off; };
     std::vector<Done> done;
@@ -681,11 +681,10 @@ YETI_API int yeti_grad_lin_elast_work(yeti_ctx *ctx, const yeti_u1_model *m,
         for (int64_t le = 0; le < P.nactive; le++) {
             const int64_t jel = P.act[le] + 1;
             int nb = 0;
-            for (int64_t il = 0; il < m->nb_load; il++)
-                if (marks.on(il, jel)) {
-                    terms.push_back((int32_t)il);
-                    nb += m->jdltype[il] == 101;
-                }
+            for (const int64_t il : eloads.of(jel)) {
+                terms.push_back((int32_t)il);
+                nb += m->jdltype[il] == 101;
+            }
             YETI_CHECK(nb <= 8, YETI_EUNSUPPORTED, "more than 8 centrifugal loads on one element");
             max_body = std::max(max_body, nb);
             elems.push_back((int32_t)le);

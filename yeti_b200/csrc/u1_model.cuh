@@ -2,6 +2,7 @@
 // sys_linmat_lindef_static) into per-patch device arrays, shared by the
 // assembly and the shape-gradient kernels.
 #pragma once
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -83,29 +84,52 @@ int launch_u1_stiffness_sf(yeti_ctx *ctx, const U1Patch &P, const double *coords
                            double lam, double mu, double *kdata, int32_t *krow,
                            int32_t *kcol, size_t smem_cap);
 
-// Which elements carry a distributed or body load, per load: on(il, jel) for
-// load il and 1-based element jel.
-class LoadMarks {
-    std::vector<std::vector<char>> mark;   // empty: not such a load
+// The distributed and body loads of each element, in order: of(jel) for a
+// 1-based element.  As large as the loads' lists of targets and one entry per
+// element (a mark per load and element would be gigabytes for a thousand loads
+// on a million elements).
+class ElementLoads {
+    std::vector<int64_t> ptr, loads;   // loads of jel: ptr[jel] .. ptr[jel + 1]
 
 public:
+    struct Range {
+        const int64_t *b, *e;
+        const int64_t *begin() const { return b; }
+        const int64_t *end() const { return e; }
+    };
     // takes(type): the loads of interest
     template <class F>
-    LoadMarks(const yeti_u1_model *m, F takes) : mark(m->nb_load > 0 ? m->nb_load : 0) {
-        int64_t k = 0;
-        for (int64_t il = 0; il < m->nb_load; il++) {
-            const int64_t n = m->load_target_nbelem[il];
-            if (takes(m->jdltype[il])) {
-                mark[il].assign(m->nb_elem + 1, 0);
-                for (int64_t i = 0; i < n; i++) {
-                    const int64_t e = m->inddload[k + i];
-                    if (e >= 1 && e <= m->nb_elem) mark[il][e] = 1;
+    ElementLoads(const yeti_u1_model *m, F takes) {
+        std::vector<int64_t> last;     // the load that listed an element last
+        auto walk = [&](auto visit) {
+            int64_t k = 0;
+            for (int64_t il = 0; il < m->nb_load; il++) {
+                const int64_t n = m->load_target_nbelem[il];
+                if (takes(m->jdltype[il])) {
+                    last.resize(m->nb_elem + 1, -1);
+                    ptr.resize(m->nb_elem + 2, 0);
+                    for (int64_t i = 0; i < n; i++) {
+                        const int64_t e = m->inddload[k + i];
+                        if (e < 1 || e > m->nb_elem || last[e] == il) continue;
+                        last[e] = il;
+                        visit(e, il);
+                    }
                 }
+                k += n;
             }
-            k += n;
-        }
+        };
+        walk([&](int64_t e, int64_t) { ptr[e + 1]++; });
+        if (ptr.empty()) return;
+        for (int64_t e = 0; e <= m->nb_elem; e++) ptr[e + 1] += ptr[e];
+        loads.resize(ptr.back());
+        std::fill(last.begin(), last.end(), -1);
+        std::vector<int64_t> at(ptr.begin(), ptr.end() - 1);
+        walk([&](int64_t e, int64_t il) { loads[at[e]++] = il; });
     }
-    bool on(int64_t il, int64_t jel) const { return !mark[il].empty() && mark[il][jel]; }
+    Range of(int64_t jel) const {
+        if (ptr.empty()) return {nullptr, nullptr};
+        return {loads.data() + ptr[jel], loads.data() + ptr[jel + 1]};
+    }
 };
 
 }  // namespace yeti
