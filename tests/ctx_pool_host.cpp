@@ -20,6 +20,8 @@ uintptr_t next_event = 1, next_stream = 0x1000;
 std::set<uintptr_t> events;
 std::map<uintptr_t, cudaStream_t> recorded;            // event -> stream
 std::vector<std::pair<cudaStream_t, cudaStream_t>> waits;   // (waiting stream, stream of the event)
+std::map<cudaStream_t, unsigned long long> ids;         // handle -> the stream it names now
+unsigned long long next_id = 1;
 }  // namespace fake
 using namespace fake;
 
@@ -58,6 +60,10 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
     waits.push_back({s, recorded.at(reinterpret_cast<uintptr_t>(e))});
     return cudaSuccess;
+}
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long *id) {
+    if (!ids.count(s)) ids[s] = next_id++;
+    return *id = ids[s], cudaSuccess;
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 0.f, cudaSuccess; }
@@ -207,23 +213,27 @@ static void given_back() {
     yeti_ctx_destroy(b);
 }
 
-// The stream that takes a block waits for the one that freed it, also where
-// the same handle names a stream created since.
+// A stream that takes a block waits for the one that freed it, unless it is
+// the same; a handle that names a stream created since is not.
 static void order() {
     yeti_ctx *c = context();
     cudaStream_t s[] = {reinterpret_cast<cudaStream_t>(0x11), reinterpret_cast<cudaStream_t>(0x22)};
     size_t n = 0;
     for (int from : {0, 1})
-        for (int to : {0, 1}) {
-            HOLDS(yeti_ctx_set_stream(c, s[from]) == YETI_OK);
-            void *p = take(c, 3 * MiB);
-            HOLDS(p && waits.size() == n);
-            yeti::dev_free(c, p, 3 * MiB);
-            HOLDS(yeti_ctx_set_stream(c, s[to]) == YETI_OK);
-            HOLDS(take(c, 3 * MiB) == p && waits.size() == ++n && waits.back() == std::make_pair(s[to], s[from]));
-            yeti::dev_free(c, p, 3 * MiB);
-            HOLDS(yeti_ctx_trim(c) == YETI_OK);
-        }
+        for (int to : {0, 1})
+            for (bool again : {false, true}) {
+                HOLDS(yeti_ctx_set_stream(c, s[from]) == YETI_OK);
+                void *p = take(c, 3 * MiB);
+                HOLDS(p && waits.size() == n);
+                yeti::dev_free(c, p, 3 * MiB);
+                if (again) ids[s[to]] = next_id++;       // destroyed, and created at the same place
+                HOLDS(yeti_ctx_set_stream(c, s[to]) == YETI_OK);
+                HOLDS(take(c, 3 * MiB) == p);
+                if (from != to || again) HOLDS(waits.size() == ++n && waits.back() == std::make_pair(s[to], s[from]));
+                HOLDS(waits.size() == n);
+                yeti::dev_free(c, p, 3 * MiB);
+                HOLDS(yeti_ctx_trim(c) == YETI_OK);
+            }
     yeti_ctx_destroy(c);
     HOLDS(used == 0 && events.empty());
 }

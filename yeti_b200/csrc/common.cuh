@@ -69,7 +69,7 @@ struct yeti_ctx {
     // larger (no larger under an HBM budget, which therefore bounds what the
     // device gives); a new block has the size asked for.  Each kept block
     // carries an event recorded on the context's stream when it was freed, which
-    // the stream that takes the block waits for.  At most kPoolBytes
+    // another stream waits for before it takes the block.  At most kPoolBytes
     // are kept, the blocks freed last; they are given back with the context, and
     // earlier by yeti_ctx_trim, when an allocation of any context on the device
     // fails, or when the HBM budget needs the room.  (When
@@ -79,6 +79,8 @@ struct yeti_ctx {
     struct PoolBlock {
         void *ptr;
         cudaEvent_t freed;
+        unsigned long long stream;   // id of the stream it was recorded on: a
+                                     // handle may come back as a new stream's
         uint64_t age;          // count of blocks kept before it
     };
     std::mutex pool_mu;

@@ -68,8 +68,9 @@ static void *pool_take(yeti_ctx *ctx, size_t size) {
     auto it = ctx->pool.lower_bound(size);
     if (it == ctx->pool.end() || it->first > most) return nullptr;
     const yeti_ctx::PoolBlock b = it->second;
-    // on the same stream too: a handle may be that of a stream created since
-    if (cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
+    unsigned long long id = 0;
+    if ((cudaStreamGetId(ctx->stream, &id) != cudaSuccess || id != b.stream) &&
+        cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
@@ -144,8 +145,9 @@ static bool pool_put(yeti_ctx *ctx, void *ptr, size_t bytes) {
         ctx->pool_bytes -= old->first;
         ctx->pool.erase(old);
     }
-    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->pool_age++};
-    if (cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
+    yeti_ctx::PoolBlock b{ptr, nullptr, 0, ctx->pool_age++};
+    if (cudaStreamGetId(ctx->stream, &b.stream) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventRecord(b.freed, ctx->stream) != cudaSuccess) {
         (void)cudaGetLastError();
         if (b.freed) cudaEventDestroy(b.freed);
