@@ -25,7 +25,7 @@
 // backward with U).  Each pass is a small-K GEMM over the lines of the box,
 // its operands staged whole in shared memory; the vectors (a few MB) stay in
 // L2 between passes.  FP64 runs on the FP64 matrix instructions, FP32 on
-// packed FMAs over 8x8 register tiles (struct FdGemm).
+// packed FMAs over 4x8 register tiles (struct FdGemm).
 #include <algorithm>
 #include <cmath>
 #include <deque>

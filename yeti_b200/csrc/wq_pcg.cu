@@ -25,7 +25,10 @@ constexpr int kRedThreads = 256;
 constexpr int kFusedThreads = 1024; // k_cg_fused: one CTA per SM
 constexpr int kChunk = 16;          // iterations enqueued per host check
 // ... of the mixed FD solve, which stops itself about every nine iterations
-// (k_pause): the kernels of the rest of a chunk are launched to return at once
+// (k_pause): the kernels of the rest of a chunk are launched to return at once.
+// Solves to 1e-10 with 12 / 16 (ms): 16^3 p=2 4.41 / 4.86, 24^3 p=3 5.40 / 5.93,
+// 48^3 p=3 8.85 / 9.36, 64^3 p=3 14.87 / 15.40, 40^3 p=4 7.54 / 8.07, 128x128x32
+// p=4 28.3 / 29.0; where no pause comes in 20,000 iterations, 2181 / 2179.
 constexpr int kPauseChunk = 12;
 
 // Sum of nparts partials (single block, fixed order).
