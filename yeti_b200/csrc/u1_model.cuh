@@ -2,7 +2,6 @@
 // sys_linmat_lindef_static) into per-patch device arrays, shared by the
 // assembly and the shape-gradient kernels.
 #pragma once
-#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -85,50 +84,55 @@ int launch_u1_stiffness_sf(yeti_ctx *ctx, const U1Patch &P, const double *coords
                            int32_t *kcol, size_t smem_cap);
 
 // The distributed and body loads of each element, in order: of(jel) for a
-// 1-based element.  As large as the loads' lists of targets and one entry per
+// 1-based element.  As large as the loads' lists of targets and one number per
 // element (a mark per load and element would be gigabytes for a thousand loads
 // on a million elements).
 class ElementLoads {
-    std::vector<int64_t> ptr, loads;   // loads of jel: ptr[jel] .. ptr[jel + 1]
+    struct Node {
+        int32_t load, next;
+    };
+    std::vector<int32_t> head;   // first node of an element, -1: none; empty: no such loads
+    std::vector<Node> nodes;
 
 public:
+    struct Iter {
+        const Node *nodes;
+        int32_t i;
+        int64_t operator*() const { return nodes[i].load; }
+        Iter &operator++() { return i = nodes[i].next, *this; }
+        bool operator!=(const Iter &o) const { return i != o.i; }
+    };
     struct Range {
-        const int64_t *b, *e;
-        const int64_t *begin() const { return b; }
-        const int64_t *end() const { return e; }
+        Iter b, e;
+        Iter begin() const { return b; }
+        Iter end() const { return e; }
     };
     // takes(type): the loads of interest
     template <class F>
     ElementLoads(const yeti_u1_model *m, F takes) {
-        std::vector<int64_t> last;     // the load that listed an element last
-        auto walk = [&](auto visit) {
-            int64_t k = 0;
-            for (int64_t il = 0; il < m->nb_load; il++) {
-                const int64_t n = m->load_target_nbelem[il];
-                if (takes(m->jdltype[il])) {
-                    last.resize(m->nb_elem + 1, -1);
-                    ptr.resize(m->nb_elem + 2, 0);
-                    for (int64_t i = 0; i < n; i++) {
-                        const int64_t e = m->inddload[k + i];
-                        if (e < 1 || e > m->nb_elem || last[e] == il) continue;
-                        last[e] = il;
-                        visit(e, il);
-                    }
-                }
-                k += n;
+        int64_t k = 0, targets = 0;
+        for (int64_t il = 0; il < m->nb_load; il++) {
+            k += m->load_target_nbelem[il];
+            if (takes(m->jdltype[il])) targets += m->load_target_nbelem[il];
+        }
+        if (!targets) return;
+        head.assign(m->nb_elem + 1, -1);
+        nodes.reserve(targets);
+        // from the last load on, each before those that an element has
+        for (int64_t il = m->nb_load - 1; il >= 0; il--) {
+            const int64_t n = m->load_target_nbelem[il];
+            k -= n;
+            if (!takes(m->jdltype[il])) continue;
+            for (int64_t i = 0; i < n; i++) {
+                const int64_t e = m->inddload[k + i];
+                if (e < 1 || e > m->nb_elem || (head[e] >= 0 && nodes[head[e]].load == il)) continue;
+                nodes.push_back({(int32_t)il, head[e]});
+                head[e] = (int32_t)nodes.size() - 1;
             }
-        };
-        walk([&](int64_t e, int64_t) { ptr[e + 1]++; });
-        if (ptr.empty()) return;
-        for (int64_t e = 0; e <= m->nb_elem; e++) ptr[e + 1] += ptr[e];
-        loads.resize(ptr.back());
-        std::fill(last.begin(), last.end(), -1);
-        std::vector<int64_t> at(ptr.begin(), ptr.end() - 1);
-        walk([&](int64_t e, int64_t il) { loads[at[e]++] = il; });
+        }
     }
     Range of(int64_t jel) const {
-        if (ptr.empty()) return {nullptr, nullptr};
-        return {loads.data() + ptr[jel], loads.data() + ptr[jel + 1]};
+        return {{nodes.data(), head.empty() ? -1 : head[jel]}, {nodes.data(), -1}};
     }
 };
 
