@@ -234,6 +234,13 @@ static void order() {
                 yeti::dev_free(c, p, 3 * MiB);
                 HOLDS(yeti_ctx_trim(c) == YETI_OK);
             }
+    // the handle of each thread's own stream says nothing about which
+    HOLDS(yeti_ctx_set_stream(c, cudaStreamPerThread) == YETI_OK);
+    for (int k = 0; k < 2; k++) {
+        void *p = take(c, 3 * MiB);
+        HOLDS(p && waits.size() == n + k);
+        yeti::dev_free(c, p, 3 * MiB);
+    }
     yeti_ctx_destroy(c);
     HOLDS(used == 0 && events.empty());
 }

@@ -56,6 +56,7 @@ struct yeti_ctx {
     std::atomic<bool> closed{false};    // yeti_ctx_destroy was called
     int device = 0;
     cudaStream_t stream = nullptr;      // stream all work goes to
+    unsigned long long stream_id = 0;   // its id (ctx.cu), taken when it was set
     cudaStream_t own_stream = nullptr;  // stream created by the context
     size_t hbm_budget = 0;              // 0: unbounded
     std::atomic<size_t> bytes_in_use{0};
@@ -79,8 +80,7 @@ struct yeti_ctx {
     struct PoolBlock {
         void *ptr;
         cudaEvent_t freed;
-        unsigned long long stream;   // id of the stream it was recorded on: a
-                                     // handle may come back as a new stream's
+        unsigned long long stream;   // id of the stream it was recorded on
         uint64_t age;          // count of blocks kept before it
     };
     std::mutex pool_mu;

@@ -61,6 +61,18 @@ static void pools_release(int device) {
         if (c->device == device) pool_release(c);
 }
 
+// Id of the stream that a handle names now: one for each stream of the
+// process, never given again (a handle may come back as a new stream's).  None
+// for the handle that names another stream in every thread.
+constexpr unsigned long long kNoStreamId = ~0ull;
+static unsigned long long stream_id(cudaStream_t s) {
+    unsigned long long id = 0;
+    if (s == cudaStreamPerThread) return kNoStreamId;
+    if (cudaStreamGetId(s, &id) == cudaSuccess) return id;
+    (void)cudaGetLastError();
+    return kNoStreamId;
+}
+
 // A block of at least `size` from the pool, or nullptr.
 static void *pool_take(yeti_ctx *ctx, size_t size) {
     const size_t most = ctx->hbm_budget ? size : size + std::max<size_t>(size / 8, 4096);
@@ -68,8 +80,7 @@ static void *pool_take(yeti_ctx *ctx, size_t size) {
     auto it = ctx->pool.lower_bound(size);
     if (it == ctx->pool.end() || it->first > most) return nullptr;
     const yeti_ctx::PoolBlock b = it->second;
-    unsigned long long id = 0;
-    if ((cudaStreamGetId(ctx->stream, &id) != cudaSuccess || id != b.stream) &&
+    if ((b.stream == kNoStreamId || b.stream != ctx->stream_id) &&
         cudaStreamWaitEvent(ctx->stream, b.freed, 0) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
@@ -145,9 +156,8 @@ static bool pool_put(yeti_ctx *ctx, void *ptr, size_t bytes) {
         ctx->pool_bytes -= old->first;
         ctx->pool.erase(old);
     }
-    yeti_ctx::PoolBlock b{ptr, nullptr, 0, ctx->pool_age++};
-    if (cudaStreamGetId(ctx->stream, &b.stream) != cudaSuccess ||
-        cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
+    yeti_ctx::PoolBlock b{ptr, nullptr, ctx->stream_id, ctx->pool_age++};
+    if (cudaEventCreateWithFlags(&b.freed, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventRecord(b.freed, ctx->stream) != cudaSuccess) {
         (void)cudaGetLastError();
         if (b.freed) cudaEventDestroy(b.freed);
@@ -238,6 +248,7 @@ YETI_API int yeti_ctx_create(int device, size_t hbm_budget_bytes,
         return cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
     c->stream = c->own_stream;
+    c->stream_id = stream_id(c->stream);
     {
         std::lock_guard<std::mutex> lock(all_mu());
         all_contexts().insert(c);
@@ -259,7 +270,9 @@ YETI_API int yeti_ctx_destroy(yeti_ctx *ctx) {
 
 YETI_API int yeti_ctx_set_stream(yeti_ctx *ctx, void *stream) {
     YETI_CHECK(ctx, YETI_EINVAL, "yeti_ctx_set_stream: ctx is NULL");
+    DeviceGuard g(ctx->device);
     ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+    ctx->stream_id = stream_id(ctx->stream);
     return YETI_OK;
 }
 

@@ -364,7 +364,7 @@ YETI_API int yeti_serve_open(int device, size_t hbm_budget_bytes, int max_active
         YETI_CUDA(cudaStreamCreateWithPriority(&hs, cudaStreamNonBlocking, prio_high));
         cudaStreamDestroy(wc->own_stream);
         wc->own_stream = hs;
-        wc->stream = hs;
+        YETI_TRY(yeti_ctx_set_stream(wc, nullptr));
         s->wctx.push_back(wc);
         cudaStream_t cs;
         YETI_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
